@@ -301,7 +301,13 @@ def bench_ours(args):
         bricks += br
     tiles /= 2
     bricks //= 2
+    kernel = phases[-1]["kernel"]
+    solve_name = {1: "solve_kernel", 2: "solve_tb_kernel", 3: "dt_plane_kernel + dt_depth_kernel"}[kernel]
     b_iter = 3 * 4096 * tiles
+    if kernel == 3:
+        # distance transform: a byte per voxel of the domain (bounding box of
+        # A u B, x in words) and direction, written once and read once
+        b_iter = sum(4 * _domain_voxels(x, y) for x, y in pairs) / 2
     b_pack = 2 * N + 2 * (N // 8)
     pk = statistics.mean(p["pack_ms"] for p in phases)
     su = statistics.mean(p["setup_ms"] for p in phases)
@@ -318,7 +324,7 @@ def bench_ours(args):
     else:
         achieved = None
         alg = None
-    kname = {"solve": "solve_tb_kernel" if phases[-1]["kernel"] == 2 else "solve_kernel",
+    kname = {"solve": solve_name,
              "pack": "pack_kernel", "setup": "setup_kernel"}[dom]
     traffic = None
     try:
@@ -334,7 +340,7 @@ def bench_ours(args):
     if split_ph and dom == "solve":
         so_split = statistics.mean(p["solve_ms"] for p in split_ph)
         value_launch = {
-            "launch": f"solve_tb_kernel on the dilation SMs of the pipelined entry ({split_ph[0]['grid_ctas']} CTAs)",
+            "launch": f"{solve_name} on the dilation SMs of the pipelined entry ({split_ph[0]['grid_ctas']} CTAs)",
             "solve_ms": round(so_split, 4), "pack_ms": round(statistics.mean(p["pack_ms"] for p in split_ph), 4),
             "setup_ms": round(statistics.mean(p["setup_ms"] for p in split_ph), 4),
             "achieved": round(b_iter / (so_split * 1e-3) / 1e9, 1)}
@@ -352,7 +358,7 @@ def bench_ours(args):
         achieved = value_launch["achieved"]
         so = so_split
     roofline = {
-        "bound": "hbm", "kernel": kname + {"solve": " (persistent frontier dilation)", "pack": " (uint8 -> bits)",
+        "bound": "hbm", "kernel": kname + {"solve": " (distance transform)" if kernel == 3 else " (persistent frontier dilation)", "pack": " (uint8 -> bits)",
                                            "setup": " (crop + first queue)"}[dom],
         "achieved": round(achieved, 1) if achieved else None, "peak": peak, "unit": "GB/s",
         "frac": round(achieved / peak, 4) if achieved else None, "peak_source": f"{peak_kind} MEASURED_PEAKS hbm_gbs",
@@ -367,7 +373,7 @@ def bench_ours(args):
                                       "profile kernels launched in a green context")
         roofline["value_launch"] = value_launch
         roofline["whole_gpu_launch"] = {
-            "launch": f"solve_tb_kernel of the blocking entry on every SM ({phases[-1]['grid_ctas']} CTAs)",
+            "launch": f"{solve_name} of the blocking entry on every SM ({phases[-1]['grid_ctas']} CTAs)",
             "solve_ms": round(so_whole, 4), "achieved": round(b_iter / (so_whole * 1e-3) / 1e9, 1),
             "frac": round(b_iter / (so_whole * 1e-3) / 1e9 / peak, 4)}
     gvox = (refs[0]["hd"] + refs[1]["hd"]) / 2 * 2 * N / (step_ms * 1e-3) / 1e9
@@ -381,7 +387,7 @@ def bench_ours(args):
         "config": {"workload": WORKLOAD, "W": W_, "H": H_, "D": D_, "element": "se6",
                    "l2": "inputs larger than L2: two distinct pairs alternate (2 x 134 MB of masks)",
                    "parallelism": f"replicas x{ws}" if ws > 1 else "single GPU",
-                   "kernel": "temporally blocked" if phases[-1]["kernel"] == 2 else "one step per barrier",
+                   "kernel": {1: "one step per barrier", 2: "temporally blocked", 3: "distance transform"}[kernel],
                    "steps_per_barrier": phases[-1]["steps_per_barrier"],
                    "brick_words_rows_planes": [phases[-1]["brick_x_words"], phases[-1]["brick_rows"],
                                                phases[-1]["brick_z"]], "grid_ctas": phases[-1]["grid_ctas"]},
@@ -397,7 +403,7 @@ def bench_ours(args):
                 "blocking_ms_per_step": round(blocking_e2e_ms, 4),
                 "blocking_path": "hd_compute_u8, one call per pair, masks read in place over the host link",
                 "staged_copy_ms_per_step": round(staged_ms, 4)},
-        "gpu_launches": 3 * args.steps,  # per pair: pack, set-up, persistent dilation (decodes the result too)
+        "gpu_launches": 3 * args.steps,  # per pair: pack, in-plane distances, distances at the targets (decodes the result too)
         "value_path": "hd_compute_u8_device_pipelined x K, hd_pipeline_flush: packing and set-up on 56 SMs, "
                       "consecutive pairs dilating side by side on three groups of 32 (green contexts, six "
                       "workspaces in turn)",
@@ -777,6 +783,14 @@ def bench_worst_case(ctx, tctx, dev):
         "solve_algorithmic_gbs": round(alg / (tim["solve_ms"] * 1e-3) / 1e9, 1),
         "solve_ms": round(tim["solve_ms"], 3), "pack_ms": round(tim["pack_ms"], 3),
     }
+
+
+def _domain_voxels(a, b):
+    """Voxels of the pair's domain: the bounding box of A u B, x in whole words."""
+    u = (a != 0) | (b != 0)
+    axes = [u.any(2).any(1), u.any(2).any(0), u.any(1).any(0)]  # z, y, x
+    lo, hi = zip(*[(int(v.nonzero().min()), int(v.nonzero().max())) for v in axes])
+    return (hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * 32 * (hi[2] // 32 - lo[2] // 32 + 1)
 
 
 def cpu_baseline(a_np, b_np, ref):

@@ -380,9 +380,21 @@ hd_status decode_result(const hdk::PairInfo& I, const hdk::JobState& s0, const h
     return (hd_status)st;
 }
 
-Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n) {
-    // built-in default (the autotuner's winners on GB300): the blocked kernel
-    // with 4 x (32 - 2 steps) x 8 bricks; 4 steps per barrier for a single
+bool dt_takes(int se, const PairIn* pairs, int n) {
+    return se == 0 && n == 1 && hdk::dt_fits(pairs[0].W, pairs[0].H, pairs[0].D);
+}
+
+bool loop_asked(const hd_options& o) {
+    return o.kernel != 0 || o.brick_x_words > 0 || o.brick_z > 0 || o.steps_per_barrier > 0 || o.ctas_per_sm > 0 ||
+           o.max_iterations > 0 || o.barrier_timeout_ns > 0;
+}
+
+Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n, bool dt) {
+    // built-in default: the distance transform for single pairs under the
+    // 6-neighbour element unless an option asks for the dilation loop (a
+    // kernel, a brick shape, a cap on its steps or on its waits); else
+    // (the autotuner's winners on GB300) the blocked kernel with
+    // 4 x (32 - 2 steps) x 8 bricks; 4 steps per barrier for a single
     // pair (fewest barriers), 2 for batches (the work per barrier is large)
     Shape sh;
     double vox = 0;
@@ -390,8 +402,15 @@ Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n) {
     vox /= std::max(1, n);
     sh.steps = n <= 1 ? 4 : 2;
     auto it = ctx->tune.entries.find(tune_key(se, vox, n));
-    if (it != ctx->tune.entries.end()) sh = it->second.shape;
     const hd_options& o = ctx->opt;
+    const bool dt_ok = dt && !loop_asked(o) && dt_takes(se, pairs, n);
+    const bool tuned = it != ctx->tune.entries.end();
+    if (dt_ok && (!tuned || it->second.shape.kernel == 3)) {
+        sh.kernel = 3;
+        sh.finish();
+        return sh;
+    }
+    if (tuned && it->second.shape.kernel != 3) sh = it->second.shape;
     if (o.kernel == 1 || o.kernel == 2) sh.kernel = o.kernel;
     if (o.kernel == 0 && o.brick_x_words > 0 && o.steps_per_barrier == 0) sh.kernel = 1;
     if (o.brick_x_words > 0) sh.bxw = o.brick_x_words;
@@ -413,9 +432,10 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (n > hdk::kMaxPairsPerLaunch) return set_error(ctx, HD_ERR_BAD_ARG, "too many pairs in one launch");
     const int se = ro.se;
     const bool stats = ro.stats != 0;
-    Shape sh = ro.force_shape ? ro.shape : pick_shape(ctx, se, pairs, n);
-    if (stats || ro.map_a || ro.map_b) {
-        // instrumented runs and per-voxel maps are implemented by the one-step kernel
+    Shape sh = ro.force_shape ? ro.shape : pick_shape(ctx, se, pairs, n, !stats);
+    if (stats || ((ro.map_a || ro.map_b) && sh.kernel != 3)) {
+        // instrumented runs, and per-voxel maps without the distance transform,
+        // are implemented by the one-step kernel
         if (sh.kernel != 1) {
             sh.kernel = 1;
             sh.bxw = 4;
@@ -443,8 +463,9 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         for (int i = 0; i < n; ++i) out[perm[i]] = tmp[i];
         return st;
     }
-    const void* solve_fn = solve_fn_of(se, sh);
-    if (!solve_fn)
+    const bool dt = sh.kernel == 3;
+    const void* solve_fn = dt ? nullptr : solve_fn_of(se, sh);
+    if (!solve_fn && !dt)
         return set_error(ctx, HD_ERR_BAD_ARG, "kernel %d with %d words x %d rows x %d planes (%d steps) not compiled in",
                          sh.kernel, sh.bxw, sh.by, sh.bz, sh.steps);
     const int bxw = sh.bxw, by = sh.by, bz = sh.bz, cps = sh.ctas_per_sm;
@@ -476,7 +497,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         q.full_words = (long long)hdk::packed_pitch(P.W) * P.H * P.D;
         const long long pitch = (q.wxf + 3) / 4 * 4;
         q.dom_words = pitch * P.H * P.D;
-        q.bricks = (long long)((q.wxf + bxw - 1) / bxw) * ((P.H + by - 1) / by) * ((P.D + bz - 1) / bz);
+        q.bricks = dt ? 0 : (long long)((q.wxf + bxw - 1) / bxw) * ((P.H + by - 1) / by) * ((P.D + bz - 1) / bz);
         int kmax = P.W + P.H + P.D;
         if (ctx->opt.max_iterations > 0) kmax = std::min(kmax, ctx->opt.max_iterations);
         q.kmax = kmax;
@@ -498,8 +519,15 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         PairPlan& q = plan[i];
         q.off_pa = take(4ULL * q.full_words);
         q.off_pb = take(4ULL * q.full_words);
-        for (int j = 0; j < 2; ++j)
-            for (int b = 0; b < 3; ++b) q.off_jb[j][b] = take(4ULL * q.dom_words);
+        for (int j = 0; j < 2; ++j) {
+            if (dt) {
+                q.off_jb[j][0] = take(4ULL * hdk::dt_vol_words(pairs[i].W, pairs[i].H, pairs[i].D));
+                q.off_jb[j][1] = take(2ULL * hdk::dt_bases(pairs[i].W, pairs[i].H, pairs[i].D));
+                q.off_jb[j][2] = take(8ULL * hdk::dt_bases(pairs[i].W, pairs[i].H, pairs[i].D));
+            } else {
+                for (int b = 0; b < 3; ++b) q.off_jb[j][b] = take(4ULL * q.dom_words);
+            }
+        }
         const size_t nb = (size_t)pairs[i].W * pairs[i].H * pairs[i].D;
         q.off_in_a = (pairs[i].host_a && !ro.async_out) ? take(nb) : 0;
         q.off_in_b = (pairs[i].host_b && !ro.async_out) ? take(nb) : 0;
@@ -521,7 +549,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     // group), both the caller's stream otherwise.  The caller's stream waits
     // for the dilations only at a flush (or the next other call).
     const bool async = ro.async_out != nullptr;
-    const bool split = async && ro.pipelined && n == 1 && sh.kernel == 2 &&
+    const bool split = async && ro.pipelined && n == 1 && sh.kernel != 1 &&
                        (double)pairs[0].W * pairs[0].H * pairs[0].D <= (double)(1 << 26) && split_ready(ctx);
     if (!split && ctx->split.pending) {  // every other call follows the pipelined ones
         const cudaError_t e0 = wait_split_dilations(ctx, s);
@@ -547,6 +575,13 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
 
     if (total_bytes > arena.cap) drain_split();
     cudaError_t e = arena.ensure(total_bytes);
+    if (e != cudaSuccess && dt && !ro.force_shape) {
+        // the distance transform's workspace is larger: the dilation loop's may fit
+        RunOpts r2 = ro;
+        r2.force_shape = true;
+        r2.shape = pick_shape(ctx, se, pairs, n, false);
+        return run_pairs(ctx, pairs, n, s, r2, out);
+    }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "device workspace");
     if (split) {
         // the packing waits for the caller's earlier work and for the
@@ -657,7 +692,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         Dd.pa = (uint32_t*)(dbase + q.off_pa);
         Dd.pb = (uint32_t*)(dbase + q.off_pb);
         for (int j = 0; j < 2; ++j) {
-            for (int b = 0; b < 3; ++b) Dd.jb[j][b] = (uint32_t*)(dbase + q.off_jb[j][b]);
+            for (int b = 0; b < 3 && !dt; ++b) Dd.jb[j][b] = (uint32_t*)(dbase + q.off_jb[j][b]);
             Dd.hist[j] = (unsigned long long*)(dbase + q.off_hist) + (size_t)j * (q.kmax + 1);
             Dd.brick0[j] = q.brick0 + (unsigned long long)j * q.bricks;
             Dd.tstamp[j] = stats ? (int32_t*)(dbase + q.off_tstamp[j]) : nullptr;
@@ -675,7 +710,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         Dd.tile0 = pack_tiles;
         Dd.stile0 = setup_tiles;
         pack_tiles += hdk::pack_tiles_of(P.W, P.H, P.D);
-        setup_tiles += hdk::setup_tiles_of(P.W, P.H, P.D, setup_mode, bxw, by, bz);
+        if (!dt) setup_tiles += hdk::setup_tiles_of(P.W, P.H, P.D, setup_mode, bxw, by, bz);
     }
 
     // ---- uploads ----------------------------------------------------------
@@ -726,7 +761,8 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (stime) cudaEventRecord(ctx->split.ev[1], sq);
     const bool spec = sh.kernel == 2;  // the blocked kernel reads first entries early (kSpecSlots zeroed slots)
     const int nz = spec ? (int)std::min<unsigned long long>(total_bricks, hdk::kSpecSlots) : 0;
-    e = hdk::launch_setup(ddesc, n, setup_tiles, split ? prep_sms : 0, djobs, dstates, dq[g0 % 3], dctl, g0, bxw, by, bz,
+    if (!dt)
+        e = hdk::launch_setup(ddesc, n, setup_tiles, split ? prep_sms : 0, djobs, dstates, dq[g0 % 3], dctl, g0, bxw, by, bz,
                           setup_mode, sq, dq[(g0 + 1) % 3], dq[(g0 + 2) % 3], nz);
     if (e == cudaSuccess && split) {
         // the dilation follows the set-up; the caller's stream follows the
@@ -759,13 +795,13 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     sp.map_h = pairs[0].H;
     sp.map_d = pairs[0].D;
     sp.g0 = g0;
-    sp.max_iters = kmax_all / sh.steps + 2;
+    sp.max_iters = dt ? 0 : kmax_all / sh.steps + 2;
     sp.stats = stats ? 1 : 0;
     sp.spread = sh.spread;
     sp.job_cache = (n == 1 && sh.kernel == 2) ? hdk::kJobCache : 0;  // a single pair's two jobs
     sp.spec_first = nz;  // slots of each queue the set-up zeroed
     sp.timeout_ns = ctx->opt.barrier_timeout_ns > 0 ? ctx->opt.barrier_timeout_ns : 10000000000LL;
-    const int occ = occupancy_of(ctx, solve_fn, sh.threads, sh.smem);
+    const int occ = dt ? 1 : occupancy_of(ctx, solve_fn, sh.threads, sh.smem);
     if (occ <= 0) return set_error(ctx, HD_ERR_CUDA, "dilation kernel cannot be made resident");
     const int per_sm = cps > 0 ? std::min(cps, occ) : occ;
     dim3 grid((split ? ctx->split.solve_sms[part] : ctx->sm_count) * per_sm), block(sh.threads);
@@ -779,7 +815,31 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     void* args[] = {&sp};
     if (timing) cudaEventRecord(ctx->ev[2], s);
     if (stime) cudaEventRecord(ctx->split.ev[3], sv);  // after the previous dilation and this set-up
-    e = cudaLaunchCooperativeKernel(solve_fn, grid, block, args, (size_t)sh.smem, sv);
+    if (dt) {
+        hdk::DtParams dp{};
+        dp.info = (const PairInfo*)(dbase + off_infos);
+        dp.packed[0] = (const uint32_t*)(dbase + plan[0].off_pa);
+        dp.packed[1] = (const uint32_t*)(dbase + plan[0].off_pb);
+        for (int j = 0; j < 2; ++j) {
+            dp.vol[j] = (uint32_t*)(dbase + plan[0].off_jb[j][0]);
+            dp.base[j] = (uint16_t*)(dbase + plan[0].off_jb[j][1]);
+            dp.rows[j] = (uint32_t*)(dbase + plan[0].off_jb[j][2]);
+            dp.hist[j] = (unsigned long long*)(dbase + plan[0].off_hist) + (size_t)j * (plan[0].kmax + 1);
+        }
+        dp.state = (hdk::DtState*)(dbase + off_states);  // the plane kernel zeroes it
+        dp.map[0] = ro.map_b;
+        dp.map[1] = ro.map_a;
+        dp.W = pairs[0].W;
+        dp.H = pairs[0].H;
+        dp.D = pairs[0].D;
+        dp.pitch = hdk::packed_pitch(pairs[0].W);
+        dp.kmax = plan[0].kmax;
+        dp.pct = pct;
+        dp.out = sp.out;
+        e = hdk::launch_dt(dp, split ? ctx->split.solve_sms[part] : ctx->sm_count, sv);
+    } else {
+        e = cudaLaunchCooperativeKernel(solve_fn, grid, block, args, (size_t)sh.smem, sv);
+    }
     if (e == cudaSuccess && stime) {
         cudaEventRecord(ctx->split.ev[4], sv);
         ctx->split.timed = true;
@@ -802,7 +862,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (async) {
         // the step counter moves past any step this launch can reach (its
         // stamps stay below the next call's steps)
-        ctx->g_next = g0 + sp.max_iters + 2;
+        if (!dt) ctx->g_next = g0 + sp.max_iters + 2;
         return HD_OK;
     }
 
@@ -827,7 +887,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (e != cudaSuccess) return cuda_fail(ctx, e, "dilation");
 
     const Ctl* hctl = (const Ctl*)(hbase + off_ctl);
-    ctx->g_next = std::max(ctx->g_next, hctl->g_end) + 2;
+    if (!dt) ctx->g_next = std::max(ctx->g_next, hctl->g_end) + 2;
     if (timing) {
         ctx->split.timed = false;
         hd_timings& T = ctx->last_timings;

@@ -67,6 +67,42 @@ struct PairDesc {
     long long stile0;              // first set-up tile of this pair
 };
 
+// Distance transform: sizes it takes (a plane's tiles of 64 rows in one CTA,
+// a column's segments and the distances' counters in shared memory).
+constexpr int kDtMaxW = 2048;
+constexpr int kDtMaxH = 512;
+constexpr int kDtMaxD = 1024;
+constexpr int kDtMaxSum = 2304;
+// Words of in-plane distances and number of tile bases, one direction.
+__host__ __device__ __forceinline__ long long dt_vol_words(int W, int H, int D) {
+    return (long long)D * ((H + 3) / 4) * ((W + 31) / 32) * 32;
+}
+__host__ __device__ __forceinline__ long long dt_bases(int W, int H, int D) {
+    return (long long)D * ((H + 63) / 64) * ((W + 31) / 32);
+}
+
+// Counters of the distance transform's second kernel.
+struct DtState {
+    unsigned int done;  // CTAs that have added their counts
+    int32_t hd[2];      // largest distance per direction
+};
+
+// One pair, by value (direction 0: A's distances at B's voxels, 1: the reverse).
+struct DtParams {
+    const PairInfo* info;
+    const uint32_t* packed[2];   // pa, pb
+    uint32_t* vol[2];            // in-plane distances as bytes, four rows per word: dt_vol_words
+    uint16_t* base[2];           // base of each 64-row x 32-column tile's bytes: dt_bases
+    uint32_t* rows[2];           // rows with target voxels, per word column, 32 rows and plane: 2 dt_bases
+    unsigned long long* hist[2]; // kmax + 1 counters
+    DtState* state;
+    int32_t* map[2];             // optional dense per-voxel distance maps (B's voxels, A's voxels)
+    int32_t W, H, D, pitch;      // pitch: packed_pitch(W)
+    int32_t kmax;
+    float pct;                   // robust HD percentile
+    hd_result* out;
+};
+
 // Packing and set-up split every pair into tiles; one launch covers the
 // tiles of all pairs.  Packing tiles are kPackTileWords words of the packed
 // volume (wxf * H * D words), set-up tiles kTileWords words of the domain

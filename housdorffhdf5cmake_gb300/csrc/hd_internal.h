@@ -31,6 +31,7 @@ struct PinnedArena {
 // Dilation kernel and brick geometry.
 //   kernel 1: one step per grid barrier, bricks bxw words x 32/bxw rows x bz planes
 //   kernel 2: `steps` steps per grid barrier, bricks 4 words x (32 - 2 steps) rows x bz planes
+//   kernel 3: distance transform (6-neighbour single pairs), no bricks
 struct Shape {  // default: the autotuner's choice on the 512x512x256, 512^3 and ragged-batch workloads
     int kernel = 2;
     int bxw = 4;
@@ -54,6 +55,8 @@ struct Shape {  // default: the autotuner's choice on the 512x512x256, 512^3 and
             by = hdk::tb_brick_rows(steps);
             threads = hdk::kTbWarps * 32;
             smem = hdk::kTbWarps * hdk::tb_warp_bytes(steps, bz);
+        } else if (kernel == 3) {
+            bxw = by = bz = steps = ctas_per_sm = order = spread = 0;
         } else {
             by = 32 / bxw;
             steps = 1;
@@ -200,8 +203,14 @@ const uint8_t* zero_copy_ptr(hd_context* ctx, const uint8_t* p);
 hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s, const RunOpts& ro,
                     hd_result* out);
 
-// Kernel and brick shape for a workload (options, then tuning table, then default).
-Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n);
+// Kernel and brick shape for a workload (options, then tuning table, then
+// default); dt: the distance transform may be chosen.
+Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n, bool dt);
+
+// Whether the distance transform takes these pairs, and whether a context's
+// options ask for the dilation loop instead.
+bool dt_takes(int se, const PairIn* pairs, int n);
+bool loop_asked(const hd_options& o);
 
 // Host stub of the persistent kernel of a shape (nullptr if not compiled in).
 const void* solve_fn_of(int se, const Shape& sh);

@@ -47,4 +47,9 @@ const void* solve_tb_kernel_ptr(int se, int steps, int bz);
 const void* solve_tb_kernel_ptr_se6(int steps, int bz);
 const void* solve_tb_kernel_ptr_se18(int steps, int bz);
 
+// Distance transform of one 6-neighbour pair (hd_dt.cu): both kernels, after
+// the packing, on a stream of `sms` SMs.  dt_fits: the sizes it takes.
+bool dt_fits(int W, int H, int D);
+cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s);
+
 }  // namespace hdk

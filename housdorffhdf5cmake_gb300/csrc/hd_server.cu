@@ -697,7 +697,7 @@ hd_status hd_server_create(hd_context* ctx, const hd_server_options* opt, hd_ser
         PairIn typical{nullptr, nullptr, 256, 256, 160, nullptr, nullptr};
         unsigned long long brick_bytes = ~0ull;
         for (int m = 0; m < 2; ++m) {
-            Shape sh = pick_shape(ctx, s->se, &typical, m == 0 ? 1 : 16);  // one pair / a batch-like mix
+            Shape sh = pick_shape(ctx, s->se, &typical, m == 0 ? 1 : 16, false);  // one pair / a batch-like mix
             const void* fn = solve_fn_of(s->se, sh);
             if (!fn) {
                 delete s;

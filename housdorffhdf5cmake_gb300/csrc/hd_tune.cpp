@@ -207,9 +207,15 @@ extern "C" hd_status hd_autotune(hd_context* ctx, const hd_pair_desc* pairs, int
             c.bz = bz;
             cands.push_back(c);
         }
+    if (dt_takes(se, in.data(), n) && !loop_asked(ctx->opt)) {
+        Shape c;
+        c.kernel = 3;
+        cands.push_back(c);
+    }
     std::vector<std::pair<double, Shape>> scored;
     for (Shape c : cands) {
         for (int cps : {0, 1}) {
+            if (c.kernel == 3 && cps) continue;  // no persistent grid
             c.ctas_per_sm = cps;
             c.order = c.spread = 0;
             c.finish();
@@ -225,6 +231,7 @@ extern "C" hd_status hd_autotune(hd_context* ctx, const hd_pair_desc* pairs, int
                      [](const std::pair<double, Shape>& x, const std::pair<double, Shape>& y) { return x.first < y.first; });
     const size_t top = std::min<size_t>(3, scored.size());
     for (size_t k = 0; k < top; ++k) {
+        if (scored[k].second.kernel == 3) continue;  // no queue
         for (int order : {0, 1})
             for (int spread : {0, 1}) {
                 if (!order && !spread) continue;  // measured in stage 1

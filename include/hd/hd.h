@@ -66,7 +66,7 @@ typedef enum hd_metric {
 typedef struct hd_result {
     int32_t hd;          /* max(hd_ab, hd_ba); -1 when status != HD_OK */
     int32_t iterations;  /* grid-barrier iterations of the device loop for this call (each runs one
-                            or more dilation steps, see hd_options.kernel) */
+                            or more dilation steps, see hd_options.kernel; 0: distance transform) */
     uint64_t sum_ab;
     uint64_t sum_ba;
     uint64_t n_a;
@@ -92,7 +92,9 @@ typedef struct hd_options {
                                     device can address them (default 1) */
     const char* tuning_table;    /* autotuner JSON table to load/store; NULL = none */
     int32_t record_timings;      /* record CUDA events around each kernel (hd_context_last_timings) */
-    int32_t kernel;              /* dilation kernel: 0 = tuned/default, 1 = one step per grid barrier
+    int32_t kernel;              /* dilation kernel: 0 = tuned/default (single pairs under HD_SE6 without any
+                                    option that asks for the dilation loop - a kernel, a brick shape, a cap on
+                                    its steps or waits - take an exact distance transform instead), 1 = one step per grid barrier
                                     (brick_x_words x 32/brick_x_words rows x brick_z planes),
                                     2 = temporally blocked (steps_per_barrier steps per barrier,
                                     4 words x (32 - 2 steps) rows x brick_z planes) */
@@ -112,7 +114,9 @@ typedef struct hd_timings {
     int32_t iterations;  /* grid-barrier iterations run by the persistent loop */
     int32_t grid_ctas;   /* CTAs of the persistent launch */
     int32_t brick_x_words, brick_z;
-    int32_t kernel;      /* 1 = one step per barrier, 2 = temporally blocked */
+    int32_t kernel;      /* 1 = one step per barrier, 2 = temporally blocked, 3 = distance
+                            transform (no loop: iterations, bricks and steps are 0; its
+                            two kernels count as solve_ms) */
     int32_t steps_per_barrier;
     int32_t brick_rows;
     int32_t dilation_partitions; /* pipelined entry on split SMs: dilations in

@@ -1,0 +1,93 @@
+"""The distance-transform path (6-neighbour single pairs by default) against
+the dilation loop (a context that asks for it) and the oracle, on every field
+but the barrier-loop count: sizes around its tiles (64 rows, 32 columns,
+groups of 4 words, segments of 16 planes, 16 segments per CTA) and the limits
+of the sizes it takes.  Integers: no tolerance."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("hd", "hd_ab", "hd_ba", "hd_robust", "sum_ab", "sum_ba", "n_a", "n_b", "n_a_not_b", "n_b_not_a", "status",
+        "avg_hd")
+
+
+def same(g, w, tag):
+    for k in KEYS:
+        assert g[k] == w[k] or (k == "avg_hd" and g[k] != g[k] and w[k] != w[k]), (tag, k, g, w)
+
+
+@pytest.fixture(scope="module")
+def loop(hd):
+    c = hd.Context(0, kernel=2)
+    yield c
+    c.close()
+
+
+def masks(rng, shape, kind):
+    a = np.zeros(shape, np.uint8)
+    b = np.zeros(shape, np.uint8)
+    D, H, W = shape
+    if kind == "corners":  # the longest distance of the volume
+        a[0, 0, 0] = 1
+        b[-1, -1, -1] = 1
+    elif kind == "sparse":
+        for m in (a, b):
+            for _ in range(3):
+                m[rng.integers(D), rng.integers(H), rng.integers(W)] = 1
+    elif kind == "slabs":  # empty planes and rows in between
+        a[0] = 1
+        b[:, H // 2, :] = 1
+        b[-1, :, W // 3] = 1
+    else:
+        a[...] = rng.random(shape) < 0.03
+        b[...] = rng.random(shape) < 0.01
+        a[D // 2, H // 2, W // 2] = b[D // 3, H // 3, W // 3] = 1
+    return a, b
+
+
+SHAPES = [(1, 1, 1), (15, 31, 33), (16, 32, 32), (17, 33, 31), (2, 63, 127), (3, 64, 128), (5, 65, 129), (33, 4, 161),
+          (31, 5, 96), (65, 127, 40), (8, 129, 260), (128, 3, 64), (129, 9, 30), (255, 7, 40), (256, 6, 33),
+          (257, 5, 65), (300, 66, 20), (3, 511, 40), (2, 512, 70), (9, 449, 33), (4, 3, 2048), (1024, 4, 33)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_tile_edges(hd, ctx, loop, oracle, shape):
+    rng = np.random.default_rng(sum(shape))
+    for kind in ("corners", "sparse", "slabs", "random"):
+        a, b = masks(rng, shape, kind)
+        da, db = torch.from_numpy(a).cuda(), torch.from_numpy(b).cuda()
+        g = ctx.compute(da, db, "se6")
+        same(g, loop.compute(da, db, "se6"), (shape, kind))
+        if a.size <= 70000:
+            same(g, {**oracle.bfs_pair(a, b, "se6"), "hd_robust": g["hd_robust"]}, (shape, kind, "oracle"))
+
+
+@pytest.mark.parametrize("shape", [(2, 513, 33), (1025, 3, 32), (2, 3, 2049)])
+def test_sizes_beyond_its_limits_take_the_loop(hd, ctx, loop, shape):
+    a, b = (torch.from_numpy(m).cuda() for m in masks(np.random.default_rng(1), shape, "corners"))
+    with hd.Context(0, record_timings=True) as c:
+        same(c.compute(a, b, "se6"), loop.compute(a, b, "se6"), shape)
+        assert c.last_timings()["kernel"] == 2
+
+
+def test_options_that_ask_for_the_loop(hd):
+    a, b = (torch.from_numpy(m).cuda() for m in masks(np.random.default_rng(2), (20, 40, 70), "random"))
+    for opts, kernel in (({}, 3), ({"kernel": 2}, 2), ({"brick_z": 8}, 2), ({"max_iterations": 500}, 2),
+                         ({"ctas_per_sm": 1}, 2), ({"barrier_timeout_ns": 10**9}, 2), ({"steps_per_barrier": 2}, 2)):
+        with hd.Context(0, record_timings=True, **opts) as c:
+            c.compute(a, b, "se6")
+            assert c.last_timings()["kernel"] == kernel, opts
+
+
+@pytest.mark.parametrize("shape", [(17, 33, 70), (40, 66, 129), (257, 5, 33)])
+def test_maps(hd, ctx, shape):
+    rng = np.random.default_rng(3)
+    with hd.Context(0, kernel=1) as one:
+        for kind in ("sparse", "random"):
+            a, b = (torch.from_numpy(m).cuda() for m in masks(rng, shape, kind))
+            r, ma, mb = ctx.distance_map(a, b, "se6")
+            w, wa, wb = one.distance_map(a, b, "se6")
+            same(r, w, (shape, kind))
+            assert torch.equal(ma, wa) and torch.equal(mb, wb)
