@@ -47,20 +47,12 @@ __device__ __forceinline__ uint32_t fg16(uint4 v, uint32_t pat) {
            ((fg4_top<kLabel>(v.z, pat) >> 20) & 0xF00u) | ((fg4_top<kLabel>(v.w, pat) >> 16) & 0xF000u);
 }
 
-__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
-    return v;
-}
-__device__ __forceinline__ int warp_min(int v) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, s));
-    return v;
-}
-__device__ __forceinline__ int warp_max(int v) {
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, s));
-    return v;
+// The same for 16 bytes that are all 0 or 1: each dot product weighs four
+// bytes with their bits.
+__device__ __forceinline__ uint32_t bits16(uint4 v) {
+    const uint32_t lo = __dp4a(v.y, 0x80402010u, __dp4a(v.x, 0x08040201u, 0u));
+    const uint32_t hi = __dp4a(v.w, 0x80402010u, __dp4a(v.z, 0x08040201u, 0u));
+    return lo | (hi << 8);
 }
 
 // The pair that owns work tile `tile` (first tiles increase with the pair
@@ -98,16 +90,22 @@ struct PackAcc {
     }
 };
 
+constexpr int kPackWarps = 8;  // (flush_acc's scratch holds this many)
+constexpr int kPackThreads = 32 * kPackWarps;
+
 // Block-wide reduction of the accumulators, then one set of atomics per CTA
 // (many CTAs update one PairInfo: per-warp atomics serialise on its lines).
-// Called by all threads of the CTA.
+// Called by all threads of the CTA.  A warp's counts fit in 32 bits: a volume
+// has fewer than 2^36 voxels, spread over hundreds of warps.
 __device__ __forceinline__ void flush_acc(const PairDesc& P, const PackAcc& acc) {
-    __shared__ unsigned long long s_cnt[3][8];
-    __shared__ int s_bb[6][8];
+    __shared__ unsigned s_cnt[3][kPackWarps];
+    __shared__ int s_bb[6][kPackWarps];
     const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    unsigned long long na = warp_sum_u64(acc.na), nb = warp_sum_u64(acc.nb), nab = warp_sum_u64(acc.nab);
-    int bb[6] = {warp_min(acc.wmin), warp_max(acc.wmax), warp_min(acc.ymin),
-                 warp_max(acc.ymax), warp_min(acc.rmin), warp_max(acc.rmax)};
+    const unsigned na = __reduce_add_sync(0xffffffffu, acc.na), nb = __reduce_add_sync(0xffffffffu, acc.nb),
+                   nab = __reduce_add_sync(0xffffffffu, acc.nab);
+    const int bb[6] = {__reduce_min_sync(0xffffffffu, acc.wmin), __reduce_max_sync(0xffffffffu, acc.wmax),
+                       __reduce_min_sync(0xffffffffu, acc.ymin), __reduce_max_sync(0xffffffffu, acc.ymax),
+                       __reduce_min_sync(0xffffffffu, acc.rmin), __reduce_max_sync(0xffffffffu, acc.rmax)};
     __syncthreads();  // earlier readers of the scratch are done
     if ((threadIdx.x & 31) == 0) {
         s_cnt[0][warp] = na;
@@ -117,238 +115,250 @@ __device__ __forceinline__ void flush_acc(const PairDesc& P, const PackAcc& acc)
         for (int i = 0; i < 6; ++i) s_bb[i][warp] = bb[i];
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    // one thread per value
+    PairInfo* const I = P.info;
+    if (threadIdx.x < 3) {
+        unsigned long long n = 0;
+        for (int w = 0; w < nwarps; ++w) n += s_cnt[threadIdx.x][w];
+        if (n) atomicAdd(threadIdx.x == 0 ? &I->n_a : (threadIdx.x == 1 ? &I->n_b : &I->n_ab), n);
+    } else if (threadIdx.x >= 32 && threadIdx.x < 38) {
+        const int i = threadIdx.x - 32;
+        int v = s_bb[i][0];
+        bool any = s_bb[1][0] >= 0;
         for (int w = 1; w < nwarps; ++w) {
-            na += s_cnt[0][w];
-            nb += s_cnt[1][w];
-            nab += s_cnt[2][w];
-            for (int i = 0; i < 6; i += 2) {
-                bb[i] = min(bb[i], s_bb[i][w]);
-                bb[i + 1] = max(bb[i + 1], s_bb[i + 1][w]);
-            }
+            v = (i & 1) ? max(v, s_bb[i][w]) : min(v, s_bb[i][w]);
+            any = any || s_bb[1][w] >= 0;
         }
-        PairInfo* I = P.info;
-        if (na) atomicAdd(&I->n_a, na);
-        if (nb) atomicAdd(&I->n_b, nb);
-        if (nab) atomicAdd(&I->n_ab, nab);
-        if (bb[1] >= 0) {
-            const int H = P.H;
-            atomicMin(&I->bb[0], bb[0]);
-            atomicMax(&I->bb[1], bb[1]);
-            atomicMin(&I->bb[2], bb[2]);
-            atomicMax(&I->bb[3], bb[3]);
-            atomicMin(&I->bb[4], bb[4] / H);
-            atomicMax(&I->bb[5], bb[5] / H);
+        if (i >= 4) v = v / P.H;
+        if (any) {
+            if (i & 1) atomicMax(&I->bb[i], v);
+            else atomicMin(&I->bb[i], v);
         }
     }
 }
 
-// Foreground bytes (nonzero, or equal to a nonzero label) among the 16 at p
-// that lie inside [lo, hi), as 16 bits (a mask's first and last 16-byte
-// chunks may stick out of it).  The byte loads
-// are predicated, not branched over, so all sixteen are in flight together.
-__device__ __noinline__ uint32_t chunk_bits_edge(const uint8_t* p, const uint8_t* lo, const uint8_t* hi, int label) {
-    uint32_t bits = 0;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const bool in = p + i >= lo && p + i < hi;
-        const uint8_t v = in ? __ldg(p + i) : (uint8_t)0;
-        const bool fg = label ? (in && v == (uint8_t)label) : (v != 0);
-        bits |= (fg ? 1u : 0u) << i;
-    }
-    return bits;
-}
-
-constexpr int kPackThreads = 256;
-constexpr int kPackGroups = 4;  // words per thread and tile: a warp packs 32 * kPackGroups consecutive words
-constexpr int kPackMinCtas = 2;  // resident CTAs per SM (register budget: 65536 / (kPackThreads * kPackMinCtas))
-static_assert(kPackTileWords == (kPackThreads / 32) * 32 * kPackGroups, "one tile = one span per warp");
+constexpr int kPackCtas = 2;            // resident CTAs per SM
+constexpr int kWords = 4;               // words per lane and span
+constexpr int kSpan = 32 * kWords;      // words a warp packs at a time
+constexpr int kRounds = 2 * kWords;     // 16-byte chunks per lane and mask
+constexpr int kSpanChunks = 2 * kSpan;  // chunks of a span (one more when unaligned)
+constexpr int kBitWords = kSpan + 4;    // words of a span's bit stream
+static_assert(kPackTileWords == kPackWarps * kSpan, "one tile = one span per warp");
 
 // Constants of one pair's packing walk (taken when a CTA's run of tiles
 // enters the pair).
 struct PackWalk {
     const uint8_t* src[2];
-    const uint8_t* end[2];
+    size_t nbytes;              // bytes of a mask
     unsigned wxf, W, H, total;  // words per row, bytes per row, rows per plane, words of the pair
-    unsigned pitch, npad;       // packed row pitch (words): wxf rounded up to 4, npad zero words
+    unsigned pitch;             // packed row pitch (words): wxf rounded up to 4, zero words in between
     unsigned dq, dr;            // 32 words = dq rows + dr words
-    uint32_t tail;              // valid bits of a row's last word
+    unsigned tq, tr;            // from a span's end to the warp's next span = tq rows + tr words
+};
+
+// One warp's span of a pair: words t0 .. t0 + kSpan - 1 of both masks (word t =
+// row r, word w of the row, stored at r * pitch + w), the bytes that hold them
+// and the 16-byte chunks that cover these.
+struct PackSpan {
+    unsigned cnt;            // words of the span
+    size_t lo;               // first byte
+    unsigned sh[2], nch[2];  // per mask: bytes of the first chunk before it, chunks
 };
 
 __device__ __forceinline__ PackWalk make_walk(const PairDesc& P) {
     PackWalk k;
-    const size_t nbytes = (size_t)P.W * P.H * P.D;
     k.src[0] = P.a;
     k.src[1] = P.b;
-    k.end[0] = P.a + nbytes;
-    k.end[1] = P.b + nbytes;
+    k.nbytes = (size_t)P.W * P.H * P.D;
     k.wxf = (unsigned)P.wxf;
     k.pitch = (unsigned)packed_pitch(P.W);
-    k.npad = k.pitch - k.wxf;
     k.W = (unsigned)P.W;
     k.H = (unsigned)P.H;
     k.total = (unsigned)((long long)P.wxf * P.H * P.D);  // < 2^31 words
     k.dq = 32u / k.wxf;
     k.dr = 32u - k.dq * k.wxf;
-    const unsigned tb = k.W - 32u * (k.wxf - 1);
-    k.tail = tb >= 32 ? 0xffffffffu : ((1u << tb) - 1u);
+    k.tq = ((unsigned)kPackTileWords - kSpan) / k.wxf;
+    k.tr = ((unsigned)kPackTileWords - kSpan) - k.tq * k.wxf;
     return k;
 }
 
-// One tile of a pair, any width, alignment or memory kind (device or
-// host-mapped).  Warp v packs words w_lo + 128 v + 32 i + lane (i < 4) of
-// both masks (word t = row r, word w is stored at r * pitch + w; the row's
-// last word also zeroes the padding after it).  Word t holds the mask bytes [o, o + n) with
-// o = r W + 32 w, n = min(32, W - 32 w); with q = o rounded down to 16 and
-// s = o - q they lie in the 16-byte chunks at q, q + 16 and, if s + n > 32,
-// q + 32.  Rows are contiguous, so word t + 1 starts at o + n, and when
-// s + n > 32 (then 32 < s + n <= 47) its first chunk is the one at q + 32.
-// Each thread therefore loads two chunks per word and takes the third from
-// the thread that holds word t + 1: the next lane, or lane 0's next group
-// for lane 31.  Only lane 31's last group (and a pair's last word) loads a
-// third chunk.  All loads are issued before any is used, as streaming loads.
-// kEdge = false: every word of the tile is in the pair and every chunk it
-// touches lies inside the masks (see pack_kernel); kEdge = true: both are
-// checked word by word.
-template <bool kEdge, bool kLabel>
-__device__ __forceinline__ void pack_tile(const PairDesc& P, const PackWalk& k, long long tile_in_pair,
-                                          PackAcc& acc, int label, uint32_t pat) {
+// Locates the span of words t0 ..: row r and word w are its first word's.
+__device__ __forceinline__ PackSpan locate(const PackWalk& k, unsigned t0, unsigned r, unsigned w) {
+    PackSpan n;
+    n.cnt = min((unsigned)kSpan, k.total - t0);
+    n.lo = (size_t)r * k.W + 32u * w;
+    // the last word: cnt - 1 words on
+    const unsigned lw = w + n.cnt - 1u, q = lw / k.wxf, x = lw - q * k.wxf;
+    const unsigned len = q * k.W + 32u * x - 32u * w + min(32u, k.W - 32u * x);
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        n.sh[m] = (unsigned)((uintptr_t)(k.src[m] + n.lo) & 15u);
+        n.nch[m] = (n.sh[m] + len + 15u) >> 4;
+    }
+    return n;
+}
+
+// Issues the loads of a span's chunks of mask m (streaming).  Lanes past the
+// last chunk, and chunks that stick out of the mask (the first or last of a
+// pair), repeat a neighbouring one: those bits are not used, or written by
+// put_bits byte by byte.  x: a lane's byte of the one chunk more that an unaligned span may have.
+__device__ __forceinline__ void load_chunks(const PackWalk& k, const PackSpan& n, int m, uint4 (&c)[kRounds], unsigned& x) {
     const int lane = threadIdx.x & 31;
-    const unsigned t0 = (unsigned)(tile_in_pair * kPackTileWords) + (threadIdx.x >> 5) * (32u * kPackGroups) + lane;
-    unsigned r = t0 / k.wxf, w = t0 - r * k.wxf;
-    unsigned y = r % k.H;
-    uint4 c[kPackGroups][2][2];
-    uint4 c3[2] = {make_uint4(0u, 0u, 0u, 0u), make_uint4(0u, 0u, 0u, 0u)};
-    unsigned rr[kPackGroups], ww[kPackGroups], yy[kPackGroups];
+    const uint8_t* const q = k.src[m] + n.lo - n.sh[m];
+    const bool head = n.lo < n.sh[m], tail = n.lo - n.sh[m] + 16ull * n.nch[m] > k.nbytes && !(head && n.nch[m] == 1u);
+    const int c_lo = head ? 1 : 0, c_hi = (int)n.nch[m] - (tail ? 2 : 1);  // first and last chunk inside
+    if (c_hi >= c_lo) {  // uniform
 #pragma unroll
-    for (int i = 0; i < kPackGroups; ++i) {
-        rr[i] = r;
-        ww[i] = w;
-        yy[i] = y;
-        const unsigned t = t0 + 32u * i;
-        const size_t off = (size_t)r * k.W + 32u * w;
-        const bool valid = !kEdge || t < k.total;
-        const unsigned nbits = w + 1 == k.wxf ? k.W - 32u * w : 32u;
-        const bool own3 = (i == kPackGroups - 1 && lane == 31) || (kEdge && t + 1 == k.total);
+        for (int i = 0; i < kRounds; ++i)
+            c[i] = __ldcs(reinterpret_cast<const uint4*>(q) + max(min(32 * i + lane, c_hi), c_lo));
+    }
+    x = 0u;
+    if (n.nch[m] > kSpanChunks) {  // uniform
+        const size_t o = n.lo - n.sh[m] + 16u * kSpanChunks + lane;
+        if (lane < 16 && o < k.nbytes) x = __ldg(k.src[m] + o);
+    }
+}
+
+// Foreground flags of the span's chunks of mask m, as a stream of bits.
+template <bool kLabel>
+__device__ __forceinline__ void put_bits(const PackWalk& k, const PackSpan& n, int m, const uint4 (&c)[kRounds], unsigned x,
+                                         unsigned label, uint32_t* s_bits) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t pat = label * 0x01010101u;
+    uint16_t* const s = reinterpret_cast<uint16_t*>(s_bits);
+    bool general = kLabel;
+    if constexpr (!kLabel) {
+        uint32_t any = 0u;
 #pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const uint8_t* x = k.src[m] + off;
-            const uint8_t* q = (const uint8_t*)((uintptr_t)x & ~(uintptr_t)15);
-            const unsigned sh = (unsigned)((uintptr_t)x & 15);
-            if (!kEdge || (valid && q >= k.src[m] && q + 48 <= k.end[m])) {
-                c[i][m][0] = __ldcs(reinterpret_cast<const uint4*>(q));
-                c[i][m][1] = __ldcs(reinterpret_cast<const uint4*>(q) + 1);
-                if (own3 && sh + nbits > 32) c3[m] = __ldcs(reinterpret_cast<const uint4*>(q) + 2);
-            } else {
-                c[i][m][0] = c[i][m][1] = make_uint4(0u, 0u, 0u, 0u);
+        for (int i = 0; i < kRounds; ++i) any |= c[i].x | c[i].y | c[i].z | c[i].w;
+        general = __any_sync(0xffffffffu, (any & 0xfefefefeu) != 0u);
+    }
+    if (general) {
+#pragma unroll
+        for (int i = 0; i < kRounds; ++i) s[32 * i + lane] = (uint16_t)fg16<kLabel>(c[i], pat);
+    } else {
+#pragma unroll
+        for (int i = 0; i < kRounds; ++i) s[32 * i + lane] = (uint16_t)bits16(c[i]);
+    }
+    if (n.nch[m] > kSpanChunks) {  // uniform
+        const unsigned bits = __ballot_sync(0xffffffffu, lane < 16 && (kLabel ? x == label : x != 0u));
+        if (lane == 0) s[kSpanChunks] = (uint16_t)bits;
+    }
+    const bool head = n.lo < n.sh[m], tail = n.lo - n.sh[m] + 16ull * n.nch[m] > k.nbytes;
+    if (head || tail) {  // uniform: a chunk sticks out of the mask
+#pragma unroll 1
+        for (int e = 0; e < 2; ++e) {
+            __syncwarp();
+            if (!(e ? tail : head)) continue;
+            const unsigned ch = e ? n.nch[m] - 1u : 0u;
+            const size_t o = n.lo + 16u * ch + lane;  // byte of the mask, plus sh
+            const bool in = lane < 16 && o >= n.sh[m] && o - n.sh[m] < k.nbytes;
+            const unsigned v = in ? __ldg(k.src[m] + (o - n.sh[m])) : 0u;
+            const unsigned bits = __ballot_sync(0xffffffffu, in && (kLabel ? v == label : v != 0u));
+            if (lane == 0) s[ch] = (uint16_t)bits;
+        }
+    }
+}
+
+// Cuts the span's words out of the bit streams (a row starts at any bit).
+// (r, w, y): this lane's first word, advanced past the span.
+__device__ __forceinline__ void put_words(const PairDesc& P, const PackWalk& k, const PackSpan& n, unsigned& r,
+                                          unsigned& w, unsigned& y, PackAcc& acc, const uint32_t (*s_bits)[kBitWords]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+        if (32u * i + lane < n.cnt) {
+            const bool last = w + 1u == k.wxf;
+            const unsigned nbits = last ? k.W - 32u * w : 32u;
+            const uint32_t mask = 0xffffffffu >> (32u - nbits);
+            const unsigned d = (unsigned)((size_t)r * k.W + 32u * w - n.lo);
+            uint32_t out[2];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const unsigned o = d + n.sh[m];
+                out[m] = __funnelshift_r(s_bits[m][o >> 5], s_bits[m][(o >> 5) + 1], o & 31u) & mask;
             }
+            const size_t o = (size_t)r * k.pitch + w;
+            P.pa[o] = out[0];
+            P.pb[o] = out[1];
+            if (last)  // the row's last word also writes its padding (up to 3 words)
+#pragma unroll 1
+                for (unsigned x = k.wxf; x < k.pitch; ++x) P.pa[o + 1u + x - k.wxf] = P.pb[o + 1u + x - k.wxf] = 0u;
+            acc.add(out[0], out[1], (int)r, (int)y, (int)w);
         }
-        // next group: 32 words on
-        w += k.dr;
-        unsigned dy = k.dq;
-        if (w >= k.wxf) {
-            w -= k.wxf;
-            ++dy;
-        }
+        w += k.dr;  // 32 words on
+        const unsigned dy = k.dq + (w >= k.wxf ? 1u : 0u);
+        if (w >= k.wxf) w -= k.wxf;
         r += dy;
         y += dy;
         if (y >= k.H) y %= k.H;
-    }
-    // mask bits of each word's first two chunks
-    uint32_t lo[kPackGroups][2];
-#pragma unroll
-    for (int i = 0; i < kPackGroups; ++i) {
-        const size_t off = (size_t)rr[i] * k.W + 32u * ww[i];
-        const unsigned t = t0 + 32u * i;
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            if (kEdge) {
-                const uint8_t* q = (const uint8_t*)((uintptr_t)(k.src[m] + off) & ~(uintptr_t)15);
-                if (t < k.total && !(q >= k.src[m] && q + 48 <= k.end[m])) {
-                    lo[i][m] = chunk_bits_edge(q, k.src[m], k.end[m], label) |
-                               (chunk_bits_edge(q + 16, k.src[m], k.end[m], label) << 16);
-                    continue;
-                }
-            }
-            lo[i][m] = fg16<kLabel>(c[i][m][0], pat) | (fg16<kLabel>(c[i][m][1], pat) << 16);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < kPackGroups; ++i) {
-        const unsigned t = t0 + 32u * i;
-        const unsigned wi = ww[i];
-        const size_t off = (size_t)rr[i] * k.W + 32u * wi;
-        const bool last = wi + 1 == k.wxf;
-        const unsigned nbits = last ? k.W - 32u * wi : 32u;
-        const bool own3 = (i == kPackGroups - 1 && lane == 31) || (kEdge && t + 1 == k.total);
-        uint32_t out[2];
-#pragma unroll
-        for (int m = 0; m < 2; ++m) {
-            const unsigned sh = (unsigned)((uintptr_t)(k.src[m] + off) & 15);
-            uint32_t hi = __shfl_down_sync(0xffffffffu, lo[i][m] & 0xffffu, 1);
-            if (i + 1 < kPackGroups) {
-                const uint32_t wrap = __shfl_sync(0xffffffffu, lo[i + 1 < kPackGroups ? i + 1 : i][m] & 0xffffu, 0);
-                if (lane == 31) hi = wrap;
-            }
-            if (own3 && sh + nbits > 32) {  // rare: the warp's last word, the pair's last word
-                if (kEdge) {
-                    const uint8_t* q = (const uint8_t*)((uintptr_t)(k.src[m] + off) & ~(uintptr_t)15);
-                    hi = (q >= k.src[m] && q + 48 <= k.end[m]) ? fg16<kLabel>(c3[m], pat)  // loaded above
-                                                                : chunk_bits_edge(q + 32, k.src[m], k.end[m], label);
-                } else {
-                    hi = fg16<kLabel>(c3[m], pat);
-                }
-            }
-            out[m] = __funnelshift_r(lo[i][m], hi, sh) & (last ? k.tail : 0xffffffffu);
-        }
-        if (!kEdge || t < k.total) {
-            const size_t o = (size_t)rr[i] * k.pitch + wi;
-            P.pa[o] = out[0];
-            P.pb[o] = out[1];
-            if (last && k.npad) {  // the row's last word also writes its padding (1-3 words)
-                P.pa[o + 1] = P.pb[o + 1] = 0u;
-                if (k.npad > 1) P.pa[o + 2] = P.pb[o + 2] = 0u;
-                if (k.npad > 2) P.pa[o + 3] = P.pb[o + 3] = 0u;
-            }
-            acc.add(out[0], out[1], (int)rr[i], (int)yy[i], (int)wi);
-        }
     }
 }
 
 // Packing launch: one wave of resident CTAs, each over a contiguous run of
 // tiles (a run crosses few pairs, so the pair lookup and the accumulator
-// flush are rare).  A tile takes the checked path if it is a pair's first
-// tile or reaches within 48 words of the pair's end: every other word then
-// starts at byte >= kPackTileWords (each word holds >= 1 byte) and ends >= 48
-// bytes before the mask's end, so its three chunks lie inside the mask.
+// flush are rare); a tile is one span per warp, of any width, alignment or
+// memory kind (device or host-mapped).  Rows are contiguous in the mask, so a
+// span is one run of bytes: it is read in the 16-byte chunks that cover it,
+// each once and coalesced, their foreground flags go to shared memory as a
+// stream of bits (masks of zeros and ones, by a vote over the span, with one
+// dot product per four bytes), and the words are cut out of that stream.
+// Bound by HBM for large volumes (8 KB in flight per warp, 128 KB per SM) and
+// by its own start for small ones, where short code counts.  Between events,
+// against one 16-byte chunk pair per word with shuffles for the third chunk
+// (80 KB of code): 512^3 52 against 55.5 us, 512x512x256 27 against 29.5 us,
+// 301x287x173 with a label 15 against 19 us, 64^3 8.7 against 14.7 us, 48
+// patches 18 against 27 us, 256 ragged pairs 1.025 against 1.040 ms (with each
+// warp on a contiguous share of the CTA's run 1.043 ms).  64-word spans at 3
+// CTAs per SM were 14 % slower at 512^3, with the next span's loads issued
+// between the two masks' 37 %.
 template <bool kLabel>
-__global__ void __launch_bounds__(kPackThreads, kPackMinCtas) pack_kernel(const PairDesc* __restrict__ descs, int npairs,
+__global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const PairDesc* __restrict__ descs, int npairs,
                                                                long long ntiles, int label) {
-    const uint32_t pat = (uint32_t)label * 0x01010101u;
-    PackAcc acc;
-    PackWalk walk;
-    int pi = -1;
+    __shared__ uint32_t s_bits_all[kPackWarps][2][kBitWords];
     const long long per = (ntiles + gridDim.x - 1) / gridDim.x;
-    const long long t_lo = (long long)blockIdx.x * per, t_hi = min(ntiles, t_lo + per);
-    for (long long tile = t_lo; tile < t_hi; ++tile) {
-        // tiles only increase: walk forward to the owning pair
-        int np = pi < 0 ? pair_of_tile(descs, npairs, tile, false) : pi;
-        while (np + 1 < npairs && descs[np + 1].tile0 <= tile) ++np;
-        if (np != pi) {
-            if (pi >= 0) {
-                flush_acc(descs[pi], acc);
-                acc = PackAcc();
-            }
-            pi = np;
-            walk = make_walk(descs[pi]);
+    long long tile = (long long)blockIdx.x * per;
+    const long long t_hi = min(ntiles, tile + per);
+    if (tile >= t_hi) return;
+    int pi = npairs == 1 ? 0 : pair_of_tile(descs, npairs, tile, false);
+    uint32_t (*const s_bits)[kBitWords] = s_bits_all[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+#pragma unroll 1
+    for (;;) {  // the pairs of this CTA's run
+        const PairDesc& P = descs[pi];
+        const PackWalk k = make_walk(P);
+        const long long end = pi + 1 < npairs ? min(t_hi, descs[pi + 1].tile0) : t_hi;
+        PackAcc acc;
+        unsigned t0 = (unsigned)((tile - P.tile0) * kPackTileWords) + (threadIdx.x >> 5) * kSpan;
+        const unsigned t1 = min((unsigned)((end - P.tile0) * kPackTileWords), k.total);
+        unsigned r = (t0 + lane) / k.wxf;
+        unsigned w = t0 + lane - r * k.wxf;
+        unsigned y = r % k.H;
+#pragma unroll 1
+        for (; t0 < t1; t0 += (unsigned)kPackTileWords) {
+            const PackSpan n = locate(k, t0, __shfl_sync(0xffffffffu, r, 0), __shfl_sync(0xffffffffu, w, 0));
+            uint4 c[2][kRounds];
+            unsigned x[2];
+#pragma unroll
+            for (int m = 0; m < 2; ++m) load_chunks(k, n, m, c[m], x[m]);
+            __syncwarp();  // the last span's bits have been read
+#pragma unroll
+            for (int m = 0; m < 2; ++m) put_bits<kLabel>(k, n, m, c[m], x[m], (unsigned)label, s_bits[m]);
+            __syncwarp();
+            put_words(P, k, n, r, w, y, acc, s_bits);
+            // this warp's span of the next tile
+            w += k.tr;
+            const unsigned dr = k.tq + (w >= k.wxf ? 1u : 0u);
+            if (w >= k.wxf) w -= k.wxf;
+            r += dr;
+            y += dr;
+            if (y >= k.H) y %= k.H;
         }
-        const long long tp = tile - descs[pi].tile0;
-        if (tp >= 1 && (tp + 1) * kPackTileWords + 48 <= (long long)walk.total)
-            pack_tile<false, kLabel>(descs[pi], walk, tp, acc, label, pat);
-        else
-            pack_tile<true, kLabel>(descs[pi], walk, tp, acc, label, pat);
+        flush_acc(P, acc);
+        tile = end;
+        if (tile >= t_hi) break;
+        ++pi;
     }
-    if (pi >= 0) flush_acc(descs[pi], acc);
 }
 
 struct Domain {
