@@ -138,13 +138,37 @@ def _ready(*bufs):
         torch.cuda.current_stream().synchronize()
 
 
+def _import_torch():
+    global _torch
+    if _torch is None:
+        try:
+            import torch
+            _torch = torch
+        except ImportError:
+            pass
+    return _torch
+
+
 def _current_stream_ptr():
     """torch's current stream as a cudaStream_t for the C ABI.  torch's
     default stream is the legacy NULL stream, which the C ABI would read as
     "the context's own stream": pass the cudaStreamLegacy handle (0x1)
     instead, so the work is ordered with torch's."""
-    import torch
-    return torch.cuda.current_stream().cuda_stream or 0x1
+    return _import_torch().cuda.current_stream().cuda_stream or 0x1
+
+
+def _plain_pair(a, b):
+    """(pointer a, pointer b, W, H, D) of two contiguous 3-D uint8 CUDA tensors
+    of one shape, the form most calls pass; None for anything else (_Buf
+    looks at those)."""
+    T = _import_torch()
+    if (T is None or type(a) is not T.Tensor or type(b) is not T.Tensor or a.dtype is not T.uint8
+            or b.dtype is not T.uint8 or not (a.is_cuda and b.is_cuda and a.is_contiguous() and b.is_contiguous())):
+        return None
+    sh = a.shape
+    if len(sh) != 3 or sh != b.shape:
+        return None
+    return a.data_ptr(), b.data_ptr(), sh[2], sh[1], sh[0]
 
 
 class Context:
@@ -224,6 +248,14 @@ class Context:
         """HD of one pair.  Host inputs go through hd_compute_u8 (copies or
         zero-copy reads inside the call); CUDA tensors through
         hd_compute_u8_device on `stream` (default: torch's current stream)."""
+        plain = _plain_pair(a, b)
+        if plain is not None:
+            r = N.HdResult()
+            s = _current_stream_ptr() if stream is None else stream
+            code = N.load().hd_compute_u8_device(self._h, *plain, metric_code(metric), s, ctypes.byref(r))
+            if code != HD_OK:
+                _check(code, self._h)
+            return r.as_dict()
         A, B = _Buf(a), _Buf(b)
         if (A.W, A.H, A.D) != (B.W, B.H, B.D):
             raise ValueError("mask shapes differ")
@@ -252,6 +284,13 @@ class Context:
         RESULT_BYTES bytes (allocated if None), once the stream reaches it;
         decode it with result_from_bytes(out.cpu()).  Host masks must stay
         unchanged until then.  Calls on one context must stay on one stream."""
+        plain = _plain_pair(a, b)
+        if plain is not None and out is not None:
+            s = _current_stream_ptr() if stream is None else stream
+            code = N.load().hd_compute_u8_device_async(self._h, *plain, metric_code(metric), s, out.data_ptr())
+            if code != HD_OK:
+                _check(code, self._h, allow_empty=False)
+            return out
         import torch
         A, B = _Buf(a), _Buf(b)
         if (A.W, A.H, A.D) != (B.W, B.H, B.D):
@@ -280,6 +319,14 @@ class Context:
         the dilation, which the stream waits for only at flush(), so the
         context keeps a reference to it until then.  Calls on one context
         must stay on one stream."""
+        plain = _plain_pair(a, b)
+        if plain is not None and out is not None:
+            s = _current_stream_ptr() if stream is None else stream
+            code = N.load().hd_compute_u8_device_pipelined(self._h, *plain, metric_code(metric), s, out.data_ptr())
+            if code != HD_OK:
+                _check(code, self._h, allow_empty=False)
+            self._unflushed.append(out)
+            return out
         import torch
         A, B = _Buf(a), _Buf(b)
         if (A.W, A.H, A.D) != (B.W, B.H, B.D):
@@ -393,13 +440,7 @@ class PreparedBatch:
         n = len(pairs)
         keep, rows = [], []
         any_dev = False
-        global _torch
-        if _torch is None:
-            try:
-                import torch
-                _torch = torch
-            except ImportError:
-                pass
+        _import_torch()
         T = _torch.Tensor if _torch is not None else None
         u8 = _torch.uint8 if _torch is not None else None
         for i, (a, b) in enumerate(pairs):

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 import threading
 
 from . import build as _build
@@ -58,7 +59,12 @@ class HdResult(ctypes.Structure):
     ]
 
     def as_dict(self) -> dict:
-        return {f: getattr(self, f) for f, _ in self._fields_}
+        return dict(zip(_RESULT_NAMES, _RESULT_STRUCT.unpack_from(self)))
+
+
+_RESULT_NAMES = tuple(f for f, _ in HdResult._fields_)
+_RESULT_STRUCT = struct.Struct("=ii6Qd4i")  # the fields in order, without padding
+assert _RESULT_STRUCT.size == ctypes.sizeof(HdResult)
 
 
 class HdOptions(ctypes.Structure):
@@ -148,6 +154,8 @@ def lib_path() -> str:
 def load(build_if_missing: bool = True) -> ctypes.CDLL:
     """Load libhd_gb300.so (building it first if it is absent and nvcc exists)."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

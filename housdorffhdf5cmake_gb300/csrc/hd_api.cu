@@ -484,9 +484,6 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     const size_t off_descs = take(sizeof(PairDesc) * n);
     const size_t upload_bytes = cur;           // [ctl .. descs]
     const size_t off_jobs = take(sizeof(Job) * 2 * n);
-    // results decoded by the persistent launch (synchronous calls read them
-    // back; asynchronous ones write to the caller's array instead)
-    const size_t off_out = take(sizeof(hd_result) * n);
     size_t hist_words = 0;
     unsigned long long total_bricks = 0;
     int kmax_all = 0;
@@ -539,6 +536,8 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         }
     }
     const size_t total_bytes = cur;
+    // A single pair's descriptor goes to the kernels by value: no upload.
+    const bool direct = n == 1;
     const size_t pinned_bytes = upload_bytes + sizeof(hd_result) * n + (stats ? sizeof(uint64_t) * hist_words : 0);
 
     // Pipelined single pairs of up to 2^26 voxels run on split SMs: their
@@ -614,29 +613,36 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         ctx->stamp_slots = want;
         ctx->g_next = 1;
     }
-    int slot = -1;
-    if (async) {
-        // first asynchronous call: every staging buffer and event at once
-        // (pinned allocations are slow; later calls should not meet one)
-        if (!ctx->async_done[0]) {
-            for (int i = 0; i < hd_context::kAsyncSlots && e == cudaSuccess; ++i) {
-                e = cudaEventCreateWithFlags(&ctx->async_done[i], cudaEventDisableTiming);
-                if (e == cudaSuccess) e = ctx->async_stage[i].ensure(std::max<size_t>(upload_bytes, 1 << 16));
-            }
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "staging buffers");
-        }
-        // a staging buffer whose previous upload has run
-        slot = ctx->async_next;
-        ctx->async_next = (ctx->async_next + 1) % hd_context::kAsyncSlots;
-        e = cudaEventSynchronize(ctx->async_done[slot]);
-        if (e == cudaSuccess) e = ctx->async_stage[slot].ensure(upload_bytes);
-    } else {
+    {
+        // not under stream capture: the workspace and the step counter belong
+        // to the calls, not to a replay
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        e = cudaStreamIsCapturing(s, &cap);
+        if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "stream");
+    }
+    if (!async) {
         e = ctx->pinned.ensure(pinned_bytes);
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "pinned staging");
+    PairInfo* dinfos = nullptr;  // a single pair's counts, in the workspace's own place
+    if (direct) {
+        constexpr size_t kStride = 256;
+        if (!ctx->infos.ptr) {
+            e = ctx->infos.ensure(kStride * hd_context::Split::kWorkspaces);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "device workspace");
+        }
+        dinfos = (PairInfo*)((char*)ctx->infos.ptr + kStride * ws);
+        if (!ctx->info_clean[ws]) {
+            const PairInfo start = hdk::pair_info_start();
+            e = cudaMemcpyAsync(dinfos, &start, sizeof start, cudaMemcpyHostToDevice, sq);
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "start values");
+        }
+        ctx->info_clean[ws] = false;  // until this call's launches are complete
+    }
 
     char* dbase = (char*)arena.ptr;
-    char* hbase = (char*)(async ? ctx->async_stage[slot].ptr : ctx->pinned.ptr);
+    char* hbase = async ? nullptr : (char*)ctx->pinned.ptr;  // (asynchronous calls are single pairs)
     const int g0 = ctx->g_next;
     long long pack_tiles = 0, setup_tiles = 0;
     // blocked kernel: a single pair reads the packed masks in place unless
@@ -677,15 +683,14 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     }
 
     // ---- host-side descriptors ------------------------------------------
-    std::memset(hbase, 0, upload_bytes);
-    PairInfo* hinfo = (PairInfo*)(hbase + off_infos);
-    PairDesc* hdesc = (PairDesc*)(hbase + off_descs);
+    PairDesc one{};
+    if (!direct) std::memset(hbase, 0, upload_bytes);
+    PairInfo* hinfo = direct ? nullptr : (PairInfo*)(hbase + off_infos);
+    PairDesc* hdesc = direct ? &one : (PairDesc*)(hbase + off_descs);
     for (int i = 0; i < n; ++i) {
         const PairIn& P = pairs[i];
         const PairPlan& q = plan[i];
-        PairInfo& I = hinfo[i];
-        I.bb[0] = I.bb[2] = I.bb[4] = 0x7fffffff;
-        I.bb[1] = I.bb[3] = I.bb[5] = -1;
+        if (hinfo) hinfo[i] = hdk::pair_info_start();
         PairDesc& Dd = hdesc[i];
         Dd.a = P.host_a ? (staged[0] ? staged[0] : (const uint8_t*)(dbase + q.off_in_a)) : P.a;
         Dd.b = P.host_b ? (staged[1] ? staged[1] : (const uint8_t*)(dbase + q.off_in_b)) : P.b;
@@ -706,7 +711,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         Dd.aligned = ((((uintptr_t)Dd.a) | ((uintptr_t)Dd.b)) & 15) == 0;
         Dd.kmax = q.kmax;
         Dd.job0 = 2 * i;
-        Dd.info = (PairInfo*)(dbase + off_infos) + i;
+        Dd.info = direct ? dinfos : (PairInfo*)(dbase + off_infos) + i;
         Dd.tile0 = pack_tiles;
         Dd.stile0 = setup_tiles;
         pack_tiles += hdk::pack_tiles_of(P.W, P.H, P.D);
@@ -714,9 +719,10 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     }
 
     // ---- uploads ----------------------------------------------------------
-    e = cudaMemcpyAsync(dbase, hbase, upload_bytes, cudaMemcpyHostToDevice, sq);
-    if (e == cudaSuccess && async) e = cudaEventRecord(ctx->async_done[slot], sq);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "descriptor upload");
+    if (!direct) {
+        e = cudaMemcpyAsync(dbase, hbase, upload_bytes, cudaMemcpyHostToDevice, sq);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "descriptor upload");
+    }
     for (int i = 0; i < n && mb < 0; ++i) {
         const size_t nb = (size_t)pairs[i].W * pairs[i].H * pairs[i].D;
         if (pairs[i].host_a) {
@@ -742,16 +748,17 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     // ---- pack, set-up -----------------------------------------------------
     // one CTA per tile up to 8 per SM, then striding
     const int grid_pack = (int)std::min<long long>(std::max(prep_sms * 8, 1), pack_tiles);
-    const PairDesc* ddesc = (const PairDesc*)(dbase + off_descs);
+    PairDesc* const ddesc = (PairDesc*)(dbase + off_descs);
+    Ctl* dctl = (Ctl*)(dbase + off_ctl);
     const bool timing = ctx->opt.record_timings != 0 && ctx->ev[0] != nullptr && !async;
     if (timing) cudaEventRecord(ctx->ev[0], s);
     // the split path times its phases on the streams they run on
     const bool stime = split && ctx->opt.record_timings != 0 && ctx->split.ev[0] != nullptr;
     if (stime) cudaEventRecord(ctx->split.ev[0], sq);
-    e = hdk::launch_pack(ddesc, n, pack_tiles, grid_pack, ctx->opt.label, split ? prep_sms : 0, sq);
+    e = hdk::launch_pack(direct ? nullptr : ddesc, n, pack_tiles, grid_pack, ctx->opt.label, split ? prep_sms : 0, sq,
+                         direct ? &one : nullptr, direct && !dt ? dctl : nullptr);
     if (e == cudaSuccess && mb >= 0) e = cudaEventRecord(ctx->mask_free[mb], sq);  // staging buffer read
     if (e != cudaSuccess) return cuda_fail(ctx, e, "pack launch");
-    Ctl* dctl = (Ctl*)(dbase + off_ctl);
     Job* djobs = (Job*)(dbase + off_jobs);
     JobState* dstates = (JobState*)(dbase + off_states);
     unsigned long long* dq[3] = {(unsigned long long*)(dbase + off_q[0]),
@@ -762,8 +769,9 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     const bool spec = sh.kernel == 2;  // the blocked kernel reads first entries early (kSpecSlots zeroed slots)
     const int nz = spec ? (int)std::min<unsigned long long>(total_bricks, hdk::kSpecSlots) : 0;
     if (!dt)
-        e = hdk::launch_setup(ddesc, n, setup_tiles, split ? prep_sms : 0, djobs, dstates, dq[g0 % 3], dctl, g0, bxw, by, bz,
-                          setup_mode, sq, dq[(g0 + 1) % 3], dq[(g0 + 2) % 3], nz);
+        e = hdk::launch_setup(direct ? nullptr : ddesc, n, setup_tiles, split ? prep_sms : 0, djobs, dstates, dq[g0 % 3],
+                              dctl, g0, bxw, by, bz, setup_mode, sq, dq[(g0 + 1) % 3], dq[(g0 + 2) % 3], nz,
+                              direct ? &one : nullptr, direct ? ddesc : nullptr);
     if (e == cudaSuccess && split) {
         // the dilation follows the set-up; the caller's stream follows the
         // packing's reads of its masks (work it queues later may overwrite
@@ -775,8 +783,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "setup launch");
     if (ro.map_a || ro.map_b) {
-        e = hdk::launch_map_init(ddesc, ro.map_a, ro.map_b,
-                                 (long long)pairs[0].W * pairs[0].H * pairs[0].D, ctx->opt.label, s);
+        e = hdk::launch_map_init(one, ro.map_a, ro.map_b, ctx->opt.label, s);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "map init launch");
     }
 
@@ -811,13 +818,15 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     sp.descs = ddesc;
     sp.npairs = n;
     sp.pct = pct;
-    sp.out = async ? ro.async_out : (hd_result*)(dbase + off_out);
+    sp.reset_info = direct ? 1 : 0;
+    hd_result* const hres = async ? nullptr : (hd_result*)(hbase + upload_bytes);
+    sp.out = async ? ro.async_out : hres;  // synchronous calls: pinned host memory, no read-back
     void* args[] = {&sp};
     if (timing) cudaEventRecord(ctx->ev[2], s);
     if (stime) cudaEventRecord(ctx->split.ev[3], sv);  // after the previous dilation and this set-up
     if (dt) {
         hdk::DtParams dp{};
-        dp.info = (const PairInfo*)(dbase + off_infos);
+        dp.info = dinfos;
         dp.packed[0] = (const uint32_t*)(dbase + plan[0].off_pa);
         dp.packed[1] = (const uint32_t*)(dbase + plan[0].off_pb);
         for (int j = 0; j < 2; ++j) {
@@ -858,6 +867,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         ctx->split.next = (ws + 1) % ctx->split.nws;
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "dilation launch");
+    if (direct) ctx->info_clean[ws] = true;
     if (timing) cudaEventRecord(ctx->ev[3], s);
     if (async) {
         // the step counter moves past any step this launch can reach (its
@@ -866,12 +876,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         return HD_OK;
     }
 
-    // ---- read-back: the loop control and the decoded results ------------------
-    hd_result* hres = (hd_result*)(hbase + upload_bytes);
-    e = cudaMemcpyAsync(hbase + off_ctl, dbase + off_ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, s);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(hres, dbase + off_out, sizeof(hd_result) * n, cudaMemcpyDeviceToHost, s);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "result read-back");
+    // ---- the results, once the launch has written them ------------------------
     uint64_t* htc = (uint64_t*)(hres + n);
     if (stats) {
         size_t o = 0;
@@ -886,8 +891,11 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "dilation");
 
-    const Ctl* hctl = (const Ctl*)(hbase + off_ctl);
-    if (!dt) ctx->g_next = std::max(ctx->g_next, hctl->g_end) + 2;
+    // past the last step run (after an error, past any step the launch could reach)
+    const int iters = hres[0].iterations;
+    bool hard = false;
+    for (int i = 0; i < n; ++i) hard = hard || (hres[i].status != HD_OK && hres[i].status != HD_EMPTY_MASK);
+    if (!dt) ctx->g_next = g0 + (hard ? std::max(sp.max_iters, iters) : iters) + 2;
     if (timing) {
         ctx->split.timed = false;
         hd_timings& T = ctx->last_timings;
@@ -895,7 +903,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         cudaEventElapsedTime(&T.setup_ms, ctx->ev[1], ctx->ev[2]);
         cudaEventElapsedTime(&T.solve_ms, ctx->ev[2], ctx->ev[3]);
         cudaEventElapsedTime(&T.total_ms, ctx->ev[0], ctx->ev[3]);
-        T.iterations = hctl->iters_run;
+        T.iterations = iters;
         T.grid_ctas = (int)grid.x;
         T.brick_x_words = bxw;
         T.brick_z = bz;
@@ -1027,15 +1035,12 @@ hd_status hd_context_destroy(hd_context* ctx) {
         DeviceGuard g(ctx->device);
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
         split_release(ctx);
+        ctx->infos.release();
         ctx->arena.release();
         for (DeviceArena& a : ctx->ws_arena) a.release();
         ctx->stamps.release();
         for (DeviceArena& a : ctx->part_stamps) a.release();
         ctx->pinned.release();
-        for (int i = 0; i < hd_context::kAsyncSlots; ++i) {
-            ctx->async_stage[i].release();
-            if (ctx->async_done[i]) cudaEventDestroy(ctx->async_done[i]);
-        }
         if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
         for (int i = 0; i < 2; ++i) {
             ctx->mask_stage[i].release();

@@ -44,6 +44,14 @@ struct PairInfo {
     int32_t pad[2];
 };
 
+// Start values of the counts and the bounding box.
+__host__ __device__ __forceinline__ PairInfo pair_info_start() {
+    PairInfo I{};
+    I.bb[0] = I.bb[2] = I.bb[4] = 0x7fffffff;
+    I.bb[1] = I.bb[3] = I.bb[5] = -1;
+    return I;
+}
+
 // Packing / set-up descriptor of one pair (host-written).
 struct PairDesc {
     const uint8_t* a;
@@ -89,7 +97,7 @@ struct DtState {
 
 // One pair, by value (direction 0: A's distances at B's voxels, 1: the reverse).
 struct DtParams {
-    const PairInfo* info;
+    PairInfo* info;              // put back to the start values by the decode
     const uint32_t* packed[2];   // pa, pb
     uint32_t* vol[2];            // in-plane distances as bytes, four rows per word: dt_vol_words
     uint16_t* base[2];           // base of each 64-row x 32-column tile's bytes: dt_bases
@@ -261,6 +269,9 @@ struct SolveParams {
     // serving: decode only pairs whose descriptor is live (info != null) and
     // whose jobs have both finished; the others' out[i] is left as it is
     int32_t decode_done_only;
+    // single pairs: the decode puts the pair's counts and bounding box back to
+    // their start values, for the next packing (see launch_pack)
+    int32_t reset_info;
     // serving: a word the host advances while a launch runs (requests
     // waiting for admission); once it differs from yield_gen the loop ends
     // at the next grid barrier (null: never)

@@ -101,6 +101,8 @@ constexpr int kPlaneEnds = 2 * kPlaneWarps * 2 * 32;
 // pair, 97-114 us for 512^3 (both directions).
 __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __grid_constant__ DtParams p) {
     extern __shared__ uint32_t sm[];
+    cudaGridDependencySynchronize();  // launched while the packing ends
+    cudaTriggerProgrammaticLaunchCompletion();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* const tr = sm + warp * kTr;
     uint32_t* const s_end = sm + kPlaneWarps * kTr;  // [2][warps][2][32]
@@ -335,6 +337,7 @@ __device__ __forceinline__ void dt_decode(const DtParams& p, const PairInfo& I) 
         r.hd_robust = max(rk[0] < 0 ? p.kmax : rk[0], rk[1] < 0 ? p.kmax : rk[1]);
     }
     *p.out = r;
+    *p.info = pair_info_start();  // for the next packing
 }
 
 namespace {
@@ -373,17 +376,14 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
     __shared__ unsigned s_any[3];
     __shared__ int s_max[2], s_last;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+    cudaGridDependencySynchronize();  // launched while the plane kernel ends
     const PairInfo I = *p.info;
     const bool act0 = I.n_b > I.n_ab, act1 = I.n_a > I.n_ab;  // directions with targets
     const int nact = (I.n_a == 0 || I.n_b == 0) ? 0 : act0 + act1;
-    if (nact == 0) {  // nothing to measure
-        if (blockIdx.x == 0 && warp == 0) dt_decode(p, I);
-        return;
-    }
     const Geom g = dt_geom(I);
-    const int nseg = (g.d + kSeg - 1) / kSeg;
-    const int units = g.nyq * g.wx;                      // per direction
-    const int bins = min(32 * g.wx, p.W) + g.h + g.d;    // above any distance in the domain
+    const int nseg = nact ? (g.d + kSeg - 1) / kSeg : 0;
+    const int units = g.nyq * g.wx;                                  // per direction
+    const int bins = nact ? min(32 * g.wx, p.W) + g.h + g.d : 0;     // above any distance in the domain
     uint2* const s_v = (uint2*)sm4 + warp * kHalf * 32;
     uint4* const s_end = sm4 + nwarps * kHalf * 16;         // [nseg][32]: first and last plane
     unsigned* const s_zm = (unsigned*)(s_end + nseg * 32);  // [nseg]: planes with targets
@@ -561,12 +561,24 @@ cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s) {
     const long long dunits = 2ll * ((p.H + 3) / 4) * ((p.W + 31) / 32);
     const unsigned pg = (unsigned)std::min<long long>(punits, 3ll * sms);
     const unsigned dg = (unsigned)std::min<long long>(dunits, 4ll * kDepthMaxWarps / dwarps * sms);
-    dt_plane_kernel<<<pg, kPlaneWarps * 32, plane_sm, s>>>(p);
-    e = cudaGetLastError();
+    // each may be scheduled while the kernel before it ends (it waits for that
+    // kernel's results itself)
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    c.gridDim = dim3(pg);
+    c.blockDim = dim3(kPlaneWarps * 32);
+    c.dynamicSmemBytes = plane_sm;
+    e = cudaLaunchKernelEx(&c, dt_plane_kernel, p);
     if (e != cudaSuccess) return e;
-    if (p.map[0]) dt_depth_kernel<true><<<dg, dwarps * 32, depth_sm, s>>>(p);
-    else dt_depth_kernel<false><<<dg, dwarps * 32, depth_sm, s>>>(p);
-    return cudaGetLastError();
+    c.gridDim = dim3(dg);
+    c.blockDim = dim3(dwarps * 32);
+    c.dynamicSmemBytes = depth_sm;
+    return cudaLaunchKernelEx(&c, p.map[0] ? dt_depth_kernel<true> : dt_depth_kernel<false>, p);
 }
 
 }  // namespace hdk

@@ -115,12 +115,6 @@ struct hd_context {
     hdh::TuneTable tune;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // record_timings: before pack/setup/solve, after solve
     hd_timings last_timings{};
-    // asynchronous calls: descriptor staging buffers that stay untouched
-    // until their upload has run (an event per buffer)
-    static constexpr int kAsyncSlots = 4;
-    hdh::PinnedArena async_stage[kAsyncSlots];
-    cudaEvent_t async_done[kAsyncSlots] = {nullptr, nullptr, nullptr, nullptr};
-    int async_next = 0;
     // asynchronous calls with host masks: two device buffers the masks are
     // copied into on a copy stream, so a pair's copy overlaps the previous
     // pair's kernels (ready: copy done; free: the packing that read it done)
@@ -158,6 +152,12 @@ struct hd_context {
         hd_timings shape{};  // the fields of hd_timings that are not times
     } split;
     hdh::DeviceArena ws_arena[Split::kWorkspaces - 1];  // the split path's workspaces 1, 2, ...
+    // single pairs, per workspace: the counts and bounding box that a packing
+    // adds to.  The decode at the end of a pair's launch puts the start values
+    // back; info_clean[ws] is false until the first call has uploaded them and
+    // while a call's launches are incomplete
+    hdh::DeviceArena infos;
+    bool info_clean[Split::kWorkspaces] = {};
 };
 
 namespace hdh {

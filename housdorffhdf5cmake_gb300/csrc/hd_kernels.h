@@ -15,13 +15,18 @@ namespace hdk {
 // label: 0 = every nonzero byte is foreground, 1..255 = bytes equal to label.
 // sms (packing and set-up): SMs the stream's kernels run on (0: the
 // device's); the grid is one resident wave of them.
+// d_descs null: one pair, whose descriptor `one` (host memory) is passed by
+// value; its counts must hold their start values (pair_info_start), and ctl,
+// if given, is cleared.
 cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, int grid, int label, int sms,
-                        cudaStream_t s);
-// zq1 / zq2 (may be null): queues whose first nz slots are zeroed.
+                        cudaStream_t s, const PairDesc* one = nullptr, Ctl* ctl = nullptr);
+// zq1 / zq2 (may be null): queues whose first nz slots are zeroed.  d_descs
+// null: one pair, `one` by value as above, copied to desc_out (device).
 cudaError_t launch_setup(const PairDesc* d_descs, int npairs, long long ntiles, int sms, Job* jobs,
                          JobState* states, unsigned long long* queue0, Ctl* ctl, int g0, int bxw, int by, int bz,
                          int mode, cudaStream_t s, unsigned long long* zq1 = nullptr,
-                         unsigned long long* zq2 = nullptr, int nz = 0);
+                         unsigned long long* zq2 = nullptr, int nz = 0, const PairDesc* one = nullptr,
+                         PairDesc* desc_out = nullptr);
 // Start values of descs[i].info (counts 0, empty bounding box), i < npairs;
 // with slot_descs, also copies descs[i] to slot_descs[descs[i].job0 / 2].
 cudaError_t launch_info_init(const PairDesc* d_descs, int npairs, cudaStream_t s, PairDesc* slot_descs = nullptr);
@@ -29,8 +34,7 @@ cudaError_t launch_info_init(const PairDesc* d_descs, int npairs, cudaStream_t s
 // take the epoch and slot_descs[slot].info becomes null.
 cudaError_t launch_retire(Job* jobs, PairDesc* slot_descs, const uint32_t* list, int n, cudaStream_t s);
 cudaError_t launch_zero_i32(int32_t* p, long long n, cudaStream_t s);
-cudaError_t launch_map_init(const PairDesc* d_descs, int32_t* map_a, int32_t* map_b, long long n, int label,
-                            cudaStream_t s);
+cudaError_t launch_map_init(const PairDesc& one, int32_t* map_a, int32_t* map_b, int label, cudaStream_t s);
 
 // The persistent dilation kernel for one (element, brick width, brick depth).
 // Returns the kernel's host stub for cudaLaunchCooperativeKernel, or nullptr

@@ -97,7 +97,7 @@ constexpr int kPackThreads = 32 * kPackWarps;
 // (many CTAs update one PairInfo: per-warp atomics serialise on its lines).
 // Called by all threads of the CTA.  A warp's counts fit in 32 bits: a volume
 // has fewer than 2^36 voxels, spread over hundreds of warps.
-__device__ __forceinline__ void flush_acc(const PairDesc& P, const PackAcc& acc) {
+__device__ __forceinline__ void flush_acc(PairInfo* const I, int H, const PackAcc& acc) {
     __shared__ unsigned s_cnt[3][kPackWarps];
     __shared__ int s_bb[6][kPackWarps];
     const int warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -116,7 +116,6 @@ __device__ __forceinline__ void flush_acc(const PairDesc& P, const PackAcc& acc)
     }
     __syncthreads();
     // one thread per value
-    PairInfo* const I = P.info;
     if (threadIdx.x < 3) {
         unsigned long long n = 0;
         for (int w = 0; w < nwarps; ++w) n += s_cnt[threadIdx.x][w];
@@ -129,7 +128,7 @@ __device__ __forceinline__ void flush_acc(const PairDesc& P, const PackAcc& acc)
             v = (i & 1) ? max(v, s_bb[i][w]) : min(v, s_bb[i][w]);
             any = any || s_bb[1][w] >= 0;
         }
-        if (i >= 4) v = v / P.H;
+        if (i >= 4) v = v / H;
         if (any) {
             if (i & 1) atomicMax(&I->bb[i], v);
             else atomicMin(&I->bb[i], v);
@@ -149,6 +148,7 @@ static_assert(kPackTileWords == kPackWarps * kSpan, "one tile = one span per war
 // enters the pair).
 struct PackWalk {
     const uint8_t* src[2];
+    uint32_t* dst[2];           // packed masks
     size_t nbytes;              // bytes of a mask
     unsigned wxf, W, H, total;  // words per row, bytes per row, rows per plane, words of the pair
     unsigned pitch;             // packed row pitch (words): wxf rounded up to 4, zero words in between
@@ -169,6 +169,8 @@ __device__ __forceinline__ PackWalk make_walk(const PairDesc& P) {
     PackWalk k;
     k.src[0] = P.a;
     k.src[1] = P.b;
+    k.dst[0] = P.pa;
+    k.dst[1] = P.pb;
     k.nbytes = (size_t)P.W * P.H * P.D;
     k.wxf = (unsigned)P.wxf;
     k.pitch = (unsigned)packed_pitch(P.W);
@@ -262,7 +264,7 @@ __device__ __forceinline__ void put_bits(const PackWalk& k, const PackSpan& n, i
 
 // Cuts the span's words out of the bit streams (a row starts at any bit).
 // (r, w, y): this lane's first word, advanced past the span.
-__device__ __forceinline__ void put_words(const PairDesc& P, const PackWalk& k, const PackSpan& n, unsigned& r,
+__device__ __forceinline__ void put_words(const PackWalk& k, const PackSpan& n, unsigned& r,
                                           unsigned& w, unsigned& y, PackAcc& acc, const uint32_t (*s_bits)[kBitWords]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
@@ -279,11 +281,11 @@ __device__ __forceinline__ void put_words(const PairDesc& P, const PackWalk& k, 
                 out[m] = __funnelshift_r(s_bits[m][o >> 5], s_bits[m][(o >> 5) + 1], o & 31u) & mask;
             }
             const size_t o = (size_t)r * k.pitch + w;
-            P.pa[o] = out[0];
-            P.pb[o] = out[1];
+            k.dst[0][o] = out[0];
+            k.dst[1][o] = out[1];
             if (last)  // the row's last word also writes its padding (up to 3 words)
 #pragma unroll 1
-                for (unsigned x = k.wxf; x < k.pitch; ++x) P.pa[o + 1u + x - k.wxf] = P.pb[o + 1u + x - k.wxf] = 0u;
+                for (unsigned x = 1u; x <= k.pitch - k.wxf; ++x) k.dst[0][o + x] = k.dst[1][o + x] = 0u;
             acc.add(out[0], out[1], (int)r, (int)y, (int)w);
         }
         w += k.dr;  // 32 words on
@@ -314,8 +316,11 @@ __device__ __forceinline__ void put_words(const PairDesc& P, const PackWalk& k, 
 // between the two masks' 37 %.
 template <bool kLabel>
 __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const PairDesc* __restrict__ descs, int npairs,
-                                                               long long ntiles, int label) {
+                                                               long long ntiles, int label,
+                                                               const __grid_constant__ PairDesc one, Ctl* ctl) {
     __shared__ uint32_t s_bits_all[kPackWarps][2][kBitWords];
+    cudaTriggerProgrammaticLaunchCompletion();  // the distance transform's CTAs may take over as these end
+    if (ctl && blockIdx.x == 0 && threadIdx.x == 0) *ctl = Ctl{};  // nobody else uses it before the set-up
     const long long per = (ntiles + gridDim.x - 1) / gridDim.x;
     long long tile = (long long)blockIdx.x * per;
     const long long t_hi = min(ntiles, tile + per);
@@ -325,12 +330,13 @@ __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const Pai
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
     for (;;) {  // the pairs of this CTA's run
-        const PairDesc& P = descs[pi];
+        const PairDesc& P = descs ? descs[pi] : one;
         const PackWalk k = make_walk(P);
+        const long long first = P.tile0;
         const long long end = pi + 1 < npairs ? min(t_hi, descs[pi + 1].tile0) : t_hi;
         PackAcc acc;
-        unsigned t0 = (unsigned)((tile - P.tile0) * kPackTileWords) + (threadIdx.x >> 5) * kSpan;
-        const unsigned t1 = min((unsigned)((end - P.tile0) * kPackTileWords), k.total);
+        unsigned t0 = (unsigned)((tile - first) * kPackTileWords) + (threadIdx.x >> 5) * kSpan;
+        const unsigned t1 = min((unsigned)((end - first) * kPackTileWords), k.total);
         unsigned r = (t0 + lane) / k.wxf;
         unsigned w = t0 + lane - r * k.wxf;
         unsigned y = r % k.H;
@@ -345,7 +351,7 @@ __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const Pai
 #pragma unroll
             for (int m = 0; m < 2; ++m) put_bits<kLabel>(k, n, m, c[m], x[m], (unsigned)label, s_bits[m]);
             __syncwarp();
-            put_words(P, k, n, r, w, y, acc, s_bits);
+            put_words(k, n, r, w, y, acc, s_bits);
             // this warp's span of the next tile
             w += k.tr;
             const unsigned dr = k.tq + (w >= k.wxf ? 1u : 0u);
@@ -354,7 +360,7 @@ __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const Pai
             y += dr;
             if (y >= k.H) y %= k.H;
         }
-        flush_acc(P, acc);
+        flush_acc(P.info, P.H, acc);
         tile = end;
         if (tile >= t_hi) break;
         ++pi;
@@ -444,8 +450,10 @@ __device__ __forceinline__ long long setup_tile(const PairDesc& P, long long til
 __global__ void __launch_bounds__(256) setup_kernel(const PairDesc* __restrict__ descs, int npairs, long long ntiles,
                                                     Job* jobs, JobState* states, unsigned long long* queue0,
                                                     Ctl* ctl, int g0, int bxw, int by, int bz, int mode,
-                                                    unsigned long long* zq1, unsigned long long* zq2, int nz) {
+                                                    unsigned long long* zq1, unsigned long long* zq2, int nz,
+                                                    const __grid_constant__ PairDesc one, PairDesc* desc_out) {
     __shared__ unsigned s_base;
+    if (desc_out && blockIdx.x == 0 && threadIdx.x == 0) *desc_out = one;  // for the result decode
     int pi = -1;
     const long long G = gridDim.x;
     // the first nz slots of the two queues the first step does not read
@@ -461,8 +469,9 @@ __global__ void __launch_bounds__(256) setup_kernel(const PairDesc* __restrict__
         int np = pi < 0 ? pair_of_tile(descs, npairs, tile, true) : pi;
         while (np + 1 < npairs && descs[np + 1].stile0 <= tile) ++np;  // tiles only increase
         pi = np;
-        const long long t0 = descs[pi].stile0;
-        const long long need = setup_tile(descs[pi], tile - t0, jobs, states, queue0, ctl, g0, bxw, by, bz, mode,
+        const PairDesc& P = descs ? descs[pi] : one;
+        const long long t0 = P.stile0;
+        const long long need = setup_tile(P, tile - t0, jobs, states, queue0, ctl, g0, bxw, by, bz, mode,
                                           &s_base);
         // The pair's tiles from `need` on have nothing to do (the host sizes
         // the tiles for the largest domain and for copies that reading the
@@ -617,11 +626,7 @@ __global__ void info_init_kernel(const PairDesc* __restrict__ descs, int npairs,
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= npairs) return;
     if (slot_descs) slot_descs[descs[i].job0 / 2] = descs[i];  // serving: the slot's copy for the result decode
-    PairInfo* I = descs[i].info;
-    I->n_a = I->n_b = I->n_ab = 0ull;
-    I->bb[0] = I->bb[2] = I->bb[4] = INT_MAX;
-    I->bb[1] = I->bb[3] = I->bb[5] = -1;
-    I->pad[0] = I->pad[1] = 0;
+    *descs[i].info = pair_info_start();
 }
 
 // Serving: retire finished pairs' slots.  list holds (slot, epoch) pairs: the
@@ -646,8 +651,7 @@ __global__ void zero_i32_kernel(int32_t* p, long long n) {
 
 // Per-voxel maps: -1 outside the mask, 0 on the overlap, and (filled later by
 // the dilation) the distance on voxels of one mask outside the other.
-__global__ void map_init_kernel(const PairDesc* __restrict__ descs, int32_t* map_a, int32_t* map_b, int label) {
-    const PairDesc& P = descs[0];
+__global__ void map_init_kernel(const __grid_constant__ PairDesc P, int32_t* map_a, int32_t* map_b, int label) {
     const long long n = (long long)P.W * P.H * P.D;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n;
          t += (long long)gridDim.x * blockDim.x) {
@@ -663,7 +667,7 @@ __global__ void map_init_kernel(const PairDesc* __restrict__ descs, int32_t* map
 namespace hdk {
 
 cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, int grid, int label, int sms,
-                        cudaStream_t s) {
+                        cudaStream_t s, const PairDesc* one, Ctl* ctl) {
     // one wave of resident CTAs (per device and variant, from the occupancy calculator)
     static int resident[2][64] = {{0}};
     static int per_sm_of[2][64] = {{0}};
@@ -684,14 +688,16 @@ cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, i
     if (dev < 64) grid = sms > 0 ? per_sm_of[v][dev] * sms : resident[v][dev];
     if (grid > ntiles) grid = (int)ntiles;
     if (grid < 1) grid = 1;
-    if (label) pack_kernel<true><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, label);
-    else pack_kernel<false><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, 0);
+    const PairDesc P = one ? *one : PairDesc{};
+    if (label) pack_kernel<true><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, label, P, ctl);
+    else pack_kernel<false><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, 0, P, ctl);
     return cudaGetLastError();
 }
 
 cudaError_t launch_setup(const PairDesc* d_descs, int npairs, long long ntiles, int sms, Job* jobs,
                          JobState* states, unsigned long long* queue0, Ctl* ctl, int g0, int bxw, int by, int bz,
-                         int mode, cudaStream_t s, unsigned long long* zq1, unsigned long long* zq2, int nz) {
+                         int mode, cudaStream_t s, unsigned long long* zq1, unsigned long long* zq2, int nz,
+                         const PairDesc* one, PairDesc* desc_out) {
     // one wave of resident CTAs (per device, from the occupancy calculator):
     // CTAs whose tiles have nothing to do leave at once, later waves would
     // only add their scheduling
@@ -717,7 +723,7 @@ cudaError_t launch_setup(const PairDesc* d_descs, int npairs, long long ntiles, 
     long long grid = std::min<long long>((long long)per_sm * nsm, ntiles);
     if (grid < 1) grid = 1;
     setup_kernel<<<(unsigned)grid, 256, 0, s>>>(d_descs, npairs, ntiles, jobs, states, queue0, ctl, g0, bxw, by, bz,
-                                                mode, zq1, zq2, zq1 && zq2 ? nz : 0);
+                                                mode, zq1, zq2, zq1 && zq2 ? nz : 0, one ? *one : PairDesc{}, desc_out);
     return cudaGetLastError();
 }
 
@@ -741,11 +747,11 @@ cudaError_t launch_zero_i32(int32_t* p, long long n, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_map_init(const PairDesc* d_descs, int32_t* map_a, int32_t* map_b, long long n, int label,
-                            cudaStream_t s) {
+cudaError_t launch_map_init(const PairDesc& one, int32_t* map_a, int32_t* map_b, int label, cudaStream_t s) {
+    const long long n = (long long)one.W * one.H * one.D;
     long long blocks = (n + 255) / 256;
     if (blocks > 8192) blocks = 8192;
-    map_init_kernel<<<(int)blocks, 256, 0, s>>>(d_descs, map_a, map_b, label);
+    map_init_kernel<<<(int)blocks, 256, 0, s>>>(one, map_a, map_b, label);
     return cudaGetLastError();
 }
 

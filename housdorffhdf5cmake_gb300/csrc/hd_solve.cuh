@@ -210,7 +210,11 @@ static __device__ __noinline__ void decode_pair_warp(const SolveParams& p, int i
         r.hd_robust = robust_k_warp2(P.hist[1], r.n_a_not_b, P.hist[0], r.n_b_not_a, kp1, p.pct);
         if (st != HD_OK) r.hd = r.hd_ab = r.hd_ba = r.hd_robust = -1;
     }
-    if ((threadIdx.x & 31) == 0) p.out[i] = r;
+    __syncwarp();  // every lane has read the counts
+    if ((threadIdx.x & 31) == 0) {
+        p.out[i] = r;
+        if (p.reset_info) *P.info = pair_info_start();
+    }
 }
 
 template <int BXW, int BZ, bool SE18>
