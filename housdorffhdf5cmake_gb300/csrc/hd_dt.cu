@@ -21,7 +21,7 @@
 // byte per voxel over a base per tile holds them exactly.
 //
 // Both kernels together, against the dilation loop with its set-up: 512^3
-// with 451 steps 0.15 against 3.5 ms, 512x512x256 with 19 to 30 steps 0.047
+// with 451 steps 0.10 against 3.5 ms, 512x512x256 with 19 to 30 steps 0.045
 // against 0.10 to 0.13 ms, 64^3 0.021 against 0.08 ms.
 #include <algorithm>
 #include <atomic>
@@ -96,17 +96,20 @@ constexpr int kPlaneEnds = 2 * kPlaneWarps * 2 * 32;
 //   y: after a transpose through shared memory, lane = column, registers =
 //      rows; segments of 32 rows (the two halves) sweep on their own, then
 //      take the carry over the segments above and below from shared memory
-// About 400 warp instructions per 2048 voxels; issue slots 37 % busy (the
-// barrier per word column and the sweeps' chains).  20 us for a 512x512x256
-// pair, 97-114 us for 512^3 (both directions).
+// About 400 warp instructions per 2048 voxels; issue slots 40 % busy (the
+// barrier per word column and the sweeps' chains).  A CTA whose planes have no
+// source voxel skips them, and rows are scanned once, from the right (the
+// words come one at a time after that, from L1): 512x512x256 pair 16 to 19 us
+// against 19 to 22 us with the words in groups of four registers, 512^3 with
+// small blobs (both directions) 51 to 65 against 97 to 114 us.  64 registers
+// and 4 CTAs per SM (32 bytes spilled): 8 % slower.
 __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __grid_constant__ DtParams p) {
     extern __shared__ uint32_t sm[];
     cudaGridDependencySynchronize();  // launched while the packing ends
-    cudaTriggerProgrammaticLaunchCompletion();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* const tr = sm + warp * kTr;
     uint32_t* const s_end = sm + kPlaneWarps * kTr;  // [2][warps][2][32]
-    uint32_t* const s_r = s_end + kPlaneEnds;        // [groups of words][warps][32]
+    uint32_t* const s_r = s_end + kPlaneEnds;        // [words][warps][32]
     const PairInfo I = *p.info;
     // histograms and counters of the depth kernel
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= p.kmax; t += gridDim.x * blockDim.x)
@@ -135,31 +138,24 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
         const ptrdiff_t other = (const uint4*)p.packed[1 - j] - (const uint4*)p.packed[j];
         const bool va = act && ya < g.h, vb = act && yb < g.h;
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        // carries from the right at each group of four words
+        // One scan of the rows from the right: the carries at each word, the
+        // rows with target voxels, and whether the plane has a source at all
+        unsigned ca = kInf, cb = kInf;
+        const int tz = t * g.d + (act ? z : 0);
         if (act) {
-            unsigned ca = kInf, cb = kInf;
 #pragma unroll 1
             for (int q = g.nq - 1; q >= 0; --q) {
-                s_r[(q * kPlaneWarps + warp) * 32 + lane] = ca | (cb << 16);
                 const uint4 a = va ? __ldg(ra + q) : zero, b = vb ? __ldg(rb + q) : zero;
-                ca = carry_right(carry_right(carry_right(carry_right(ca, a.w), a.z), a.y), a.x);
-                cb = carry_right(carry_right(carry_right(carry_right(cb, b.w), b.z), b.y), b.x);
-            }
-        }
-        unsigned la = kInf, lb = kInf;
-        uint32_t* const vol = p.vol[j] + (size_t)(act ? z : 0) * g.nyq * vrow;
-        const int tz = t * g.d + (act ? z : 0);
-#pragma unroll 1
-        for (int q = 0; q < g.nq; ++q) {
-            const uint4 a4 = va ? __ldg(ra + q) : zero, b4 = vb ? __ldg(rb + q) : zero;
-            const uint32_t wa[4] = {a4.x, a4.y, a4.z, a4.w}, wb[4] = {b4.x, b4.y, b4.z, b4.w};
-            {  // rows with target voxels, per word
                 const uint4 c = va ? __ldg(ra + other + q) : zero, d = vb ? __ldg(rb + other + q) : zero;
-                const uint32_t ta[4] = {c.x & ~a4.x, c.y & ~a4.y, c.z & ~a4.z, c.w & ~a4.w};
-                const uint32_t tb[4] = {d.x & ~b4.x, d.y & ~b4.y, d.z & ~b4.z, d.w & ~b4.w};
+                const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+                const uint32_t ta[4] = {c.x & ~a.x, c.y & ~a.y, c.z & ~a.z, c.w & ~a.w};
+                const uint32_t tb[4] = {d.x & ~b.x, d.y & ~b.y, d.z & ~b.z, d.w & ~b.w};
                 unsigned fa = 0, fb = 0;
 #pragma unroll
-                for (int k = 0; k < 4; ++k) {
+                for (int k = 3; k >= 0; --k) {
+                    s_r[((4 * q + k) * kPlaneWarps + warp) * 32 + lane] = ca | (cb << 16);
+                    ca = carry_right(ca, wa[k]);
+                    cb = carry_right(cb, wb[k]);
                     const unsigned ba = __ballot_sync(kFull, ta[k] != 0u), bb = __ballot_sync(kFull, tb[k] != 0u);
                     if (lane == k) {
                         fa = ba;
@@ -167,30 +163,32 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
                     }
                 }
                 const int w = 4 * (q0 + q) + lane;
-                if (act && lane < 4 && w >= g.wx0 && w <= g.w1) {
+                if (lane < 4 && w >= g.wx0 && w <= g.w1) {
                     uint32_t* const f = p.rows[j] + (size_t)(w - g.wx0) * 2 * g.ntile * g.d + t * g.d + tz;
                     f[0] = fa;
                     f[g.d] = fb;
                 }
             }
-            const uint32_t r0 = act ? s_r[(q * kPlaneWarps + warp) * 32 + lane] : 0u;
-            uint32_t rc[4];  // carry from the right at each word
-            {
-                unsigned ca = r0 & 0xffffu, cb = r0 >> 16;
-#pragma unroll
-                for (int k = 3; k >= 0; --k) {
-                    rc[k] = ca | (cb << 16);
-                    ca = carry_right(ca, wa[k]);
-                    cb = carry_right(cb, wb[k]);
-                }
-            }
+        }
+        if (!__syncthreads_or(act && (ca < kInf || cb < kInf))) {  // nothing to measure from
+            if (act)
+                for (int w = lane; w < g.wx; w += 32) p.base[j][(size_t)w * g.ntile * g.d + tz] = (uint16_t)kInf;
+            continue;
+        }
+        unsigned la = kInf, lb = kInf;
+        uint32_t* const vol = p.vol[j] + (size_t)(act ? z : 0) * g.nyq * vrow;
+        const uint32_t* const pa = (const uint32_t*)(ra - q0);
+        const uint32_t* const pb = (const uint32_t*)(rb - q0);
+        uint32_t na = va ? __ldg(pa + g.wx0) : 0u, nb = vb ? __ldg(pb + g.wx0) : 0u;
 #pragma unroll 1
-            for (int k = 0; k < 4; ++k) {
-                const int w = 4 * (q0 + q) + k;
-                if (w < g.wx0 || w > g.w1) continue;  // uniform; words outside the domain are zero
-                const uint32_t ua = k == 0 ? wa[0] : k == 1 ? wa[1] : k == 2 ? wa[2] : wa[3];
-                const uint32_t ub = k == 0 ? wb[0] : k == 1 ? wb[1] : k == 2 ? wb[2] : wb[3];
-                const uint32_t rcw = k == 0 ? rc[0] : k == 1 ? rc[1] : k == 2 ? rc[2] : rc[3];
+        for (int w = g.wx0; w <= g.w1; ++w) {
+            const uint32_t ua = na, ub = nb;
+            if (w < g.w1) {  // the next word's
+                na = va ? __ldg(pa + w + 1) : 0u;
+                nb = vb ? __ldg(pb + w + 1) : 0u;
+            }
+            {
+                const uint32_t rcw = act ? s_r[((w - 4 * q0) * kPlaneWarps + warp) * 32 + lane] : 0u;
                 uint32_t V[32];
                 uint32_t* const end = s_end + ((w & 1) * kPlaneWarps) * 64;
                 if (act) {
@@ -537,7 +535,7 @@ bool dt_fits(int W, int H, int D) {
 cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s) {
     const int nq = ((p.W + 31) / 32 + 3) / 4;
     const int nseg = (p.D + kSeg - 1) / kSeg;
-    const size_t plane_sm = sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)nq * kPlaneWarps * 32);
+    const size_t plane_sm = sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)nq * 4 * kPlaneWarps * 32);
     const int dwarps = nseg > 8 ? kDepthMaxWarps : 4;
     const size_t depth_sm = depth_smem(dwarps, nseg, p.W + p.H + p.D);
     // the limit of dynamic shared memory, once per device for the largest size
