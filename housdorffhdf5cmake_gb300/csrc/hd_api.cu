@@ -484,6 +484,8 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     const size_t off_descs = take(sizeof(PairDesc) * n);
     const size_t upload_bytes = cur;           // [ctl .. descs]
     const size_t off_jobs = take(sizeof(Job) * 2 * n);
+    const int ncols = dt ? hdk::dt_cols(pairs[0].W, pairs[0].H) : 0;
+    const size_t off_cols = take(sizeof(uint32_t) * 2 * ncols);
     size_t hist_words = 0;
     unsigned long long total_bricks = 0;
     int kmax_all = 0;
@@ -756,7 +758,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     const bool stime = split && ctx->opt.record_timings != 0 && ctx->split.ev[0] != nullptr;
     if (stime) cudaEventRecord(ctx->split.ev[0], sq);
     e = hdk::launch_pack(direct ? nullptr : ddesc, n, pack_tiles, grid_pack, ctx->opt.label, split ? prep_sms : 0, sq,
-                         direct ? &one : nullptr, direct && !dt ? dctl : nullptr);
+                         direct ? &one : nullptr, direct && !dt ? dctl : nullptr, (uint32_t*)(dbase + off_cols), 2 * ncols);
     if (e == cudaSuccess && mb >= 0) e = cudaEventRecord(ctx->mask_free[mb], sq);  // staging buffer read
     if (e != cudaSuccess) return cuda_fail(ctx, e, "pack launch");
     Job* djobs = (Job*)(dbase + off_jobs);
@@ -835,6 +837,8 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
             dp.rows[j] = (uint32_t*)(dbase + plan[0].off_jb[j][2]);
             dp.hist[j] = (unsigned long long*)(dbase + plan[0].off_hist) + (size_t)j * (plan[0].kmax + 1);
         }
+        dp.cols = (uint32_t*)(dbase + off_cols);
+        dp.ncols = ncols;
         dp.state = (hdk::DtState*)(dbase + off_states);  // the plane kernel zeroes it
         dp.map[0] = ro.map_b;
         dp.map[1] = ro.map_a;

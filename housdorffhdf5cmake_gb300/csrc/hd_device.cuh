@@ -89,10 +89,11 @@ __host__ __device__ __forceinline__ long long dt_bases(int W, int H, int D) {
     return (long long)D * ((H + 63) / 64) * ((W + 31) / 32);
 }
 
+__host__ __device__ __forceinline__ int dt_cols(int W, int H) { return (W + 31) / 32 * 2 * ((H + 63) / 64); }
+
 // Counters of the distance transform's second kernel.
 struct DtState {
     unsigned int done;  // CTAs that have added their counts
-    int32_t hd[2];      // largest distance per direction
 };
 
 // One pair, by value (direction 0: A's distances at B's voxels, 1: the reverse).
@@ -102,6 +103,9 @@ struct DtParams {
     uint32_t* vol[2];            // in-plane distances as bytes, four rows per word: dt_vol_words
     uint16_t* base[2];           // base of each 64-row x 32-column tile's bytes: dt_bases
     uint32_t* rows[2];           // rows with target voxels, per word column, 32 rows and plane: 2 dt_bases
+    uint32_t* cols;              // per direction (ncols each): rows with a target in any plane, per word column
+                                 // and 32 rows; zero before the plane kernel (launch_pack)
+    int32_t ncols;               // dt_cols
     unsigned long long* hist[2]; // kmax + 1 counters
     DtState* state;
     int32_t* map[2];             // optional dense per-voxel distance maps (B's voxels, A's voxels)

@@ -21,8 +21,8 @@
 // byte per voxel over a base per tile holds them exactly.
 //
 // Both kernels together, against the dilation loop with its set-up: 512^3
-// with 451 steps 0.10 against 3.5 ms, 512x512x256 with 19 to 30 steps 0.045
-// against 0.10 to 0.13 ms, 64^3 0.021 against 0.08 ms.
+// with 451 steps 0.09 against 3.5 ms, 512x512x256 with 19 to 30 steps 0.037
+// against 0.10 to 0.13 ms, 64^3 0.019 against 0.08 ms.
 #include <algorithm>
 #include <atomic>
 #include <cuda_runtime.h>
@@ -50,6 +50,12 @@ __device__ __forceinline__ uint32_t byte_signs(uint32_t a) {
     uint32_t d;
     asm("prmt.b32 %0, %1, %1, %2;" : "=r"(d) : "r"(a), "n"(kSel));
     return d;
+}
+
+// Adds 1 to a counter in shared memory if `in`; predicated, no branch.
+__device__ __forceinline__ void red_shared_inc(uint32_t at, unsigned in) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.u32 q, %1, 0;\n @q red.shared.add.u32 [%0], 1;\n}" ::"r"(at), "r"(in)
+                 : "memory");
 }
 
 // A pair's domain: the bounding box of A u B, x in whole words.
@@ -167,6 +173,9 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
                     uint32_t* const f = p.rows[j] + (size_t)(w - g.wx0) * 2 * g.ntile * g.d + t * g.d + tz;
                     f[0] = fa;
                     f[g.d] = fb;
+                    uint32_t* const c = p.cols + j * p.ncols + (w - g.wx0) * 2 * g.ntile + 2 * t;
+                    if (fa) atomicOr(c, fa);
+                    if (fb) atomicOr(c + 1, fb);
                 }
             }
         }
@@ -275,8 +284,8 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
 
 // One warp: the pair's result from the counts and the two histograms, with
 // the rules of decode_pair_warp (statuses, exact sums, one double division,
-// robust HD).  One pass over the bins: the chain of loads is the largest
-// distances, then 32 bins of both directions at a time.
+// robust HD).  One pass over the bins, 32 of both directions at a time, until
+// every target is counted.
 __device__ __forceinline__ void dt_decode(const DtParams& p, const PairInfo& I) {
     const int lane = threadIdx.x & 31;
     const unsigned long long n_ab = I.n_a - I.n_ab, n_ba = I.n_b - I.n_ab;  // A's, B's voxels outside the other
@@ -285,15 +294,18 @@ __device__ __forceinline__ void dt_decode(const DtParams& p, const PairInfo& I) 
     const bool empty = I.n_a == 0 || I.n_b == 0;
     if (!empty) {
         const float tf[2] = {(float)n_ba * p.pct, (float)n_ab * p.pct};  // job 0 measures B's voxels
-#pragma unroll
-        for (int j = 0; j < 2; ++j) hd[j] = ld_relaxed_s32(&p.state->hd[j]);
+        const unsigned long long total[2] = {n_ba, n_ab};
 #pragma unroll 1
-        for (int k0 = 0; k0 <= max(hd[0], hd[1]); k0 += 32) {
+        for (int k0 = 0; k0 <= p.kmax && (cov[0] < total[0] || cov[1] < total[1]); k0 += 32) {
             const int k = k0 + lane;
+            unsigned long long c2[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) c2[j] = k <= p.kmax ? __ldcg(p.hist[j] + k) : 0ull;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                unsigned long long c = k <= hd[j] ? __ldcg(p.hist[j] + k) : 0ull;
+                unsigned long long c = c2[j];
                 sum[j] += (unsigned long long)k * c;
+                if (c) hd[j] = k;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
                     const unsigned long long x = __shfl_up_sync(kFull, c, o);
@@ -304,6 +316,12 @@ __device__ __forceinline__ void dt_decode(const DtParams& p, const PairInfo& I) 
                 if (m && rk[j] < 0) rk[j] = k0 + __ffs(m) - 1;
                 cov[j] += __shfl_sync(kFull, c, 31);
             }
+        }
+        // (no targets at all: stops at step 0)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            hd[j] = __reduce_max_sync(kFull, hd[j]);
+            if (total[j] == 0ull && rk[j] < 0) rk[j] = 0;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -342,37 +360,41 @@ namespace {
 constexpr int kDepthMaxWarps = 8;
 constexpr int kSeg = 16;  // planes of a segment
 constexpr int kHalf = 8;  // planes of a segment staged for counting at a time
-// Dynamic shared memory of a CTA: staged distances per warp, then per segment
-// of the column its end planes and the mask of its planes with targets, then
-// the distances' counters of both directions.
-__host__ __device__ constexpr size_t depth_smem(int warps, int nseg, int bins) {
-    return (size_t)warps * kHalf * 32 * 8 + (size_t)nseg * (32 * 16 + 4) + (size_t)bins * 8;
+// Dynamic shared memory of a CTA: staged distances per warp, the column's end
+// planes per segment, the distances' counters of both directions, the masks
+// of a segment's planes with targets, and the list of columns with targets.
+__host__ __device__ constexpr size_t depth_smem(int warps, int nseg, int bins, int ncols) {
+    return (size_t)warps * kHalf * 32 * 8 + (size_t)nseg * (32 * 16 + 4) + ((size_t)bins * 8 + 16) + (size_t)ncols * 8;
 }
 }  // namespace
 
-// Columns: a unit is one direction's four rows x one word column, all
-// planes; its tasks are segments of 16 planes (a warp: lane = column, two
-// registers of 16-bit pairs per plane = the four rows).
-//   1. the segments' planes with target words, from the plane kernel's row
-//      flags; a unit without any ends here
-//   2. first pass: every segment is swept and leaves its two end planes in
+// Columns: a unit is one direction's four rows x one word column that hold a
+// target in some plane, all planes; its tasks are segments of 16 planes (a
+// warp: lane = column, two registers of 16-bit pairs per plane = the four
+// rows).
+//   1. first pass: every segment is swept and leaves its two end planes in
 //      shared memory
-//   3. second pass: the segments with targets (few: targets are a shell) are
+//   2. second pass: the segments with targets (few: targets are a shell) are
 //      swept again, now with the carry over the segments before and after
 //      from the end planes, and count the distances at their targets
+// Every CTA lists the units itself, from the plane kernel's masks of rows with
+// targets per word column, and takes every gridDim-th: about half of a
+// domain's columns have no target.
 // Sweeping twice costs less than holding a segment over the barrier: the
 // warps that have no targets would wait there for those that have.  The two
 // passes share one piece of code, and the targets of a task are visited in a
 // rolled loop: a CTA runs a few tasks only, so instruction fetches count.
-// 512x512x256 pair 25-29 us, 512^3 41-44 us, 64^3 14 us; with units of four
-// word columns and both directions 40-59 / 60-76 / 27 us (one unit per CTA
-// and half of them without targets: the chip waited for the rest), with the
-// segments held over a barrier per word column 80 us at 512x512x256.
+// Bound by the chain of loads, barriers and counters of one unit: a
+// 512x512x256 pair has 400 to 530 units for 608 CTAs.  512x512x256 pair 17 to
+// 22 us, 512^3 29 to 34 us, 64^3 12.5 us.  Before: with every column visited
+// and its segments' masks read behind a barrier 25-29 / 40-44 / 14 us; units
+// claimed from a counter 28-35 us at 512x512x256 (the claim waits once per
+// unit); 16 warps per CTA holding their segments over the barrier likewise.
 template <bool kMap>
 __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const __grid_constant__ DtParams p) {
     extern __shared__ uint4 sm4[];
-    __shared__ unsigned s_any[3];
-    __shared__ int s_max[2], s_last;
+    __shared__ int s_max[2], s_last, s_warp[kDepthMaxWarps], s_first[2];
+    __shared__ uint4 s_tgt[kDepthMaxWarps][kSeg];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
     cudaGridDependencySynchronize();  // launched while the plane kernel ends
     const PairInfo I = *p.info;
@@ -380,50 +402,111 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
     const int nact = (I.n_a == 0 || I.n_b == 0) ? 0 : act0 + act1;
     const Geom g = dt_geom(I);
     const int nseg = nact ? (g.d + kSeg - 1) / kSeg : 0;
-    const int units = g.nyq * g.wx;                                  // per direction
     const int bins = nact ? min(32 * g.wx, p.W) + g.h + g.d : 0;     // above any distance in the domain
+    const int per = g.wx * 2 * g.ntile;                              // masks of 32 rows, per direction
     uint2* const s_v = (uint2*)sm4 + warp * kHalf * 32;
-    uint4* const s_end = sm4 + nwarps * kHalf * 16;         // [nseg][32]: first and last plane
-    unsigned* const s_zm = (unsigned*)(s_end + nseg * 32);  // [nseg]: planes with targets
-    unsigned* const s_hist = s_zm + nseg;                   // [direction][bins]
-#pragma unroll 1
-    for (int t = threadIdx.x; t < 2 * bins; t += blockDim.x) s_hist[t] = 0u;
-    if (threadIdx.x < 3) s_any[threadIdx.x] = 0u;
+    uint4* const s_end = sm4 + nwarps * kHalf * 16;          // [nseg][32]: first and last plane
+    uint4* const s_hist4 = s_end + nseg * 32;                // [direction][bins]
+    unsigned* const s_hist = (unsigned*)s_hist4;
+    unsigned* const s_list = (unsigned*)(s_hist4 + (2 * bins + 3) / 4);  // per mask: four-row groups with targets, units before
+    unsigned* const s_zm = s_list + nact * per;              // [nseg]: planes with targets
+    for (int t = threadIdx.x; t < (2 * bins + 3) / 4; t += blockDim.x) s_hist4[t] = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < 2) s_max[threadIdx.x] = 0;
-    __syncthreads();
-    const size_t vrow = (size_t)g.wx * 32, vplane = vrow * g.nyq;
-    int fb = 0;
+    int units = 0;
 #pragma unroll 1
-    for (int u = blockIdx.x; u < nact * units; u += gridDim.x) {
-        const int j = act0 ? u >= units : 1, uu = act0 && j ? u - units : u;
-        const int yq = uu / g.wx, w = uu - yq * g.wx;
-        // 1. planes with targets: lane = plane
-        {
-            const uint32_t* const f = p.rows[j] + ((size_t)w * 2 * g.ntile + (yq >> 3)) * g.d;
-            unsigned any = 0;
-#pragma unroll 1
-            for (int z0 = warp * 32; z0 < g.d; z0 += nwarps * 32) {
-                const unsigned r = z0 + lane < g.d ? __ldg(f + z0 + lane) : 0u;
-                const unsigned m = __ballot_sync(kFull, ((r >> (4 * (yq & 7))) & 0xfu) != 0u);
-                any |= m;
-                if (lane < 2 && z0 + kSeg * lane < g.d) s_zm[z0 / kSeg + lane] = (m >> (kSeg * lane)) & 0xffffu;
-            }
-            if (any && lane == 0) atomicOr(&s_any[fb], any);
+    for (int i0 = 0; i0 < nact * per; i0 += blockDim.x) {
+        const int i = i0 + threadIdx.x, jj = i >= per;
+        unsigned m = i < nact * per ? __ldcg(p.cols + (act0 ? jj : 1) * p.ncols + (i - jj * per)) : 0u;
+        m |= m >> 2;
+        m = (m | (m >> 1)) & 0x11111111u;  // one bit per four rows
+        const int c = __popc(m);
+        int x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += v;
         }
-        if (threadIdx.x == 0) s_any[fb == 2 ? 0 : fb + 1] = 0u;  // the next unit's
+        if (lane == 31) s_warp[warp] = x;
         __syncthreads();
-        const unsigned flag = s_any[fb];
-        fb = fb == 2 ? 0 : fb + 1;
-        if (!flag) continue;
+        int before = units;
+        for (int v = 0; v < nwarps; ++v) {
+            if (v < warp) before += s_warp[v];
+            units += s_warp[v];
+        }
+        before += x - c;
+        if ((int)blockIdx.x >= before && (int)blockIdx.x < before + c) {  // the CTA's first unit
+            unsigned g1 = m;
+            for (int k = blockIdx.x - before; k > 0; --k) g1 &= g1 - 1u;
+            s_first[0] = i;
+            s_first[1] = (__ffs(g1) - 1) >> 2;
+        }
+        // bits 0, 4, .. 28 -> bits 24 .. 31
+        m = (m | (m >> 3)) & 0x03030303u;
+        m = (m | (m >> 6)) & 0x000f000fu;
+        m = (m | (m >> 12)) << 24;
+        if (i < nact * per) s_list[i] = m | (unsigned)before;
+        __syncthreads();
+    }
+    const size_t vrow = (size_t)g.wx * 32, vplane = vrow * g.nyq;
+    const uint32_t s_hist_at = (uint32_t)__cvta_generic_to_shared(s_hist);
+    int dmax[2] = {0, 0};
+#pragma unroll 1
+    for (int u = blockIdx.x; u < units; u += gridDim.x) {
+        int lo = s_first[0], group = s_first[1];
+        if (u != (int)blockIdx.x) {
+            // the last mask with at most u units before it that has any
+            int hi = nact * per - 1;
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if ((int)(s_list[mid] & 0xffffffu) <= u) lo = mid;
+                else hi = mid - 1;
+            }
+            const unsigned le = s_list[lo];
+            unsigned gm = le >> 24;
+            for (int k = u - (int)(le & 0xffffffu); k > 0; --k) gm &= gm - 1u;
+            group = __ffs(gm) - 1;
+        }
+        const int jj = lo >= per, j = act0 ? jj : 1, wh = lo - jj * per;
+        const int w = wh / (2 * g.ntile), half = wh - w * 2 * g.ntile;
+        const int yq = 8 * half + group;
+        const uint32_t* const rows = p.rows[j] + (size_t)wh * g.d;
 #pragma unroll 1
         for (int pass = 0; pass < 2; ++pass) {
+            // Second pass: the segments with targets; if they are few, one
+            // task per half of a segment's planes (counting takes longer than
+            // loading and sweeping again, and other warps would wait).
+            unsigned long long lower = 0ull, upper = 0ull;
+            int ntasks = nseg, nlower = 0;
+            if (pass) {
+                for (int i0 = 0; i0 < nseg; i0 += 32) {
+                    const unsigned v = i0 + lane < nseg ? s_zm[i0 + lane] : 0u;
+                    lower |= (unsigned long long)__ballot_sync(kFull, (v & 0x00ffu) != 0u) << i0;
+                    upper |= (unsigned long long)__ballot_sync(kFull, (v & 0xff00u) != 0u) << i0;
+                }
+                if (2 * __popcll(lower | upper) > nwarps) {
+                    lower |= upper;
+                    upper = 0ull;
+                }
+                nlower = __popcll(lower);
+                ntasks = nlower + __popcll(upper);
+            }
 #pragma unroll 1
-            for (int sg = warp; sg < nseg; sg += nwarps) {
-                const unsigned zm = s_zm[sg];
-                if (pass && zm == 0u) continue;
+            for (int task = warp; task < ntasks; task += nwarps) {
+                int sg = task;
+                unsigned zm = 0u;
+                if (pass) {
+                    const bool up = task >= nlower;
+                    unsigned long long m = up ? upper : lower;
+#pragma unroll 1
+                    for (int k = up ? task - nlower : task; k > 0; --k) m &= m - 1ull;
+                    sg = __ffsll(m) - 1;
+                    zm = s_zm[sg];
+                    if (upper) zm &= up ? 0xff00u : 0x00ffu;
+                }
                 // the segment's planes: distances within their planes
                 const int z0 = sg * kSeg;
-                unsigned b = kInf;
+                unsigned b = kInf, r = 0u;
+                if (pass == 0 && lane < kSeg && z0 + lane < g.d) r = __ldg(rows + z0 + lane);
                 if (lane < kSeg && z0 + lane < g.d)
                     b = __ldg(p.base[j] + ((size_t)w * g.ntile + (yq >> 4)) * g.d + z0 + lane);
                 const uint32_t* const vp = p.vol[j] + (size_t)z0 * vplane + (size_t)yq * vrow + (size_t)w * 32 + lane;
@@ -441,13 +524,13 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
                         tw0 = __ldg(p.packed[1 - j] + o) & ~__ldg(p.packed[j] + o);
                         if (y + 1 < g.h) tw1 = __ldg(p.packed[1 - j] + o + p.pitch) & ~__ldg(p.packed[j] + o + p.pitch);
                     }
-#pragma unroll 1
+#pragma unroll 4
                     for (int s = 0; s < sg; ++s) {
                         const uint4 e = s_end[s * 32 + lane];
                         f0 = addmin2(f0, two(kSeg), e.z);
                         f1 = addmin2(f1, two(kSeg), e.w);
                     }
-#pragma unroll 1
+#pragma unroll 4
                     for (int s = nseg - 1; s > sg; --s) {
                         const uint4 e = s_end[s * 32 + lane];
                         c0 = addmin2(c0, two(kSeg), e.x);
@@ -468,56 +551,70 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
                 }
                 if (pass == 0) {
                     s_end[sg * 32 + lane] = make_uint4(c0, c1, f0, f1);
+                    zm = __ballot_sync(kFull, ((r >> (4 * (yq & 7))) & 0xfu) != 0u);
+                    if (lane == 0) s_zm[sg] = zm;
                     continue;
                 }
+                ((uint2*)s_tgt[warp])[(lane & 15) * 2 + (lane >> 4)] = make_uint2(tw0, tw1);
+                const uint32_t hist = s_hist_at + 4u * (unsigned)(j * bins);
+                unsigned dm = 0u;
+                auto count = [&](int i, int h) {  // the targets of plane h + i of the segment
+                    const uint2 v = s_v[i * 32 + lane];  // this lane's own
+                    const uint4 t4 = s_tgt[warp][h + i];
+                    const uint32_t tw[4] = {t4.x, t4.y, t4.z, t4.w};
+                    const unsigned dd[4] = {v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const unsigned in = (tw[r] >> lane) & 1u;
+                        red_shared_inc(hist + 4u * dd[r], in);
+                        dm = max(dm, in ? dd[r] : 0u);
+                        if constexpr (kMap) {
+                            if (in) {
+                                const size_t row = (size_t)(g.oz + z0 + h + i) * p.H + g.oy + 4 * yq + r;
+                                p.map[j][row * p.W + 32 * (g.wx0 + w) + lane] = (int32_t)dd[r];
+                            }
+                        }
+                    }
+                };
 #pragma unroll
                 for (int h = 0; h < kSeg; h += kHalf) {
                     __syncwarp();
 #pragma unroll
                     for (int i = 0; i < kHalf; ++i) s_v[i * 32 + lane] = make_uint2(V[h + i][0], V[h + i][1]);
+                    __syncwarp();
+                    // two planes at a time: their loads overlap
 #pragma unroll 1
-                    for (unsigned m = (zm >> h) & ((1u << kHalf) - 1u); m; m &= m - 1u) {
-                        const int i = __ffs(m) - 1;
-                        const uint2 v = s_v[i * 32 + lane];  // this lane's own
-                        const unsigned dd[4] = {v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16};
-#pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const uint32_t tw = __shfl_sync(kFull, (r & 1) ? tw1 : tw0, h + i + 16 * (r >> 1));
-                            if ((tw >> lane) & 1u) {
-                                atomicAdd(&s_hist[j * bins + dd[r]], 1u);
-                                if constexpr (kMap) {
-                                    const size_t row = (size_t)(g.oz + z0 + h + i) * p.H + g.oy + 4 * yq + r;
-                                    p.map[j][row * p.W + 32 * (g.wx0 + w) + lane] = (int32_t)dd[r];
-                                }
-                            }
+                    for (unsigned m = (zm >> h) & ((1u << kHalf) - 1u); m;) {
+                        const int i0 = __ffs(m) - 1;
+                        m &= m - 1u;
+                        count(i0, h);
+                        if (m) {
+                            count(__ffs(m) - 1, h);
+                            m &= m - 1u;
                         }
                     }
                 }
+                if (j) dmax[1] = max(dmax[1], (int)dm);
+                else dmax[0] = max(dmax[0], (int)dm);
             }
             __syncthreads();  // end planes complete; after the second pass the shared data are free
         }
     }
     // this CTA's counts
-    __syncthreads();
-#pragma unroll 1
+#pragma unroll
     for (int j = 0; j < 2; ++j) {
-        int m = 0;
-#pragma unroll 1
-        for (int t = threadIdx.x; t < bins; t += blockDim.x)
-            if (const unsigned v = s_hist[j * bins + t]) {
-                atomicAdd(p.hist[j] + t, (unsigned long long)v);
-                m = t;
-            }
-        m = __reduce_max_sync(kFull, m);
+        const int m = __reduce_max_sync(kFull, dmax[j]);
         if (lane == 0 && m) atomicMax(&s_max[j], m);
     }
+    __syncthreads();
+#pragma unroll 1
+    for (int j = 0; j < 2; ++j)
+        for (int t = threadIdx.x; t <= s_max[j] && t < bins; t += blockDim.x)
+            if (const unsigned v = s_hist[j * bins + t]) atomicAdd(p.hist[j] + t, (unsigned long long)v);
     __threadfence();
     __syncthreads();
     // the last CTA to finish decodes the result
     if (threadIdx.x == 0) {
-        if (s_max[0]) atomicMax(&p.state->hd[0], s_max[0]);
-        if (s_max[1]) atomicMax(&p.state->hd[1], s_max[1]);
-        __threadfence();
         s_last = atomicAdd(&p.state->done, 1u) == gridDim.x - 1u;
     }
     __syncthreads();
@@ -536,8 +633,8 @@ cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s) {
     const int nq = ((p.W + 31) / 32 + 3) / 4;
     const int nseg = (p.D + kSeg - 1) / kSeg;
     const size_t plane_sm = sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)nq * 4 * kPlaneWarps * 32);
-    const int dwarps = nseg > 8 ? kDepthMaxWarps : 4;
-    const size_t depth_sm = depth_smem(dwarps, nseg, p.W + p.H + p.D);
+    const int dwarps = nseg > 2 ? kDepthMaxWarps : 4;
+    const size_t depth_sm = depth_smem(dwarps, nseg, p.W + p.H + p.D, p.ncols);
     // the limit of dynamic shared memory, once per device for the largest size
     // (calls of other sizes may run on other threads)
     static std::atomic<bool> raised[64];
@@ -545,7 +642,7 @@ cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (dev >= 64 || !raised[dev].load(std::memory_order_acquire)) {
-        const int lim = 226 * 1024;
+        const int lim = 200 * 1024;  // above any size taken (dt_fits), with the static part below 227 KB
         e = cudaFuncSetAttribute(&dt_plane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
         if (e == cudaSuccess)
             e = cudaFuncSetAttribute(&dt_depth_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);

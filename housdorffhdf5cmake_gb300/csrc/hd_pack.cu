@@ -317,10 +317,12 @@ __device__ __forceinline__ void put_words(const PackWalk& k, const PackSpan& n, 
 template <bool kLabel>
 __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const PairDesc* __restrict__ descs, int npairs,
                                                                long long ntiles, int label,
-                                                               const __grid_constant__ PairDesc one, Ctl* ctl) {
+                                                               const __grid_constant__ PairDesc one, Ctl* ctl, uint32_t* zero, int nzero) {
     __shared__ uint32_t s_bits_all[kPackWarps][2][kBitWords];
     cudaTriggerProgrammaticLaunchCompletion();  // the distance transform's CTAs may take over as these end
-    if (ctl && blockIdx.x == 0 && threadIdx.x == 0) *ctl = Ctl{};  // nobody else uses it before the set-up
+    // nobody uses these before the next kernel
+    if (ctl && blockIdx.x == 0 && threadIdx.x == 0) *ctl = Ctl{};
+    for (int t = blockIdx.x * kPackThreads + threadIdx.x; t < nzero; t += gridDim.x * kPackThreads) zero[t] = 0u;
     const long long per = (ntiles + gridDim.x - 1) / gridDim.x;
     long long tile = (long long)blockIdx.x * per;
     const long long t_hi = min(ntiles, tile + per);
@@ -667,7 +669,7 @@ __global__ void map_init_kernel(const __grid_constant__ PairDesc P, int32_t* map
 namespace hdk {
 
 cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, int grid, int label, int sms,
-                        cudaStream_t s, const PairDesc* one, Ctl* ctl) {
+                        cudaStream_t s, const PairDesc* one, Ctl* ctl, uint32_t* zero, int nzero) {
     // one wave of resident CTAs (per device and variant, from the occupancy calculator)
     static int resident[2][64] = {{0}};
     static int per_sm_of[2][64] = {{0}};
@@ -689,8 +691,8 @@ cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, i
     if (grid > ntiles) grid = (int)ntiles;
     if (grid < 1) grid = 1;
     const PairDesc P = one ? *one : PairDesc{};
-    if (label) pack_kernel<true><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, label, P, ctl);
-    else pack_kernel<false><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, 0, P, ctl);
+    if (label) pack_kernel<true><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, label, P, ctl, zero, nzero);
+    else pack_kernel<false><<<grid, kPackThreads, 0, s>>>(d_descs, npairs, ntiles, 0, P, ctl, zero, nzero);
     return cudaGetLastError();
 }
 
