@@ -168,7 +168,7 @@ def bench_ours(args):
         blocking.append(e0.elapsed_time(e1))
     phases = phases[-2:]
     # warm-up of the enqueue-only entries used in the timed regions (the
-    # first pipelined calls set up the split SMs and allocate the six
+    # first pipelined calls set up the split SMs and allocate the
     # workspaces, one per call)
     outs = torch.empty((args.steps, hd.RESULT_BYTES), dtype=torch.uint8, device=dev)
     for w in range(max(args.warmup, 6)):
@@ -404,8 +404,8 @@ def bench_ours(args):
                 "blocking_path": "hd_compute_u8, one call per pair, masks read in place over the host link",
                 "staged_copy_ms_per_step": round(staged_ms, 4)},
         "gpu_launches": 3 * args.steps,  # per pair: pack, in-plane distances, distances at the targets (decodes the result too)
-        "value_path": "hd_compute_u8_device_pipelined x K, hd_pipeline_flush: packing and set-up on 56 SMs, "
-                      "consecutive pairs dilating side by side on three groups of 32 (green contexts, six "
+        "value_path": "hd_compute_u8_device_pipelined x K, hd_pipeline_flush: packing on 56 SMs, "
+                      "consecutive pairs' distances side by side on two groups of 48 (green contexts, four "
                       "workspaces in turn)",
         "async_serial": {"path": "hd_compute_u8_device_async x K (each pair after the previous one)",
                          "ms_per_step": round(serial_ms, 4), "pairs_per_s": round(1000.0 / serial_ms, 1)},

@@ -191,25 +191,20 @@ using GreenDestroyFn = CUresult (*)(CUgreenCtx);
 }  // namespace
 
 // The split path's SM partitions (green contexts; the granularity is 8 SMs
-// on GB300).  One dilation partition: packing and set-up on 48 SMs, each
-// pair's dilation on the other 104 in turn.  Two or three: packing and
-// set-up on 40 / 56 SMs, the rest in equal groups (56 / 32 SMs),
-// consecutive pairs dilating side by side (workspace i on group i % parts,
-// two workspaces per group in turn).  A single pair's dilation is
-// latency-bound: on fewer SMs it takes longer, but much less than in
-// proportion (the 512x512x256 pairs: 0.124 / 0.077 ms on 104 SMs, 0.178 /
-// 0.077 ms on 56, 0.179 ms on average over both on 32), so side by side the groups
-// finish more pairs per second.  Measured on those two pairs alternating
-// (0.142 ms per pair unsplit): one partition with 24 / 32 / 48 / 64
-// packing SMs 0.155 / 0.127 / 0.107 / 0.121 ms per pair; two partitions
-// with 40 / 56 packing SMs (groups of 56 / 48) 0.094 / 0.102 ms, with one
-// workspace per group 0.137 ms (a packing waited for the dilation before
-// last in its group); three with 56 / 32 packing SMs (groups of 32 / 40)
-// 0.080 / 0.115 ms: packing and set-up on 56 SMs (0.073 ms a pair) set the
-// pace.  A lone pair's latency is higher on fewer dilation SMs (0.30 ms
-// on 56 against 0.23 ms on 104).
-constexpr int kSplitDilations = 3;
-constexpr unsigned kSplitPrepSms[hd_context::kMaxDilationParts] = {48, 40, 56};  // by dilation partitions
+// on GB300): packing (and set-up) on 56 SMs, the rest in equal groups whose
+// distance transforms or dilations run side by side (workspace i on group
+// i % parts, two workspaces per group in turn).  After the packing a single
+// pair is bound by latency: on fewer SMs it takes longer, but much less than
+// in proportion (512x512x256, 6-neighbour element: 27 / 36 / 44 us on 104 / 48
+// / 32 SMs), so side by side the groups finish more pairs per second, until
+// the packing (44 us on 56 SMs, 55 on 40) sets the pace.  Measured, us per
+// pair of 512x512x256 under the 6- / 18-neighbour element and of 301x287x173
+// likewise: two groups of 48 (56 packing) 50 / 64, 27 / 34; of 40 (72) 51 /
+// 66, 27 / 33; of 32 (88) 56 / 75, 28 / 34; of 56 (40) 59 / 70, 29 / 39; three
+// of 32 (56) 55 / 72, 28 / 35; one of 96 (56) 52 / 81, 28 / 55; unsplit 58 /
+// 104, 34 / 70.
+constexpr int kSplitDilations = 2;
+constexpr unsigned kSplitPrepSms[hd_context::kMaxDilationParts] = {56, 56, 56};  // by dilation partitions
 
 // HD_SPLIT_DILATIONS (1 to 3) in the environment overrides the dilation
 // partitions, HD_SPLIT_SMS the packing SMs: 0 = no split (profilers that
