@@ -6,15 +6,23 @@
 //   pa, pb      the full volume bit-packed along x: 32 voxels per uint32,
 //               bit i of word w of row (y, z) is voxel x = 32 w + i;
 //               wxf = ceil(W / 32) words per row, rows padded with zero
-//               words to a multiple of 4 (packed_pitch), word w of row
-//               (y, z) at (z * H + y) * packed_pitch + w
+//               words to a multiple of 4 (packed_pitch).  A plane is stored
+//               in columns of 4 words: word w of row (y, z) is at
+//               z * H * packed_pitch + ((w / 4) * H + y) * 4 + w % 4, so that
+//               a warp whose lanes hold consecutive rows of a column reads
+//               512 contiguous bytes.  Against rows of words (32 rows in as
+//               many sectors of their own): 512x512x256 under the
+//               18-neighbour element 57 to 74 against 63 to 78 us of
+//               dilation, 256 ragged pairs 1.18 to 1.54 against 1.24 to 1.62
+//               ms, their packing 1.05 against 1.03 ms
 //   per direction (a "job": dilate a source mask until it covers a target):
 //     buf[0], buf[1]  ping-pong dilation state over the job's domain
 //     U               target voxels not yet covered (one-step kernel; the
 //                     blocked kernel finds newly covered voxels as target
 //                     voxels in a step's result but not in its input)
-//               domain layout [z][y][pitch] words, pitch = ceil(wx / 4) * 4,
-//               pad words zero.  The domain is the bounding box of A u B with
+//               domain layout, pitch = ceil(wx / 4) * 4, pad words zero:
+//               columns of 4 words as above for the blocked kernel,
+//               [z][y][pitch] words for the one-step kernel.  The domain is the bounding box of A u B with
 //               x widened to whole words (6-neighbour element), widened by
 //               one more word in x and one row and plane in y and z
 //               (18-neighbour element: shortest paths may step one voxel
@@ -190,8 +198,9 @@ struct __align__(128) Job {
     // blocked kernel: the source (state of the first iteration) and the
     // target, read-only: either the packed masks pa / pb read in place
     // (domain rows start on 16-byte boundaries) or crops of them in the
-    // domain layout; domain word (x, y, z) is at
-    // vol + ((z + vz0) * vh + y + vy0) * vpitch + vx0 + x
+    // domain layout; domain word (x, y, z) is word x + vx0 (vx0 a multiple of
+    // 4), row y + vy0, plane z + vz0 of a volume of vh rows of vpitch words
+    // in columns of 4 words
     const uint32_t* vol[2];
     int32_t wx, h, d;          // domain: words per row, rows, planes
     int32_t pitch;             // row pitch (words)

@@ -124,7 +124,6 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
     if (I.n_a == 0 || I.n_b == 0) return;
     const unsigned long long rem[2] = {I.n_b - I.n_ab, I.n_a - I.n_ab};
     const Geom g = dt_geom(I);
-    const int pitch = p.pitch;
     // planes per CTA: as many as its warps have tiles for, but no fewer CTAs than the grid
     const int nact = (rem[0] > 0) + (rem[1] > 0);
     const int G = max(1, min(kPlaneWarps / g.ntile, nact * g.d / (int)gridDim.x));
@@ -138,9 +137,10 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
         const int z = (nact == 2 && j ? u - groups : u) * G + pl;
         const bool act = pl < G && z < g.d;
         const int ya = t * 64 + lane, yb = ya + 32;
-        const uint32_t* const src = p.packed[j] + ((size_t)(g.oz + (act ? z : 0)) * p.H + g.oy) * pitch;
-        const uint4* const ra = (const uint4*)(src + (size_t)(ya < g.h ? ya : 0) * pitch) + q0;
-        const uint4* const rb = (const uint4*)(src + (size_t)(yb < g.h ? yb : 0) * pitch) + q0;
+        // rows ya, yb of the plane's columns of 4 words, p.H apart
+        const uint4* const src = (const uint4*)(p.packed[j] + (size_t)(g.oz + (act ? z : 0)) * p.H * p.pitch) + g.oy;
+        const uint4* const ra = src + (ya < g.h ? ya : 0);
+        const uint4* const rb = src + (yb < g.h ? yb : 0);
         const ptrdiff_t other = (const uint4*)p.packed[1 - j] - (const uint4*)p.packed[j];
         const bool va = act && ya < g.h, vb = act && yb < g.h;
         const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
@@ -151,8 +151,9 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
         if (act) {
 #pragma unroll 1
             for (int q = g.nq - 1; q >= 0; --q) {
-                const uint4 a = va ? __ldg(ra + q) : zero, b = vb ? __ldg(rb + q) : zero;
-                const uint4 c = va ? __ldg(ra + other + q) : zero, d = vb ? __ldg(rb + other + q) : zero;
+                const ptrdiff_t o = (ptrdiff_t)(q0 + q) * p.H;
+                const uint4 a = va ? __ldg(ra + o) : zero, b = vb ? __ldg(rb + o) : zero;
+                const uint4 c = va ? __ldg(ra + other + o) : zero, d = vb ? __ldg(rb + other + o) : zero;
                 const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
                 const uint32_t ta[4] = {c.x & ~a.x, c.y & ~a.y, c.z & ~a.z, c.w & ~a.w};
                 const uint32_t tb[4] = {d.x & ~b.x, d.y & ~b.y, d.z & ~b.z, d.w & ~b.w};
@@ -186,15 +187,16 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
         }
         unsigned la = kInf, lb = kInf;
         uint32_t* const vol = p.vol[j] + (size_t)(act ? z : 0) * g.nyq * vrow;
-        const uint32_t* const pa = (const uint32_t*)(ra - q0);
-        const uint32_t* const pb = (const uint32_t*)(rb - q0);
-        uint32_t na = va ? __ldg(pa + g.wx0) : 0u, nb = vb ? __ldg(pb + g.wx0) : 0u;
+        const uint32_t* const pa = (const uint32_t*)ra;
+        const uint32_t* const pb = (const uint32_t*)rb;
+        auto word = [&](int w) { return (ptrdiff_t)(w & ~3) * p.H + (w & 3); };
+        uint32_t na = va ? __ldg(pa + word(g.wx0)) : 0u, nb = vb ? __ldg(pb + word(g.wx0)) : 0u;
 #pragma unroll 1
         for (int w = g.wx0; w <= g.w1; ++w) {
             const uint32_t ua = na, ub = nb;
             if (w < g.w1) {  // the next word's
-                na = va ? __ldg(pa + w + 1) : 0u;
-                nb = vb ? __ldg(pb + w + 1) : 0u;
+                na = va ? __ldg(pa + word(w + 1)) : 0u;
+                nb = vb ? __ldg(pb + word(w + 1)) : 0u;
             }
             {
                 const uint32_t rcw = act ? s_r[((w - 4 * q0) * kPlaneWarps + warp) * 32 + lane] : 0u;
@@ -520,9 +522,10 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
                 if (pass) {
                     const int z = z0 + (lane & 15), y = 4 * yq + 2 * (lane >> 4);
                     if (z < g.d && y < g.h) {
-                        const size_t o = ((size_t)(g.oz + z) * p.H + g.oy + y) * p.pitch + g.wx0 + w;
+                        const int wf = g.wx0 + w;
+                        const size_t o = ((size_t)(g.oz + z) * p.pitch + (wf & ~3)) * p.H + 4 * (g.oy + y) + (wf & 3);
                         tw0 = __ldg(p.packed[1 - j] + o) & ~__ldg(p.packed[j] + o);
-                        if (y + 1 < g.h) tw1 = __ldg(p.packed[1 - j] + o + p.pitch) & ~__ldg(p.packed[j] + o + p.pitch);
+                        if (y + 1 < g.h) tw1 = __ldg(p.packed[1 - j] + o + 4) & ~__ldg(p.packed[j] + o + 4);
                     }
 #pragma unroll 4
                     for (int s = 0; s < sg; ++s) {

@@ -5,7 +5,7 @@
 //               per uint32 along x (the prototype packs along z, :598-631),
 //               with |A|, |B|, |A n B| and the bounding box of A u B (x in
 //               whole words).  One pass over the bytes, 128-bit streaming
-//               loads; rows stored at a pitch of a multiple of 4 words.
+//               loads; words stored in columns of 4 (see hd_device.cuh).
 // setup_kernel  replaces firstMetaPrepareKernel (hello.cu:763-877): writes
 //               the job descriptors and queues every brick of each job for
 //               its first step; for the one-step kernel it also crops the
@@ -163,6 +163,10 @@ struct PackWalk {
         y += d;
         if (y >= H) y %= H;
     }
+    // word w of row r = y + H z in the packed volume
+    __device__ __forceinline__ size_t at(unsigned r, unsigned w, unsigned y) const {
+        return (size_t)(r - y) * pitch + ((size_t)(w >> 2) * H + y) * 4u + (w & 3u);
+    }
     __device__ __forceinline__ void next_words(unsigned& r, unsigned& w, unsigned& y) const { step(r, w, y, dq, dr); }
     __device__ __forceinline__ void next_span(unsigned& r, unsigned& w, unsigned& y) const { step(r, w, y, tq, tr); }
 };
@@ -291,7 +295,7 @@ __device__ __forceinline__ void put_words(const PackWalk& k, const PackSpan& n, 
                 const unsigned o = d + n.sh[m];
                 out[m] = __funnelshift_r(s_bits[m][o >> 5], s_bits[m][(o >> 5) + 1], o & 31u) & mask;
             }
-            const size_t o = (size_t)r * k.pitch + w;
+            const size_t o = k.at(r, w, y);
             k.dst[0][o] = out[0];
             k.dst[1][o] = out[1];
             if (last)  // the row's last word also writes its padding (up to 3 words)
@@ -353,7 +357,7 @@ __device__ __forceinline__ void pack_aligned(const PackWalk& k, unsigned t0, uns
 #pragma unroll
         for (int i = 0; i < kWords; ++i) {
             if (t0 + 32u * i + lane < k.total) {
-                const size_t o = (size_t)r * k.pitch + w;
+                const size_t o = k.at(r, w, y);
                 k.dst[0][o] = out[0][i];
                 k.dst[1][o] = out[1][i];
                 if (w + 1u == k.wxf)
@@ -639,15 +643,27 @@ __device__ __forceinline__ long long setup_tile(const PairDesc& P, long long til
     const long long words = min(words_all, w_hi);
     const int vpitch = packed_pitch(P.W);
     for (long long t = w_lo + tid0; t < words; t += nthr) {
-        // domain word index < 2^31: 32-bit divisions
+        // domain word index < 2^31: 32-bit divisions.  Rows of pitch words
+        // for the one-step kernel, columns of 4 words for the blocked one
         const unsigned tu = (unsigned)t;
-        const unsigned r = tu / (unsigned)m.pitch;
-        const int w = (int)(tu - r * (unsigned)m.pitch);
+        unsigned r;
+        int w, yl, zl;
+        if (one_step) {
+            r = tu / (unsigned)m.pitch;
+            w = (int)(tu - r * (unsigned)m.pitch);
+            zl = (int)(r / (unsigned)m.h);
+            yl = (int)(r - (unsigned)zl * (unsigned)m.h);
+        } else {
+            r = tu >> 2;
+            const unsigned c = r / (unsigned)m.h, nq = (unsigned)m.pitch >> 2;
+            yl = (int)(r - c * (unsigned)m.h);
+            zl = (int)(c / nq);
+            w = (int)(4u * (c - (unsigned)zl * nq) + (tu & 3u));
+        }
         uint32_t a = 0, b = 0;
         if (w < m.wx) {
-            const unsigned zq = r / (unsigned)m.h;
-            const int yl = (int)(r - zq * (unsigned)m.h), zl = (int)zq;
-            const long long src = ((long long)(m.oz + zl) * P.H + (m.oy + yl)) * vpitch + m.wx0 + w;
+            const int wf = m.wx0 + w;
+            const long long src = ((long long)(m.oz + zl) * vpitch + (wf & ~3)) * P.H + 4ll * (m.oy + yl) + (wf & 3);
             a = __ldg(P.pa + src);
             b = __ldg(P.pb + src);
         }

@@ -100,18 +100,19 @@ struct TbItem {
 };
 
 // Where this lane's rows of a streamed plane come from: domain plane z, row
-// y, words wx0 .. wx0 + 3 of the brick are at src + (z + zoff) * plane +
-// rowoff[k] for the lane's row k (brick row R lane + k).  The level-0 state
+// y, words wx0 .. wx0 + 3 of the brick (one column of 4 words) are at src +
+// (z + zoff) * plane + rowoff[k] for the lane's row k (brick row R lane + k),
+// the columns beside it `col` words before and after.  The level-0 state
 // is the job's ping-pong buffer, except in the job's first iteration, which
-// reads the source (vol[0]); the target always comes from vol[1].  Every
-// row copy is one 16-byte copy: the domain layout and the packed masks (rows
-// padded to a multiple of 4 words, read in place only when the domain starts
-// on a multiple of 4 words) keep a brick's 4 words in its row, and those past
-// the domain are row padding or outside the bounding box of A u B (zero).
+// reads the source (vol[0]); the target always comes from vol[1].  A plane's
+// rows are one contiguous copy of a warp: the domain layout and the packed
+// masks (read in place only when the domain starts on a multiple of 4 words)
+// keep columns of 4 words, and those past the domain are row padding or
+// outside the bounding box of A u B (zero).
 template <int R>
 struct TbRow {
     const uint32_t* src;
-    int plane, zoff, z0, Dd;
+    int plane, col, zoff, z0, Dd;
     int rowoff[R];
     bool rowv[R], hl_ok[R], hr_ok[R];
 };
@@ -127,9 +128,9 @@ __device__ __forceinline__ TbRow<tb_rows(T)> tb_row(const TbItem& it, bool targe
     const int Wx = Jp->wx, Hd = Jp->h;
     const int wx0 = it.bx * IW;
     const bool first = target || it.iter == 0;
-    const int pitch = first ? Jp->vpitch : Jp->pitch;
     const int rbase = first ? Jp->vy0 : 0;
-    const int xbase = (first ? Jp->vx0 : 0) + wx0;
+    w.col = 4 * (first ? Jp->vh : Hd);
+    const int cbase = ((first ? Jp->vx0 >> 2 : 0) + it.bx) * w.col;
     w.src = first ? Jp->vol[target ? 1 : 0] : Jp->buf[it.iter & 1];
     w.plane = first ? Jp->vpitch * Jp->vh : Jp->pitch * Hd;
     w.zoff = first ? Jp->vz0 : 0;
@@ -137,7 +138,7 @@ __device__ __forceinline__ TbRow<tb_rows(T)> tb_row(const TbItem& it, bool targe
     for (int k = 0; k < R; ++k) {
         const int y = it.by * BYI - T + lane * R + k;
         w.rowv[k] = y >= 0 && y < Hd;
-        w.rowoff[k] = ((w.rowv[k] ? y : 0) + rbase) * pitch + xbase;
+        w.rowoff[k] = cbase + 4 * ((w.rowv[k] ? y : 0) + rbase);
         w.hl_ok[k] = w.rowv[k] && wx0 > 0;
         w.hr_ok[k] = w.rowv[k] && wx0 + IW < Wx;
     }
@@ -163,8 +164,8 @@ __device__ __forceinline__ void tb_copy_plane(const TbRow<tb_rows(T)>& w, int r,
         const uint32_t s_in = base + (uint32_t)(((slot * SM::R + k) * 32 + lane) * 16);
         const uint32_t s_h = base + SM::kInBytes + (uint32_t)(((slot * SM::R + k) * 32 + lane) * 8);
         cp_async16(s_in, gp, ok ? 16u : 0u);
-        cp_async4(s_h, (ok && w.hl_ok[k]) ? gp - 1 : gp, (ok && w.hl_ok[k]) ? 4u : 0u);
-        cp_async4(s_h + 4, (ok && w.hr_ok[k]) ? gp + IW : gp, (ok && w.hr_ok[k]) ? 4u : 0u);
+        cp_async4(s_h, (ok && w.hl_ok[k]) ? gp - w.col + (IW - 1) : gp, (ok && w.hl_ok[k]) ? 4u : 0u);
+        cp_async4(s_h + 4, (ok && w.hr_ok[k]) ? gp + w.col : gp, (ok && w.hr_ok[k]) ? 4u : 0u);
     }
     cp_async_commit();
 }
@@ -479,7 +480,7 @@ __device__ __forceinline__ void tb_compute(const SolveParams& p, const TbItem& i
 #pragma unroll
                 for (int k = 0; k < R; ++k) {
                     if (inter[k] && z < w.Dd) {
-                        const int off = z * bplane + (brow0 + k) * Jp->pitch + wx0;
+                        const int off = z * bplane + 4 * (it.bx * Jp->h + brow0 + k);
                         const uint4 o4 = make_uint4(out[k][1], out[k][2], out[k][3], out[k][4]);
                         *reinterpret_cast<uint4*>(dst + off) = o4;
                         if (dst2) *reinterpret_cast<uint4*>(dst2 + off) = o4;
