@@ -333,6 +333,8 @@ struct PairPlan {
     long long bricks;       // per job, upper bound
     int kmax;
     long long tiles;        // full-volume 32^3 tiles (instrumented runs)
+    int ncols;
+    size_t off_cols;
     size_t off_pa, off_pb, off_jb[2][3], off_in_a, off_in_b, off_hist, off_tstamp[2], off_tcount[2];
     unsigned long long brick0;
 };
@@ -376,7 +378,9 @@ hd_status decode_result(const hdk::PairInfo& I, const hdk::JobState& s0, const h
 }
 
 bool dt_takes(int se, const PairIn* pairs, int n) {
-    return se == 0 && n == 1 && hdk::dt_fits(pairs[0].W, pairs[0].H, pairs[0].D);
+    bool ok = se == 0;
+    for (int i = 0; i < n && ok; ++i) ok = hdk::dt_fits(pairs[i].W, pairs[i].H, pairs[i].D);
+    return ok;
 }
 
 bool loop_asked(const hd_options& o) {
@@ -385,9 +389,9 @@ bool loop_asked(const hd_options& o) {
 }
 
 Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n, bool dt) {
-    // built-in default: the distance transform for single pairs under the
-    // 6-neighbour element unless an option asks for the dilation loop (a
-    // kernel, a brick shape, a cap on its steps or on its waits); else
+    // built-in default: the distance transform under the 6-neighbour element
+    // unless an option asks for the dilation loop (a kernel, a brick shape, a
+    // cap on its steps or on its waits) or a pair is beyond its sizes; else
     // (the autotuner's winners on GB300) the blocked kernel with
     // 4 x (32 - 2 steps) x 8 bricks; 4 steps per barrier for a single
     // pair (fewest barriers), 2 for batches (the work per barrier is large)
@@ -419,6 +423,39 @@ Shape pick_shape(hd_context* ctx, int se, const PairIn* pairs, int n, bool dt) {
 const void* solve_fn_of(int se, const Shape& sh) {
     if (sh.kernel == 2) return hdk::solve_tb_kernel_ptr(se, sh.steps, sh.bz);
     return hdk::solve_kernel_ptr(se, sh.bxw, sh.bz);
+}
+
+// A group of pairs of one launch of the distance transform.
+struct DtGroupPlan {
+    int first, n;
+    size_t off_list, bytes;
+};
+
+// Enqueues the groups of a batch's distance transform on the context's streams
+// in turn, after the work on s, and makes s wait for them.
+static cudaError_t run_dt_groups(hd_context* ctx, const hdk::DtPair* pairs, const hdk::DtPair* d_pairs,
+                                 const std::vector<DtGroupPlan>& plan, hdk::DtGroup* d_groups, char* dbase, cudaStream_t s) {
+    constexpr int kN = hd_context::kDtStreams;
+    cudaError_t e = cudaSuccess;
+    if (!ctx->dt_fork) e = cudaEventCreateWithFlags(&ctx->dt_fork, cudaEventDisableTiming);
+    for (int i = 0; i < kN && e == cudaSuccess; ++i) {
+        if (!ctx->dt_stream[i]) e = cudaStreamCreateWithFlags(&ctx->dt_stream[i], cudaStreamNonBlocking);
+        if (e == cudaSuccess && !ctx->dt_join[i]) e = cudaEventCreateWithFlags(&ctx->dt_join[i], cudaEventDisableTiming);
+    }
+    const int groups = (int)plan.size();
+    if (e == cudaSuccess) e = cudaEventRecord(ctx->dt_fork, s);
+    for (int i = 0; i < std::min(kN, groups) && e == cudaSuccess; ++i) e = cudaStreamWaitEvent(ctx->dt_stream[i], ctx->dt_fork, 0);
+    for (int g = 0; g < groups && e == cudaSuccess; ++g)
+        e = hdk::launch_dt_group(pairs + plan[g].first, d_pairs + plan[g].first, plan[g].n, (uint32_t*)(dbase + plan[g].off_list),
+                                 d_groups + g, ctx->sm_count, ctx->dt_stream[g % kN]);
+    for (int i = 0; i < std::min(kN, groups) && e == cudaSuccess; ++i) {
+        e = cudaEventRecord(ctx->dt_join[i], ctx->dt_stream[i]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(s, ctx->dt_join[i], 0);
+    }
+    if (e != cudaSuccess)  // nothing of this call may run into the next one's buffers
+        for (cudaStream_t st : ctx->dt_stream)
+            if (st) cudaStreamSynchronize(st);
+    return e;
 }
 
 hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s, const RunOpts& ro,
@@ -477,11 +514,26 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     const size_t off_states = take(sizeof(JobState) * 2 * n);
     const size_t off_infos = take(sizeof(PairInfo) * n);
     const size_t off_descs = take(sizeof(PairDesc) * n);
-    const size_t upload_bytes = cur;           // [ctl .. descs]
+    // Distance transform: pairs in groups of at most kDtMaxGroup pairs and 2^29
+    // voxels (256 ragged pairs: 2^27 0.99, 2^28 0.80, 2^29 and 2^30 0.79 ms: a
+    // group must fill the GPU, and its workspace, two bytes per voxel, grows)
+    std::vector<DtGroupPlan> groups;
+    for (int i = 0, vox = 0; dt && i < n; ++i) {
+        constexpr long long kGroupVoxels = 1 << 29;
+        const long long v = (long long)pairs[i].W * pairs[i].H * pairs[i].D;
+        if (i == 0 || vox + v > kGroupVoxels || groups.back().n == hdk::kDtMaxGroup) {
+            groups.push_back(DtGroupPlan{i, 0, 0, 0});
+            vox = 0;
+        }
+        vox += (int)std::min(v, kGroupVoxels);
+        ++groups.back().n;
+    }
+    const size_t off_dtp = dt && n > 1 ? take(sizeof(hdk::DtPair) * n) : 0;
+    const size_t off_groups = dt && n > 1 ? take(sizeof(hdk::DtGroup) * groups.size()) : 0;
+    const size_t upload_bytes = cur;           // [ctl .. descs, distance-transform pairs]
     const size_t off_jobs = take(sizeof(Job) * 2 * n);
-    const int ncols = dt ? hdk::dt_cols(pairs[0].W, pairs[0].H) : 0;
-    const size_t off_cols = take(sizeof(uint32_t) * 2 * ncols);
     size_t hist_words = 0;
+    long long cols_words = 0;  // per direction
     unsigned long long total_bricks = 0;
     int kmax_all = 0;
     for (int i = 0; i < n; ++i) {
@@ -499,8 +551,12 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         q.tiles = (long long)((P.W + 31) / 32) * ((P.H + 31) / 32) * ((P.D + 31) / 32);
         q.brick0 = total_bricks;
         total_bricks += 2ULL * (unsigned long long)q.bricks;
+        q.ncols = dt ? hdk::dt_cols(P.W, P.H) : 0;
+        q.off_cols = sizeof(uint32_t) * 2 * (size_t)cols_words;  // from off_cols
+        cols_words += q.ncols;
         hist_words += 2ULL * (kmax + 1);
     }
+    const size_t off_cols = take(sizeof(uint32_t) * 2 * cols_words);
     const size_t off_hist = take(sizeof(uint64_t) * hist_words);
     size_t hcur = 0;
     for (int i = 0; i < n; ++i) {
@@ -513,15 +569,8 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         PairPlan& q = plan[i];
         q.off_pa = take(4ULL * q.full_words);
         q.off_pb = take(4ULL * q.full_words);
-        for (int j = 0; j < 2; ++j) {
-            if (dt) {
-                q.off_jb[j][0] = take(4ULL * hdk::dt_vol_words(pairs[i].W, pairs[i].H, pairs[i].D));
-                q.off_jb[j][1] = take(2ULL * hdk::dt_bases(pairs[i].W, pairs[i].H, pairs[i].D));
-                q.off_jb[j][2] = take(8ULL * hdk::dt_bases(pairs[i].W, pairs[i].H, pairs[i].D));
-            } else {
-                for (int b = 0; b < 3; ++b) q.off_jb[j][b] = take(4ULL * q.dom_words);
-            }
-        }
+        for (int j = 0; j < 2 && !dt; ++j)
+            for (int b = 0; b < 3; ++b) q.off_jb[j][b] = take(4ULL * q.dom_words);
         const size_t nb = (size_t)pairs[i].W * pairs[i].H * pairs[i].D;
         q.off_in_a = (pairs[i].host_a && !ro.async_out) ? take(nb) : 0;
         q.off_in_b = (pairs[i].host_b && !ro.async_out) ? take(nb) : 0;
@@ -530,6 +579,39 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
                 q.off_tstamp[j] = take(sizeof(int32_t) * q.tiles);
                 q.off_tcount[j] = take(sizeof(uint64_t) * (q.kmax + 1));
             }
+        }
+    }
+    // Distance transform: the groups take kDtStreams workspaces and streams in turn.
+    for (size_t g = 0; g < groups.size(); ++g) {
+        DtGroupPlan& G = groups[g];
+        size_t bytes = 0;
+        auto put = [&](size_t b) {
+            const size_t o = bytes;
+            bytes = align_up(bytes + std::max<size_t>(b, 1));
+            return o;
+        };
+        size_t columns = 0;
+        for (int i = G.first; i < G.first + G.n; ++i) {
+            const PairIn& P = pairs[i];
+            columns += hdk::dt_list(P.W, P.H);
+            for (int j = 0; j < 2; ++j) {
+                plan[i].off_jb[j][0] = put(4ULL * hdk::dt_vol_words(P.W, P.H, P.D));
+                plan[i].off_jb[j][1] = put(2ULL * hdk::dt_bases(P.W, P.H, P.D));
+                plan[i].off_jb[j][2] = put(8ULL * hdk::dt_bases(P.W, P.H, P.D));
+            }
+        }
+        G.off_list = n > 1 ? put(4ULL * columns) : 0;
+        G.bytes = bytes;
+    }
+    for (int slot = 0; slot < hd_context::kDtStreams; ++slot) {
+        size_t need = 0;
+        for (size_t g = slot; g < groups.size(); g += hd_context::kDtStreams) need = std::max(need, groups[g].bytes);
+        const size_t at = need ? take(need) : 0;
+        for (size_t g = slot; g < groups.size(); g += hd_context::kDtStreams) {
+            groups[g].off_list += at;
+            for (int i = groups[g].first; i < groups[g].first + groups[g].n; ++i)
+                for (auto& o : plan[i].off_jb)
+                    for (size_t& b : o) b += at;
         }
     }
     const size_t total_bytes = cur;
@@ -715,6 +797,40 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         if (!dt) setup_tiles += hdk::setup_tiles_of(P.W, P.H, P.D, setup_mode, bxw, by, bz);
     }
 
+    const float pct = (ctx->opt.percentile > 0.f && ctx->opt.percentile <= 1.f) ? ctx->opt.percentile : 0.95f;
+    hd_result* const hres = async ? nullptr : (hd_result*)(hbase + upload_bytes);  // synchronous calls: pinned host memory
+    auto dt_pair = [&](int i) {
+        const PairPlan& q = plan[i];
+        hdk::DtPair d{};
+        d.info = hdesc[i].info;
+        d.packed[0] = hdesc[i].pa;
+        d.packed[1] = hdesc[i].pb;
+        for (int j = 0; j < 2; ++j) {
+            d.vol[j] = (uint32_t*)(dbase + q.off_jb[j][0]);
+            d.base[j] = (uint16_t*)(dbase + q.off_jb[j][1]);
+            d.rows[j] = (uint32_t*)(dbase + q.off_jb[j][2]);
+            d.hist[j] = hdesc[i].hist[j];
+        }
+        d.cols = (uint32_t*)(dbase + off_cols + q.off_cols);
+        d.ncols = q.ncols;
+        d.state = (hdk::DtState*)(dbase + off_states + 2 * sizeof(JobState) * i);  // the plane kernel zeroes it
+        d.map[0] = ro.map_b;
+        d.map[1] = ro.map_a;
+        d.W = pairs[i].W;
+        d.H = pairs[i].H;
+        d.D = pairs[i].D;
+        d.pitch = hdk::packed_pitch(pairs[i].W);
+        d.kmax = q.kmax;
+        d.pct = pct;
+        d.out = async ? ro.async_out : hres + i;
+        return d;
+    };
+    hdk::DtPair* const hdtp = (hdk::DtPair*)(hbase + off_dtp);
+    if (dt && n > 1) {
+        for (int i = 0; i < n; ++i) hdtp[i] = dt_pair(i);
+        std::memset(hbase + off_groups, 0, sizeof(hdk::DtGroup) * groups.size());
+    }
+
     // ---- uploads ----------------------------------------------------------
     if (!direct) {
         e = cudaMemcpyAsync(dbase, hbase, upload_bytes, cudaMemcpyHostToDevice, sq);
@@ -753,7 +869,8 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     const bool stime = split && ctx->opt.record_timings != 0 && ctx->split.ev[0] != nullptr;
     if (stime) cudaEventRecord(ctx->split.ev[0], sq);
     e = hdk::launch_pack(direct ? nullptr : ddesc, n, pack_tiles, grid_pack, ctx->opt.label, split ? prep_sms : 0, sq,
-                         direct ? &one : nullptr, direct && !dt ? dctl : nullptr, (uint32_t*)(dbase + off_cols), 2 * ncols);
+                         direct ? &one : nullptr, direct && !dt ? dctl : nullptr, (uint32_t*)(dbase + off_cols),
+                         (int)(2 * cols_words));
     if (e == cudaSuccess && mb >= 0) e = cudaEventRecord(ctx->mask_free[mb], sq);  // staging buffer read
     if (e != cudaSuccess) return cuda_fail(ctx, e, "pack launch");
     Job* djobs = (Job*)(dbase + off_jobs);
@@ -809,42 +926,20 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (occ <= 0) return set_error(ctx, HD_ERR_CUDA, "dilation kernel cannot be made resident");
     const int per_sm = cps > 0 ? std::min(cps, occ) : occ;
     dim3 grid((split ? ctx->split.solve_sms[part] : ctx->sm_count) * per_sm), block(sh.threads);
-    const float pct = (ctx->opt.percentile > 0.f && ctx->opt.percentile <= 1.f) ? ctx->opt.percentile : 0.95f;
     // the launch decodes the results on the device (one warp per pair, after
     // its last barrier): the per-step histograms never leave the device
     sp.descs = ddesc;
     sp.npairs = n;
     sp.pct = pct;
     sp.reset_info = direct ? 1 : 0;
-    hd_result* const hres = async ? nullptr : (hd_result*)(hbase + upload_bytes);
-    sp.out = async ? ro.async_out : hres;  // synchronous calls: pinned host memory, no read-back
+    sp.out = async ? ro.async_out : hres;
     void* args[] = {&sp};
     if (timing) cudaEventRecord(ctx->ev[2], s);
     if (stime) cudaEventRecord(ctx->split.ev[3], sv);  // after the previous dilation and this set-up
-    if (dt) {
-        hdk::DtParams dp{};
-        dp.info = dinfos;
-        dp.packed[0] = (const uint32_t*)(dbase + plan[0].off_pa);
-        dp.packed[1] = (const uint32_t*)(dbase + plan[0].off_pb);
-        for (int j = 0; j < 2; ++j) {
-            dp.vol[j] = (uint32_t*)(dbase + plan[0].off_jb[j][0]);
-            dp.base[j] = (uint16_t*)(dbase + plan[0].off_jb[j][1]);
-            dp.rows[j] = (uint32_t*)(dbase + plan[0].off_jb[j][2]);
-            dp.hist[j] = (unsigned long long*)(dbase + plan[0].off_hist) + (size_t)j * (plan[0].kmax + 1);
-        }
-        dp.cols = (uint32_t*)(dbase + off_cols);
-        dp.ncols = ncols;
-        dp.state = (hdk::DtState*)(dbase + off_states);  // the plane kernel zeroes it
-        dp.map[0] = ro.map_b;
-        dp.map[1] = ro.map_a;
-        dp.W = pairs[0].W;
-        dp.H = pairs[0].H;
-        dp.D = pairs[0].D;
-        dp.pitch = hdk::packed_pitch(pairs[0].W);
-        dp.kmax = plan[0].kmax;
-        dp.pct = pct;
-        dp.out = sp.out;
-        e = hdk::launch_dt(dp, split ? ctx->split.solve_sms[part] : ctx->sm_count, sv);
+    if (dt && n == 1) {
+        e = hdk::launch_dt(dt_pair(0), split ? ctx->split.solve_sms[part] : ctx->sm_count, sv);
+    } else if (dt) {
+        e = run_dt_groups(ctx, hdtp, (const hdk::DtPair*)(dbase + off_dtp), groups, (hdk::DtGroup*)(dbase + off_groups), dbase, s);
     } else {
         e = cudaLaunchCooperativeKernel(solve_fn, grid, block, args, (size_t)sh.smem, sv);
     }
@@ -1034,6 +1129,14 @@ hd_status hd_context_destroy(hd_context* ctx) {
         DeviceGuard g(ctx->device);
         if (ctx->stream) cudaStreamSynchronize(ctx->stream);
         split_release(ctx);
+        for (cudaStream_t st : ctx->dt_stream)
+            if (st) {
+                cudaStreamSynchronize(st);
+                cudaStreamDestroy(st);
+            }
+        for (cudaEvent_t ev : ctx->dt_join)
+            if (ev) cudaEventDestroy(ev);
+        if (ctx->dt_fork) cudaEventDestroy(ctx->dt_fork);
         ctx->infos.release();
         ctx->arena.release();
         for (DeviceArena& a : ctx->ws_arena) a.release();

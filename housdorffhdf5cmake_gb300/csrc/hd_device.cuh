@@ -99,13 +99,25 @@ __host__ __device__ __forceinline__ long long dt_bases(int W, int H, int D) {
 
 __host__ __device__ __forceinline__ int dt_cols(int W, int H) { return (W + 31) / 32 * 2 * ((H + 63) / 64); }
 
+// Columns of four rows x one word, both directions (the list of those with
+// targets, several pairs).
+__host__ __device__ __forceinline__ int dt_list(int W, int H) { return 2 * ((H + 3) / 4) * ((W + 31) / 32); }
+
 // Counters of the distance transform's second kernel.
 struct DtState {
-    unsigned int done;  // CTAs that have added their counts
+    unsigned int done;   // CTAs (of several pairs: columns) that have added their counts
+    unsigned int units;  // several pairs: columns with targets
 };
 
-// One pair, by value (direction 0: A's distances at B's voxels, 1: the reverse).
-struct DtParams {
+// Counters of a launch over several pairs; zero before the plane kernel.
+struct DtGroup {
+    int32_t next_plane, next_column;  // next units to claim
+    uint32_t units;                   // columns listed
+    uint32_t pad;
+};
+
+// One pair (direction 0: A's distances at B's voxels, 1: the reverse).
+struct DtPair {
     PairInfo* info;              // put back to the start values by the decode
     const uint32_t* packed[2];   // pa, pb
     uint32_t* vol[2];            // in-plane distances as bytes, four rows per word: dt_vol_words
@@ -122,6 +134,7 @@ struct DtParams {
     float pct;                   // robust HD percentile
     hd_result* out;
 };
+constexpr int kDtMaxGroup = 64;  // pairs of one launch
 
 // Packing and set-up split every pair into tiles; one launch covers the
 // tiles of all pairs.  Packing tiles are kPackTileWords words of the packed

@@ -23,6 +23,14 @@
 // Both kernels together, against the dilation loop with its set-up: 512^3
 // with 451 steps 0.09 against 3.5 ms, 512x512x256 with 19 to 30 steps 0.037
 // against 0.10 to 0.13 ms, 64^3 0.019 against 0.08 ms.
+//
+// Several pairs share launches (dt_planes_kernel, dt_list_kernel,
+// dt_columns_kernel): their planes and their columns with targets are claimed
+// from one list each, as their domains, which only the device knows, differ a
+// lot (CTAs dealt to pairs by volume: 1.4 against 0.8 ms for 256 ragged
+// pairs).  There the work fills the GPU, so a column is one warp's and no
+// warp waits for another.  256 ragged pairs of 64 to 384 voxels a side: 0.79
+// to 0.97 against 1.18 to 1.54 ms of the dilation loop.
 #include <algorithm>
 #include <atomic>
 #include <cuda_runtime.h>
@@ -58,6 +66,21 @@ __device__ __forceinline__ void red_shared_inc(uint32_t at, unsigned in) {
                  : "memory");
 }
 
+// Counts a plane's four rows of one column (a lane's distances v, target words
+// t4); found(row, distance) at each target.
+template <class F>
+__device__ __forceinline__ void count_rows(uint2 v, uint4 t4, int lane, uint32_t hist_at, unsigned& dm, F found) {
+    const uint32_t tw[4] = {t4.x, t4.y, t4.z, t4.w};
+    const unsigned dd[4] = {v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16};
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const unsigned in = (tw[r] >> lane) & 1u;
+        red_shared_inc(hist_at + 4u * dd[r], in);
+        dm = max(dm, in ? dd[r] : 0u);
+        if (in) found(r, dd[r]);
+    }
+}
+
 // A pair's domain: the bounding box of A u B, x in whole words.
 struct Geom {
     int wx0, w1;             // first and last word column
@@ -77,6 +100,11 @@ __device__ __forceinline__ Geom dt_geom(const PairInfo& I) {
     g.ntile = (g.h + 63) >> 6;
     g.nyq = (g.h + 3) >> 2;
     return g;
+}
+
+// Directions with target voxels (none of a pair with an empty mask).
+__device__ __forceinline__ int dt_directions(const PairInfo& I) {
+    return I.n_a == 0 || I.n_b == 0 ? 0 : (I.n_b > I.n_ab) + (I.n_a > I.n_ab);
 }
 
 // Nearest set voxel before (after) the end (start) of a word, carried over
@@ -109,178 +137,262 @@ constexpr int kPlaneEnds = 2 * kPlaneWarps * 2 * 32;
 // against 19 to 22 us with the words in groups of four registers, 512^3 with
 // small blobs (both directions) 51 to 65 against 97 to 114 us.  64 registers
 // and 4 CTAs per SM (32 bytes spilled): 8 % slower.
-__global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __grid_constant__ DtParams p) {
-    extern __shared__ uint32_t sm[];
-    cudaGridDependencySynchronize();  // launched while the packing ends
+// Plane z of a direction: this warp's tile t (a warp without one: act false).
+// claimed() is called once, before the first barrier.
+template <class F>
+__device__ __forceinline__ void plane_unit(const DtPair& p, const Geom& g, int j, int z, int t, bool act, uint32_t* sm, F claimed) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* const tr = sm + warp * kTr;
     uint32_t* const s_end = sm + kPlaneWarps * kTr;  // [2][warps][2][32]
     uint32_t* const s_r = s_end + kPlaneEnds;        // [words][warps][32]
+    const int q0 = g.wx0 >> 2;
+    const size_t vrow = (size_t)g.wx * 32;
+    const int ya = t * 64 + lane, yb = ya + 32;
+    // rows ya, yb of the plane's columns of 4 words, p.H apart
+    const uint4* const src = (const uint4*)(p.packed[j] + (size_t)(g.oz + (act ? z : 0)) * p.H * p.pitch) + g.oy;
+    const uint4* const ra = src + (ya < g.h ? ya : 0);
+    const uint4* const rb = src + (yb < g.h ? yb : 0);
+    const ptrdiff_t other = (const uint4*)p.packed[1 - j] - (const uint4*)p.packed[j];
+    const bool va = act && ya < g.h, vb = act && yb < g.h;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    // One scan of the rows from the right: the carries at each word, the
+    // rows with target voxels, and whether the plane has a source at all
+    unsigned ca = kInf, cb = kInf;
+    const int tz = t * g.d + (act ? z : 0);
+    if (act) {
+#pragma unroll 1
+        for (int q = g.nq - 1; q >= 0; --q) {
+            const ptrdiff_t o = (ptrdiff_t)(q0 + q) * p.H;
+            const uint4 a = va ? __ldg(ra + o) : zero, b = vb ? __ldg(rb + o) : zero;
+            const uint4 c = va ? __ldg(ra + other + o) : zero, d = vb ? __ldg(rb + other + o) : zero;
+            const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
+            const uint32_t ta[4] = {c.x & ~a.x, c.y & ~a.y, c.z & ~a.z, c.w & ~a.w};
+            const uint32_t tb[4] = {d.x & ~b.x, d.y & ~b.y, d.z & ~b.z, d.w & ~b.w};
+            unsigned fa = 0, fb = 0;
+#pragma unroll
+            for (int k = 3; k >= 0; --k) {
+                s_r[((4 * q + k) * kPlaneWarps + warp) * 32 + lane] = ca | (cb << 16);
+                ca = carry_right(ca, wa[k]);
+                cb = carry_right(cb, wb[k]);
+                const unsigned ba = __ballot_sync(kFull, ta[k] != 0u), bb = __ballot_sync(kFull, tb[k] != 0u);
+                if (lane == k) {
+                    fa = ba;
+                    fb = bb;
+                }
+            }
+            const int w = 4 * (q0 + q) + lane;
+            if (lane < 4 && w >= g.wx0 && w <= g.w1) {
+                uint32_t* const f = p.rows[j] + (size_t)(w - g.wx0) * 2 * g.ntile * g.d + t * g.d + tz;
+                f[0] = fa;
+                f[g.d] = fb;
+                uint32_t* const c = p.cols + j * p.ncols + (w - g.wx0) * 2 * g.ntile + 2 * t;
+                if (fa) atomicOr(c, fa);
+                if (fb) atomicOr(c + 1, fb);
+            }
+        }
+    }
+    claimed();
+    if (!__syncthreads_or(act && (ca < kInf || cb < kInf))) {  // nothing to measure from
+        if (act)
+            for (int w = lane; w < g.wx; w += 32) p.base[j][(size_t)w * g.ntile * g.d + tz] = (uint16_t)kInf;
+        return;
+    }
+    unsigned la = kInf, lb = kInf;
+    uint32_t* const vol = p.vol[j] + (size_t)(act ? z : 0) * g.nyq * vrow;
+    const uint32_t* const pa = (const uint32_t*)ra;
+    const uint32_t* const pb = (const uint32_t*)rb;
+    auto word = [&](int w) { return (ptrdiff_t)(w & ~3) * p.H + (w & 3); };
+    uint32_t na = va ? __ldg(pa + word(g.wx0)) : 0u, nb = vb ? __ldg(pb + word(g.wx0)) : 0u;
+#pragma unroll 1
+    for (int w = g.wx0; w <= g.w1; ++w) {
+        const uint32_t ua = na, ub = nb;
+        if (w < g.w1) {  // the next word's
+            na = va ? __ldg(pa + word(w + 1)) : 0u;
+            nb = vb ? __ldg(pb + word(w + 1)) : 0u;
+        }
+        {
+            const uint32_t rcw = act ? s_r[((w - 4 * q0) * kPlaneWarps + warp) * 32 + lane] : 0u;
+            uint32_t V[32];
+            uint32_t* const end = s_end + ((w & 1) * kPlaneWarps) * 64;
+            if (act) {
+                // x: a seed is 0 on a set voxel, else 0xffff
+                const uint32_t n0 = ~__byte_perm(ua, ub, 0x5410), n1 = ~__byte_perm(ua, ub, 0x7632);
+                uint32_t f = la | (lb << 16);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const uint32_t s = (i < 16 ? n0 : n1) << (7 - (i & 7));
+                    const uint32_t seed = (i & 8) ? byte_signs<0xBB99>(s) : byte_signs<0xAA88>(s);
+                    f = addmin2(f, two(1), seed);
+                    V[i] = f;
+                }
+                f = rcw;
+#pragma unroll
+                for (int i = 31; i >= 0; --i) {
+                    f = addmin2(f, two(1), V[i]);
+                    tr[i * 33 + lane] = f;
+                }
+                la = carry_left(la, ua);
+                lb = carry_left(lb, ub);
+                __syncwarp();
+                // y: the two segments on their own
+#pragma unroll
+                for (int i = 0; i < 32; ++i) V[i] = tr[lane * 33 + i];
+                __syncwarp();
+#pragma unroll
+                for (int i = 1; i < 32; ++i) V[i] = addmin2(V[i - 1], two(1), V[i]);
+#pragma unroll
+                for (int i = 30; i >= 0; --i) V[i] = addmin2(V[i + 1], two(1), V[i]);
+                end[warp * 64 + lane] = V[0];
+                end[warp * 64 + 32 + lane] = V[31];
+            }
+            __syncthreads();  // ends are double-buffered by word: one barrier per word
+            if (act) {
+                // carries over the segments above (value at the row before
+                // the segment) and below
+                const uint32_t* const e0 = end + (warp - t) * 64 + lane;
+                unsigned cf = kInf, cb = kInf;
+#pragma unroll 1
+                for (int s = 0; s < t; ++s) {
+                    const uint32_t e = e0[s * 64 + 32];
+                    cf = min(e & 0xffffu, cf + 32u);
+                    cf = min(e >> 16, cf + 32u);
+                }
+#pragma unroll 1
+                for (int s = g.ntile - 1; s > t; --s) {
+                    const uint32_t e = e0[s * 64];
+                    cb = min(e >> 16, cb + 32u);
+                    cb = min(e & 0xffffu, cb + 32u);
+                }
+                const uint32_t CF = cf | (min(V[31] & 0xffffu, cf + 32u) << 16);
+                const uint32_t CB = min(V[0] >> 16, cb + 32u) | (cb << 16);
+                // a carry that does not lower its first row lowers none
+                if (__any_sync(kFull, addmin2(CF, two(1), V[0]) != V[0])) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) V[i] = addmin2(CF, two(i + 1), V[i]);
+                }
+                if (__any_sync(kFull, addmin2(CB, two(1), V[31]) != V[31])) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) V[i] = addmin2(CB, two(32 - i), V[i]);
+                }
+                // bytes over the tile's base; an empty plane stores its base alone
+                const unsigned v0 = __shfl_sync(kFull, V[0] & 0xffffu, 0);
+                const unsigned b = v0 >= kInf ? kInf : (v0 > kSpread ? v0 - kSpread : 0u);
+                if (lane == 0) p.base[j][(size_t)(w - g.wx0) * g.ntile * g.d + tz] = (uint16_t)b;
+                if (b < kInf) {
+                    uint32_t* const o = vol + (size_t)(w - g.wx0) * 32 + lane;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const uint32_t p01 = __byte_perm(V[4 * i] - two(b), V[4 * i + 1] - two(b), 0x6240);
+                        const uint32_t p23 = __byte_perm(V[4 * i + 2] - two(b), V[4 * i + 3] - two(b), 0x6240);
+                        const int yl = t * 16 + i, yh = yl + 8;
+                        if (yl < g.nyq) o[yl * vrow] = __byte_perm(p01, p23, 0x5410);
+                        if (yh < g.nyq) o[yh * vrow] = __byte_perm(p01, p23, 0x7632);
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();  // the ends' buffers start over with the next planes
+}
+
+// Planes per CTA: as many as its warps have tiles for, but no fewer CTAs than
+// the grid (most: the grid's share of all planes).
+__device__ __forceinline__ int planes_per_cta(const Geom& g, int most) { return max(1, min(kPlaneWarps / g.ntile, most)); }
+
+__global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __grid_constant__ DtPair p) {
+    extern __shared__ uint4 sm4[];
+    cudaGridDependencySynchronize();  // launched while the packing ends
     const PairInfo I = *p.info;
     // histograms and counters of the depth kernel
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= p.kmax; t += gridDim.x * blockDim.x)
         p.hist[0][t] = p.hist[1][t] = 0ull;
     if (blockIdx.x == 0 && threadIdx.x == 0) *p.state = DtState{};
-    if (I.n_a == 0 || I.n_b == 0) return;
-    const unsigned long long rem[2] = {I.n_b - I.n_ab, I.n_a - I.n_ab};
+    const int nact = dt_directions(I);
+    if (nact == 0) return;
     const Geom g = dt_geom(I);
-    // planes per CTA: as many as its warps have tiles for, but no fewer CTAs than the grid
-    const int nact = (rem[0] > 0) + (rem[1] > 0);
-    const int G = max(1, min(kPlaneWarps / g.ntile, nact * g.d / (int)gridDim.x));
-    const int groups = (g.d + G - 1) / G;
+    const int G = planes_per_cta(g, nact * g.d / (int)gridDim.x);
+    const int groups = (g.d + G - 1) / G, warp = threadIdx.x >> 5;
     const int pl = warp / g.ntile, t = warp - pl * g.ntile;
-    const int q0 = g.wx0 >> 2;
-    const size_t vrow = (size_t)g.wx * 32;
 #pragma unroll 1
     for (int u = blockIdx.x; u < nact * groups; u += gridDim.x) {
-        const int j = nact == 2 ? (u >= groups) : (rem[0] > 0 ? 0 : 1);
+        const int j = nact == 2 ? (u >= groups) : !(I.n_b > I.n_ab);
         const int z = (nact == 2 && j ? u - groups : u) * G + pl;
-        const bool act = pl < G && z < g.d;
-        const int ya = t * 64 + lane, yb = ya + 32;
-        // rows ya, yb of the plane's columns of 4 words, p.H apart
-        const uint4* const src = (const uint4*)(p.packed[j] + (size_t)(g.oz + (act ? z : 0)) * p.H * p.pitch) + g.oy;
-        const uint4* const ra = src + (ya < g.h ? ya : 0);
-        const uint4* const rb = src + (yb < g.h ? yb : 0);
-        const ptrdiff_t other = (const uint4*)p.packed[1 - j] - (const uint4*)p.packed[j];
-        const bool va = act && ya < g.h, vb = act && yb < g.h;
-        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        // One scan of the rows from the right: the carries at each word, the
-        // rows with target voxels, and whether the plane has a source at all
-        unsigned ca = kInf, cb = kInf;
-        const int tz = t * g.d + (act ? z : 0);
-        if (act) {
+        plane_unit(p, g, j, z, t, pl < G && z < g.d, (uint32_t*)sm4, [] {});
+    }
+}
+
+// Several pairs: their units in one list, claimed from a counter one ahead;
+// every CTA holds all the pairs' descriptors and counts.  Issue slots 55 %
+// busy while it runs, the barriers per word column most of the rest.
+__global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_planes_kernel(const DtPair* __restrict__ many, int n, int quads,
+                                                                        DtGroup* group) {
+    extern __shared__ uint4 sm4[];
+    __shared__ int s_next[2], s_total, s_most;
+    cudaGridDependencySynchronize();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    DtPair* const s_pair = (DtPair*)((uint32_t*)sm4 + kPlaneWarps * kTr + kPlaneEnds + quads * 4 * kPlaneWarps * 32);
+    PairInfo* const s_info = (PairInfo*)(s_pair + n);
+    int* const s_begin = (int*)(s_info + n);  // [kDtMaxGroup]: first unit
+    // histograms and counters of the columns' kernel
+    for (int i = blockIdx.x; i < n; i += gridDim.x) {
+        const DtPair& p = many[i];
+        for (int t = threadIdx.x; t <= p.kmax; t += blockDim.x) p.hist[0][t] = p.hist[1][t] = 0ull;
+        if (threadIdx.x == 0) *p.state = DtState{};
+    }
+    static_assert(sizeof(DtPair) % 16 == 0 && sizeof(PairInfo) % 8 == 0 && kDtMaxGroup == 64, "copied in vectors");
+    constexpr int kV = sizeof(DtPair) / 16, kI = sizeof(PairInfo) / 8;
+    for (int t = threadIdx.x; t < n * kV; t += blockDim.x) ((uint4*)s_pair)[t] = __ldg((const uint4*)many + t);
+    __syncthreads();
+    for (int t = threadIdx.x; t < n * kI; t += blockDim.x)
+        ((uint2*)s_info)[t] = __ldcg((const uint2*)s_pair[t / kI].info + t % kI);
+    __syncthreads();
+    if (warp == 0) {
+        int planes = 0, before = 0;
+        for (int i = lane; i < n; i += 32) planes += dt_directions(s_info[i]) * dt_geom(s_info[i]).d;
+        const int most = __reduce_add_sync(kFull, planes) / (int)gridDim.x;
 #pragma unroll 1
-            for (int q = g.nq - 1; q >= 0; --q) {
-                const ptrdiff_t o = (ptrdiff_t)(q0 + q) * p.H;
-                const uint4 a = va ? __ldg(ra + o) : zero, b = vb ? __ldg(rb + o) : zero;
-                const uint4 c = va ? __ldg(ra + other + o) : zero, d = vb ? __ldg(rb + other + o) : zero;
-                const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
-                const uint32_t ta[4] = {c.x & ~a.x, c.y & ~a.y, c.z & ~a.z, c.w & ~a.w};
-                const uint32_t tb[4] = {d.x & ~b.x, d.y & ~b.y, d.z & ~b.z, d.w & ~b.w};
-                unsigned fa = 0, fb = 0;
-#pragma unroll
-                for (int k = 3; k >= 0; --k) {
-                    s_r[((4 * q + k) * kPlaneWarps + warp) * 32 + lane] = ca | (cb << 16);
-                    ca = carry_right(ca, wa[k]);
-                    cb = carry_right(cb, wb[k]);
-                    const unsigned ba = __ballot_sync(kFull, ta[k] != 0u), bb = __ballot_sync(kFull, tb[k] != 0u);
-                    if (lane == k) {
-                        fa = ba;
-                        fb = bb;
-                    }
-                }
-                const int w = 4 * (q0 + q) + lane;
-                if (lane < 4 && w >= g.wx0 && w <= g.w1) {
-                    uint32_t* const f = p.rows[j] + (size_t)(w - g.wx0) * 2 * g.ntile * g.d + t * g.d + tz;
-                    f[0] = fa;
-                    f[g.d] = fb;
-                    uint32_t* const c = p.cols + j * p.ncols + (w - g.wx0) * 2 * g.ntile + 2 * t;
-                    if (fa) atomicOr(c, fa);
-                    if (fb) atomicOr(c + 1, fb);
-                }
+        for (int i = lane; i < kDtMaxGroup; i += 32) {
+            const int nact = i < n ? dt_directions(s_info[i]) : 0;
+            int units = 0;
+            if (nact) {
+                const Geom g = dt_geom(s_info[i]);
+                const int G = planes_per_cta(g, most);
+                units = nact * ((g.d + G - 1) / G);
             }
-        }
-        if (!__syncthreads_or(act && (ca < kInf || cb < kInf))) {  // nothing to measure from
-            if (act)
-                for (int w = lane; w < g.wx; w += 32) p.base[j][(size_t)w * g.ntile * g.d + tz] = (uint16_t)kInf;
-            continue;
-        }
-        unsigned la = kInf, lb = kInf;
-        uint32_t* const vol = p.vol[j] + (size_t)(act ? z : 0) * g.nyq * vrow;
-        const uint32_t* const pa = (const uint32_t*)ra;
-        const uint32_t* const pb = (const uint32_t*)rb;
-        auto word = [&](int w) { return (ptrdiff_t)(w & ~3) * p.H + (w & 3); };
-        uint32_t na = va ? __ldg(pa + word(g.wx0)) : 0u, nb = vb ? __ldg(pb + word(g.wx0)) : 0u;
-#pragma unroll 1
-        for (int w = g.wx0; w <= g.w1; ++w) {
-            const uint32_t ua = na, ub = nb;
-            if (w < g.w1) {  // the next word's
-                na = va ? __ldg(pa + word(w + 1)) : 0u;
-                nb = vb ? __ldg(pb + word(w + 1)) : 0u;
+            int x = units;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(kFull, x, o);
+                if (lane >= o) x += v;
             }
-            {
-                const uint32_t rcw = act ? s_r[((w - 4 * q0) * kPlaneWarps + warp) * 32 + lane] : 0u;
-                uint32_t V[32];
-                uint32_t* const end = s_end + ((w & 1) * kPlaneWarps) * 64;
-                if (act) {
-                    // x: a seed is 0 on a set voxel, else 0xffff
-                    const uint32_t n0 = ~__byte_perm(ua, ub, 0x5410), n1 = ~__byte_perm(ua, ub, 0x7632);
-                    uint32_t f = la | (lb << 16);
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const uint32_t s = (i < 16 ? n0 : n1) << (7 - (i & 7));
-                        const uint32_t seed = (i & 8) ? byte_signs<0xBB99>(s) : byte_signs<0xAA88>(s);
-                        f = addmin2(f, two(1), seed);
-                        V[i] = f;
-                    }
-                    f = rcw;
-#pragma unroll
-                    for (int i = 31; i >= 0; --i) {
-                        f = addmin2(f, two(1), V[i]);
-                        tr[i * 33 + lane] = f;
-                    }
-                    la = carry_left(la, ua);
-                    lb = carry_left(lb, ub);
-                    __syncwarp();
-                    // y: the two segments on their own
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) V[i] = tr[lane * 33 + i];
-                    __syncwarp();
-#pragma unroll
-                    for (int i = 1; i < 32; ++i) V[i] = addmin2(V[i - 1], two(1), V[i]);
-#pragma unroll
-                    for (int i = 30; i >= 0; --i) V[i] = addmin2(V[i + 1], two(1), V[i]);
-                    end[warp * 64 + lane] = V[0];
-                    end[warp * 64 + 32 + lane] = V[31];
-                }
-                __syncthreads();  // ends are double-buffered by word: one barrier per word
-                if (act) {
-                    // carries over the segments above (value at the row before
-                    // the segment) and below
-                    const uint32_t* const e0 = end + (warp - t) * 64 + lane;
-                    unsigned cf = kInf, cb = kInf;
-#pragma unroll 1
-                    for (int s = 0; s < t; ++s) {
-                        const uint32_t e = e0[s * 64 + 32];
-                        cf = min(e & 0xffffu, cf + 32u);
-                        cf = min(e >> 16, cf + 32u);
-                    }
-#pragma unroll 1
-                    for (int s = g.ntile - 1; s > t; --s) {
-                        const uint32_t e = e0[s * 64];
-                        cb = min(e >> 16, cb + 32u);
-                        cb = min(e & 0xffffu, cb + 32u);
-                    }
-                    const uint32_t CF = cf | (min(V[31] & 0xffffu, cf + 32u) << 16);
-                    const uint32_t CB = min(V[0] >> 16, cb + 32u) | (cb << 16);
-                    // a carry that does not lower its first row lowers none
-                    if (__any_sync(kFull, addmin2(CF, two(1), V[0]) != V[0])) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) V[i] = addmin2(CF, two(i + 1), V[i]);
-                    }
-                    if (__any_sync(kFull, addmin2(CB, two(1), V[31]) != V[31])) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) V[i] = addmin2(CB, two(32 - i), V[i]);
-                    }
-                    // bytes over the tile's base; an empty plane stores its base alone
-                    const unsigned v0 = __shfl_sync(kFull, V[0] & 0xffffu, 0);
-                    const unsigned b = v0 >= kInf ? kInf : (v0 > kSpread ? v0 - kSpread : 0u);
-                    if (lane == 0) p.base[j][(size_t)(w - g.wx0) * g.ntile * g.d + tz] = (uint16_t)b;
-                    if (b < kInf) {
-                        uint32_t* const o = vol + (size_t)(w - g.wx0) * 32 + lane;
-#pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const uint32_t p01 = __byte_perm(V[4 * i] - two(b), V[4 * i + 1] - two(b), 0x6240);
-                            const uint32_t p23 = __byte_perm(V[4 * i + 2] - two(b), V[4 * i + 3] - two(b), 0x6240);
-                            const int yl = t * 16 + i, yh = yl + 8;
-                            if (yl < g.nyq) o[yl * vrow] = __byte_perm(p01, p23, 0x5410);
-                            if (yh < g.nyq) o[yh * vrow] = __byte_perm(p01, p23, 0x7632);
-                        }
-                    }
-                }
-            }
+            s_begin[i] = i < n ? before + x - units : 0x7fffffff;
+            before += __shfl_sync(kFull, x, 31);
         }
-        __syncthreads();  // the ends' buffers start over with the next planes
+        if (lane == 0) {
+            s_total = before;
+            s_most = most;
+        }
+    }
+    __syncthreads();
+    const int total = s_total, most = s_most;
+    int slot = 0;
+#pragma unroll 1
+    for (int u = blockIdx.x; u < total; slot ^= 1) {
+        int next = 0;
+        if (threadIdx.x == 0) next = atomicAdd(&group->next_plane, 1) + gridDim.x;
+        const int i = __popc(__ballot_sync(kFull, s_begin[lane] <= u)) + __popc(__ballot_sync(kFull, s_begin[32 + lane] <= u)) - 1;
+        const PairInfo& I = s_info[i];
+        const Geom g = dt_geom(I);
+        const int G = planes_per_cta(g, most), groups = (g.d + G - 1) / G, v = u - s_begin[i];
+        const int pl = warp / g.ntile, t = warp - pl * g.ntile;
+        const bool both = dt_directions(I) == 2;
+        const int j = both ? v >= groups : !(I.n_b > I.n_ab);
+        const int z = (both && j ? v - groups : v) * G + pl;
+        // the slots alternate: a claim is read between this barrier and the next
+        plane_unit(s_pair[i], g, j, z, t, pl < G && z < g.d, (uint32_t*)sm4, [&] {
+            if (threadIdx.x == 0) s_next[slot] = next;
+        });
+        u = s_next[slot];
     }
 }
 
@@ -288,7 +400,7 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
 // the rules of decode_pair_warp (statuses, exact sums, one double division,
 // robust HD).  One pass over the bins, 32 of both directions at a time, until
 // every target is counted.
-__device__ __forceinline__ void dt_decode(const DtParams& p, const PairInfo& I) {
+__device__ __forceinline__ void dt_decode(const DtPair& p, const PairInfo& I) {
     const int lane = threadIdx.x & 31;
     const unsigned long long n_ab = I.n_a - I.n_ab, n_ba = I.n_b - I.n_ab;  // A's, B's voxels outside the other
     unsigned long long sum[2] = {0ull, 0ull}, cov[2] = {0ull, 0ull};
@@ -393,7 +505,7 @@ __host__ __device__ constexpr size_t depth_smem(int warps, int nseg, int bins, i
 // claimed from a counter 28-35 us at 512x512x256 (the claim waits once per
 // unit); 16 warps per CTA holding their segments over the barrier likewise.
 template <bool kMap>
-__global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const __grid_constant__ DtParams p) {
+__global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const __grid_constant__ DtPair p) {
     extern __shared__ uint4 sm4[];
     __shared__ int s_max[2], s_last, s_warp[kDepthMaxWarps], s_first[2];
     __shared__ uint4 s_tgt[kDepthMaxWarps][kSeg];
@@ -562,22 +674,12 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
                 const uint32_t hist = s_hist_at + 4u * (unsigned)(j * bins);
                 unsigned dm = 0u;
                 auto count = [&](int i, int h) {  // the targets of plane h + i of the segment
-                    const uint2 v = s_v[i * 32 + lane];  // this lane's own
-                    const uint4 t4 = s_tgt[warp][h + i];
-                    const uint32_t tw[4] = {t4.x, t4.y, t4.z, t4.w};
-                    const unsigned dd[4] = {v.x & 0xffffu, v.x >> 16, v.y & 0xffffu, v.y >> 16};
-#pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const unsigned in = (tw[r] >> lane) & 1u;
-                        red_shared_inc(hist + 4u * dd[r], in);
-                        dm = max(dm, in ? dd[r] : 0u);
+                    count_rows(s_v[i * 32 + lane], s_tgt[warp][h + i], lane, hist, dm, [&](int r, unsigned d) {
                         if constexpr (kMap) {
-                            if (in) {
-                                const size_t row = (size_t)(g.oz + z0 + h + i) * p.H + g.oy + 4 * yq + r;
-                                p.map[j][row * p.W + 32 * (g.wx0 + w) + lane] = (int32_t)dd[r];
-                            }
+                            const size_t row = (size_t)(g.oz + z0 + h + i) * p.H + g.oy + 4 * yq + r;
+                            p.map[j][row * p.W + 32 * (g.wx0 + w) + lane] = (int32_t)d;
                         }
-                    }
+                    });
                 };
 #pragma unroll
                 for (int h = 0; h < kSeg; h += kHalf) {
@@ -627,40 +729,239 @@ __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const 
     }
 }
 
+// Several pairs: lists the columns with targets, a CTA per pair: bits 0-2 the
+// four-row group within its mask of 32 rows, 3-13 the mask (word column, 32
+// rows), 14 the direction, 15- the pair.
+constexpr int kListThreads = 128;
+__global__ void __launch_bounds__(kListThreads) dt_list_kernel(const DtPair* many, uint32_t* list, DtGroup* group) {
+    __shared__ unsigned s_units;
+    cudaGridDependencySynchronize();
+    const DtPair& p = many[blockIdx.x];
+    const int lane = threadIdx.x & 31;
+    const PairInfo I = *p.info;
+    const int nact = dt_directions(I);
+    if (nact == 0) {
+        if (threadIdx.x < 32) dt_decode(p, I);
+        return;
+    }
+    const Geom g = dt_geom(I);
+    const int per = g.wx * 2 * g.ntile, first = I.n_b > I.n_ab ? 0 : 1;
+    if (threadIdx.x == 0) s_units = 0u;
+    __syncthreads();
+    for (int i0 = threadIdx.x - lane; i0 < nact * per; i0 += kListThreads) {
+        const int i = i0 + lane, jj = i >= per, j = first + jj;
+        unsigned m = i < nact * per ? __ldcg(p.cols + j * p.ncols + (i - jj * per)) : 0u;
+        m |= m >> 2;
+        m = (m | (m >> 1)) & 0x11111111u;  // one bit per four rows
+        const int c = __popc(m);
+        int x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += v;
+        }
+        unsigned at = 0u;
+        if (lane == 31 && x) {
+            at = atomicAdd(&group->units, (unsigned)x);
+            atomicAdd(&s_units, (unsigned)x);
+        }
+        at = __shfl_sync(kFull, at, 31) + x - c;
+        for (; m; m &= m - 1u)
+            list[at++] = (unsigned)blockIdx.x << 15 | (unsigned)j << 14 | (unsigned)(i - jj * per) << 3 |
+                         (unsigned)(__ffs(m) - 1) >> 2;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) p.state->units = s_units;
+}
+
+// Several pairs: a column per warp at a time, claimed one ahead.  From the
+// last plane down to the first segment with targets each segment leaves the
+// carry from the planes after it in shared memory; then up to the last with
+// targets, counting where there are any.  No barrier, and every warp has a
+// histogram of its own, added to the pair's after each column.
+// Bound by latency (a third of the issue slots, 10 warps per SM: the
+// histograms and carries take the shared memory).  256 ragged pairs, planes
+// and columns: 0.79 to 0.97 ms; the next segment loaded ahead (110 registers)
+// or 64 registers: the same, 4 % more; histograms of 256 bins: 6 % less, but
+// distances have no such limit.
+constexpr int kManyWarps = 4, kManyCtas = 5;
+__host__ __device__ constexpr size_t many_warp_smem(int nseg, int bins) {
+    return (size_t)kHalf * 32 * 8 + (size_t)nseg * (32 * 8) + ((size_t)nseg * 2 + 31) / 16 * 16 +
+           ((size_t)bins * 4 + 15) / 16 * 16;
+}
+__global__ void __launch_bounds__(kManyWarps * 32, kManyCtas)
+    dt_columns_kernel(const DtPair* many, const uint32_t* list, DtGroup* group, int max_seg, int bins) {
+    extern __shared__ uint4 sm4[];
+    __shared__ uint4 s_tgt[kManyWarps][kSeg];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    char* const sm = (char*)sm4 + warp * many_warp_smem(max_seg, bins);
+    uint2* const s_v = (uint2*)sm;
+    uint2* const s_carry = s_v + kHalf * 32;            // [max_seg][32]
+    unsigned* const s_hist = (unsigned*)(s_carry + max_seg * 32);  // [bins]
+    uint16_t* const s_zm = (uint16_t*)(s_hist + (bins + 3) / 4 * 4);  // [max_seg]: planes with targets
+    const uint32_t hist_at = (uint32_t)__cvta_generic_to_shared(s_hist);
+    for (int t = lane; t < bins; t += 32) s_hist[t] = 0u;
+    cudaGridDependencySynchronize();
+    const int total = (int)__ldcg(&group->units);
+#pragma unroll 1
+    for (int u = blockIdx.x * kManyWarps + warp; u < total;) {
+        int next = 0;
+        if (lane == 0) next = atomicAdd(&group->next_column, 1) + gridDim.x * kManyWarps;
+        const unsigned rec = __ldcg(list + u);
+        const DtPair& p = many[rec >> 15];
+        const int j = (rec >> 14) & 1u, wh = (rec >> 3) & 0x7ffu;
+        const Geom g = dt_geom(*p.info);
+        const int nseg = (g.d + kSeg - 1) / kSeg;
+        const int w = wh / (2 * g.ntile), half = wh - w * 2 * g.ntile, yq = 8 * half + (int)(rec & 7u);
+        const size_t vrow = (size_t)g.wx * 32, vplane = vrow * g.nyq;
+        const uint32_t* const vol = p.vol[j] + (size_t)yq * vrow + (size_t)w * 32 + lane;
+        const uint16_t* const base = p.base[j] + ((size_t)w * g.ntile + (yq >> 4)) * g.d;
+        // planes with targets
+        const uint32_t* const rows = p.rows[j] + (size_t)wh * g.d;
+        int first = nseg, last = -1;
+        __syncwarp();
+        for (int z = 0; z < g.d; z += 32) {
+            const unsigned r = z + lane < g.d ? __ldcg(rows + z + lane) : 0u;
+            const unsigned zm = __ballot_sync(kFull, ((r >> (4 * (yq & 7))) & 0xfu) != 0u);
+            if (lane < 2) s_zm[(z >> 4) + lane] = (uint16_t)(zm >> (16 * lane));
+            if (zm) {
+                first = min(first, (z >> 4) + ((zm & 0xffffu) == 0u));
+                last = (z >> 4) + ((zm >> 16) != 0u);
+            }
+        }
+        uint32_t V[kSeg][2];
+        // A segment's in-plane distances (an empty plane's bytes are not
+        // written; over its base they are no distance whatever they are)
+        auto load = [&](int sg) {
+            const int z0 = sg * kSeg;
+            const unsigned b = lane < kSeg && z0 + lane < g.d ? (unsigned)__ldcg(base + z0 + lane) : kInf;
+#pragma unroll
+            for (int i = 0; i < kSeg; ++i) V[i][0] = z0 + i < g.d ? __ldcg(vol + (z0 + i) * vplane) : 0u;
+#pragma unroll
+            for (int i = 0; i < kSeg; ++i) {
+                const uint32_t x = V[i][0], bb = two(__shfl_sync(kFull, b, i));
+                V[i][0] = __byte_perm(x, 0u, 0x4140) + bb;
+                V[i][1] = __byte_perm(x, 0u, 0x4342) + bb;
+            }
+        };
+        uint32_t c0 = kInf2, c1 = kInf2;
+#pragma unroll 1
+        for (int sg = nseg - 1;; --sg) {
+            s_carry[sg * 32 + lane] = make_uint2(c0, c1);
+            if (sg <= first) break;
+            load(sg);
+#pragma unroll
+            for (int i = kSeg - 1; i >= 0; --i) {
+                c0 = addmin2(c0, two(1), V[i][0]);
+                c1 = addmin2(c1, two(1), V[i][1]);
+            }
+        }
+        __syncwarp();  // s_zm
+        uint32_t f0 = kInf2, f1 = kInf2;
+        unsigned dm = 0u;
+#pragma unroll 1
+        for (int sg = 0; sg <= last; ++sg) {
+            const unsigned zm = s_zm[sg];
+            const int z0 = sg * kSeg;
+            uint32_t tw0 = 0u, tw1 = 0u;  // lane = (plane, two of the four rows)
+            if (zm) {
+                const int z = z0 + (lane & 15), y = 4 * yq + 2 * (lane >> 4);
+                if (z < g.d && y < g.h) {
+                    const int wf = g.wx0 + w;
+                    const size_t o = ((size_t)(g.oz + z) * p.pitch + (wf & ~3)) * p.H + 4 * (g.oy + y) + (wf & 3);
+                    tw0 = __ldg(p.packed[1 - j] + o) & ~__ldg(p.packed[j] + o);
+                    if (y + 1 < g.h) tw1 = __ldg(p.packed[1 - j] + o + 4) & ~__ldg(p.packed[j] + o + 4);
+                }
+            }
+            load(sg);
+#pragma unroll
+            for (int i = 0; i < kSeg; ++i) {
+                V[i][0] = f0 = addmin2(f0, two(1), V[i][0]);
+                V[i][1] = f1 = addmin2(f1, two(1), V[i][1]);
+            }
+            if (!zm) continue;
+            const uint2 c = s_carry[sg * 32 + lane];
+            c0 = c.x;
+            c1 = c.y;
+#pragma unroll
+            for (int i = kSeg - 1; i >= 0; --i) {
+                V[i][0] = c0 = addmin2(c0, two(1), V[i][0]);
+                V[i][1] = c1 = addmin2(c1, two(1), V[i][1]);
+            }
+            ((uint2*)s_tgt[warp])[(lane & 15) * 2 + (lane >> 4)] = make_uint2(tw0, tw1);
+#pragma unroll
+            for (int h = 0; h < kSeg; h += kHalf) {
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < kHalf; ++i) s_v[i * 32 + lane] = make_uint2(V[h + i][0], V[h + i][1]);
+                __syncwarp();
+#pragma unroll 1
+                for (unsigned m = (zm >> h) & ((1u << kHalf) - 1u); m; m &= m - 1u) {
+                    const int i = __ffs(m) - 1;
+                    count_rows(s_v[i * 32 + lane], s_tgt[warp][h + i], lane, hist_at, dm, [](int, unsigned) {});
+                }
+            }
+            __syncwarp();
+        }
+        // to the pair's counts; the pair's last column decodes its result
+        dm = __reduce_max_sync(kFull, dm);
+        __syncwarp();
+        for (int t = lane; t <= (int)dm; t += 32)
+            if (const unsigned v = s_hist[t]) {
+                atomicAdd(p.hist[j] + t, (unsigned long long)v);
+                s_hist[t] = 0u;
+            }
+        __threadfence();
+        __syncwarp();
+        bool done = false;
+        if (lane == 0) done = atomicAdd(&p.state->done, 1u) + 1u == __ldcg(&p.state->units);
+        if (__shfl_sync(kFull, (int)done, 0)) {
+            __threadfence();
+            const PairInfo I = *p.info;
+            dt_decode(p, I);
+        }
+        u = __shfl_sync(kFull, next, 0);
+    }
+}
+
 // ---- launch wrappers --------------------------------------------------------
 bool dt_fits(int W, int H, int D) {
     return W <= kDtMaxW && H <= kDtMaxH && D <= kDtMaxD && W + H + D <= kDtMaxSum;
 }
 
-cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s) {
-    const int nq = ((p.W + 31) / 32 + 3) / 4;
-    const int nseg = (p.D + kSeg - 1) / kSeg;
-    const size_t plane_sm = sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)nq * 4 * kPlaneWarps * 32);
-    const int dwarps = nseg > 2 ? kDepthMaxWarps : 4;
-    const size_t depth_sm = depth_smem(dwarps, nseg, p.W + p.H + p.D, p.ncols);
-    // the limit of dynamic shared memory, once per device for the largest size
-    // (calls of other sizes may run on other threads)
+namespace {
+
+constexpr int kPlaneCtas = 3;  // resident CTAs per SM
+
+size_t plane_smem(int quads, int pairs) {
+    return sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)quads * 4 * kPlaneWarps * 32) +
+           (pairs ? pairs * (sizeof(DtPair) + sizeof(PairInfo)) + sizeof(int) * kDtMaxGroup : 0);
+}
+int quads_of(const DtPair& p) { return ((p.W + 31) / 32 + 3) / 4; }
+int segs_of(const DtPair& p) { return (p.D + kSeg - 1) / kSeg; }
+
+// Raises the kernels' limit of dynamic shared memory, once per device, for the
+// largest size (calls of other sizes may run on other threads).
+cudaError_t raise_limits() {
     static std::atomic<bool> raised[64];
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    if (dev >= 64 || !raised[dev].load(std::memory_order_acquire)) {
-        const int lim = 200 * 1024;  // above any size taken (dt_fits), with the static part below 227 KB
-        e = cudaFuncSetAttribute(&dt_plane_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(&dt_depth_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(&dt_depth_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-        if (e != cudaSuccess) return e;
-        if (dev < 64) raised[dev].store(true, std::memory_order_release);
-    }
-    // one resident wave, or fewer CTAs than that for small volumes
-    const long long punits = 2ll * p.D;
-    const long long dunits = 2ll * ((p.H + 3) / 4) * ((p.W + 31) / 32);
-    const unsigned pg = (unsigned)std::min<long long>(punits, 3ll * sms);
-    const unsigned dg = (unsigned)std::min<long long>(dunits, 4ll * kDepthMaxWarps / dwarps * sms);
-    // each may be scheduled while the kernel before it ends (it waits for that
-    // kernel's results itself)
+    if (e != cudaSuccess || (dev < 64 && raised[dev].load(std::memory_order_acquire))) return e;
+    const int lim = 200 * 1024;  // above any size taken (dt_fits), with the static part below 227 KB
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    e = cudaFuncSetAttribute(&dt_plane_kernel, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_planes_kernel, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_depth_kernel<false>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_depth_kernel<true>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_columns_kernel, attr, lim);
+    if (e == cudaSuccess && dev < 64) raised[dev].store(true, std::memory_order_release);
+    return e;
+}
+
+// A launch that may be scheduled while the kernel before it ends (it waits
+// for that kernel's results itself).
+template <class... P, class... A>
+cudaError_t launch_early(void (*kernel)(P...), long long grid, int threads, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchAttribute at{};
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
@@ -668,15 +969,49 @@ cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s) {
     c.stream = s;
     c.attrs = &at;
     c.numAttrs = 1;
-    c.gridDim = dim3(pg);
-    c.blockDim = dim3(kPlaneWarps * 32);
-    c.dynamicSmemBytes = plane_sm;
-    e = cudaLaunchKernelEx(&c, dt_plane_kernel, p);
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    return cudaLaunchKernelEx(&c, kernel, args...);
+}
+
+}  // namespace
+
+cudaError_t launch_dt(const DtPair& p, int sms, cudaStream_t s) {
+    cudaError_t e = raise_limits();
     if (e != cudaSuccess) return e;
-    c.gridDim = dim3(dg);
-    c.blockDim = dim3(dwarps * 32);
-    c.dynamicSmemBytes = depth_sm;
-    return cudaLaunchKernelEx(&c, p.map[0] ? dt_depth_kernel<true> : dt_depth_kernel<false>, p);
+    const int nseg = segs_of(p), dwarps = nseg > 2 ? kDepthMaxWarps : 4;
+    // one resident wave, or fewer CTAs than that for small volumes
+    const long long pg = std::min<long long>(2ll * p.D, (long long)kPlaneCtas * sms);
+    const long long dg = std::min<long long>(dt_list(p.W, p.H), 4ll * kDepthMaxWarps / dwarps * sms);
+    e = launch_early(dt_plane_kernel, pg, kPlaneWarps * 32, plane_smem(quads_of(p), 0), s, p);
+    if (e != cudaSuccess) return e;
+    return launch_early(p.map[0] ? dt_depth_kernel<true> : dt_depth_kernel<false>, dg, dwarps * 32,
+                        depth_smem(dwarps, nseg, p.W + p.H + p.D, p.ncols), s, p);
+}
+
+cudaError_t launch_dt_group(const DtPair* pairs, const DtPair* d_pairs, int n, uint32_t* d_list, DtGroup* d_group, int sms,
+                            cudaStream_t s) {
+    cudaError_t e = raise_limits();
+    int quads = 0, nseg = 0, bins = 0;
+    long long planes = 0, columns = 0;
+    for (int i = 0; i < n; ++i) {
+        const DtPair& p = pairs[i];
+        quads = std::max(quads, quads_of(p));
+        nseg = std::max(nseg, segs_of(p));
+        bins = std::max(bins, p.W + p.H + p.D);
+        planes += 2ll * p.D;
+        columns += dt_list(p.W, p.H);
+    }
+    if (e == cudaSuccess)
+        e = launch_early(dt_planes_kernel, std::min<long long>(planes, (long long)kPlaneCtas * sms), kPlaneWarps * 32,
+                         plane_smem(quads, n), s, d_pairs, n, quads, d_group);
+    if (e == cudaSuccess) e = launch_early(dt_list_kernel, n, kListThreads, 0, s, d_pairs, d_list, d_group);
+    if (e == cudaSuccess)
+        e = launch_early(dt_columns_kernel, std::min<long long>((columns + kManyWarps - 1) / kManyWarps, (long long)kManyCtas * sms),
+                         kManyWarps * 32, kManyWarps * many_warp_smem(nseg, bins), s, d_pairs, (const uint32_t*)d_list, d_group, nseg,
+                         bins);
+    return e;
 }
 
 }  // namespace hdk

@@ -31,7 +31,7 @@ struct PinnedArena {
 // Dilation kernel and brick geometry.
 //   kernel 1: one step per grid barrier, bricks bxw words x 32/bxw rows x bz planes
 //   kernel 2: `steps` steps per grid barrier, bricks 4 words x (32 - 2 steps) rows x bz planes
-//   kernel 3: distance transform (6-neighbour single pairs), no bricks
+//   kernel 3: distance transform (6-neighbour pairs), no bricks
 struct Shape {  // default: the autotuner's choice on the 512x512x256, 512^3 and ragged-batch workloads
     int kernel = 2;
     int bxw = 4;
@@ -152,6 +152,11 @@ struct hd_context {
         hd_timings shape{};  // the fields of hd_timings that are not times
     } split;
     hdh::DeviceArena ws_arena[Split::kWorkspaces - 1];  // the split path's workspaces 1, 2, ...
+    // distance transform of a batch: groups of pairs in turn on these streams,
+    // each with a workspace of its own
+    static constexpr int kDtStreams = 3;
+    cudaStream_t dt_stream[kDtStreams] = {};
+    cudaEvent_t dt_fork = nullptr, dt_join[kDtStreams] = {};
     // single pairs, per workspace: the counts and bounding box that a packing
     // adds to.  The decode at the end of a pair's launch puts the start values
     // back; info_clean[ws] is false until the first call has uploaded them and

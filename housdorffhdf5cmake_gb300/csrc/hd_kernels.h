@@ -52,9 +52,13 @@ const void* solve_tb_kernel_ptr(int se, int steps, int bz);
 const void* solve_tb_kernel_ptr_se6(int steps, int bz);
 const void* solve_tb_kernel_ptr_se18(int steps, int bz);
 
-// Distance transform of one 6-neighbour pair (hd_dt.cu): both kernels, after
-// the packing, on a stream of `sms` SMs.  dt_fits: the sizes it takes.
+// Distance transform of 6-neighbour pairs (hd_dt.cu), after the packing, on a
+// stream of `sms` SMs.  dt_fits: the sizes it takes.  Of one pair by value, or of n
+// (at most kDtMaxGroup; d_pairs: the same on the device) with a list of the
+// sum of dt_list words.
 bool dt_fits(int W, int H, int D);
-cudaError_t launch_dt(const DtParams& p, int sms, cudaStream_t s);
+cudaError_t launch_dt(const DtPair& pair, int sms, cudaStream_t s);
+cudaError_t launch_dt_group(const DtPair* pairs, const DtPair* d_pairs, int n, uint32_t* d_list, DtGroup* d_group, int sms,
+                            cudaStream_t s);
 
 }  // namespace hdk

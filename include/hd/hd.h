@@ -92,7 +92,7 @@ typedef struct hd_options {
                                     device can address them (default 1) */
     const char* tuning_table;    /* autotuner JSON table to load/store; NULL = none */
     int32_t record_timings;      /* record CUDA events around each kernel (hd_context_last_timings) */
-    int32_t kernel;              /* dilation kernel: 0 = tuned/default (single pairs under HD_SE6 without any
+    int32_t kernel;              /* dilation kernel: 0 = tuned/default (pairs under HD_SE6 without any
                                     option that asks for the dilation loop - a kernel, a brick shape, a cap on
                                     its steps or waits - take an exact distance transform instead), 1 = one step per grid barrier
                                     (brick_x_words x 32/brick_x_words rows x brick_z planes),
@@ -116,7 +116,7 @@ typedef struct hd_timings {
     int32_t brick_x_words, brick_z;
     int32_t kernel;      /* 1 = one step per barrier, 2 = temporally blocked, 3 = distance
                             transform (no loop: iterations, bricks and steps are 0; its
-                            two kernels count as solve_ms) */
+                            kernels count as solve_ms) */
     int32_t steps_per_barrier;
     int32_t brick_rows;
     int32_t dilation_partitions; /* pipelined entry on split SMs: dilations in
@@ -210,9 +210,10 @@ hd_status hd_pipeline_flush(hd_context* ctx, void* stream);
 hd_status hd_compute_u8_async(hd_context* ctx, const uint8_t* a, const uint8_t* b, int32_t W, int32_t H,
                               int32_t D, hd_metric metric, void* stream, hd_result* d_out);
 
-/* Solves n pairs of independent shapes with one packing launch, one set-up
- * launch and ONE persistent dilation launch over a shared (pair, brick) work
- * queue.  Per-pair results are bit-identical to hd_compute_u8.  out[i].status
+/* Solves n pairs of independent shapes with one packing launch and, under
+ * HD_SE6 (see hd_options.kernel), the distance transform of groups of pairs
+ * on three streams of the context, else one set-up launch and ONE persistent
+ * dilation launch over a shared (pair, brick) work queue.  Per-pair results are bit-identical to hd_compute_u8.  out[i].status
  * is the status of pair i; the return value is the first hard error.
  * This call, hd_profile_u8_device, hd_distance_map_device and hd_autotune run
  * on the context's own (non-blocking) stream: device masks must be complete

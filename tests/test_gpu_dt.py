@@ -1,4 +1,4 @@
-"""The distance-transform path (6-neighbour single pairs by default) against
+"""The distance-transform path (6-neighbour pairs by default) against
 the dilation loop (a context that asks for it) and the oracle, on every field
 but the barrier-loop count: sizes around its tiles (64 rows, 32 columns,
 groups of 4 words, segments of 16 planes, 16 segments per CTA) and the limits
@@ -91,3 +91,26 @@ def test_maps(hd, ctx, shape):
             w, wa, wb = one.distance_map(a, b, "se6")
             same(r, w, (shape, kind))
             assert torch.equal(ma, wa) and torch.equal(mb, wb)
+
+
+def test_batches(hd, loop):
+    """Groups of more pairs than one launch takes, of one pair each, more
+    groups than workspaces, pairs without targets or sources; a pair beyond
+    the limits takes the whole batch to the loop."""
+    rng = np.random.default_rng(4)
+    kinds = ("corners", "sparse", "slabs", "random")
+    small = [masks(rng, s, k) for i, s in enumerate(SHAPES) for k in (kinds[i % 4], kinds[(i + 1) % 4])]
+    z = np.zeros((9, 20, 50), np.uint8)
+    one = z.copy()
+    one[4, 5, 6] = 1
+    small[3:3] = [(z, z), (z, one), (one, z), (one, one), (one, one | (rng.random(z.shape) < 0.1).astype(np.uint8))]
+    large = [masks(rng, (200, 500, 500), "sparse") for _ in range(5)]
+    with hd.Context(0, record_timings=True) as c:
+        for tag, pairs, kernel in (("small", small, 3), ("mixed", small[:9] + large[:2] + small[9:20], 3),
+                                   ("large", large, 3), ("two", small[8:10], 3),
+                                   ("beyond", small[:3] + [masks(rng, (2, 513, 33), "sparse")], 2)):
+            dev = [tuple(torch.from_numpy(m).cuda() for m in p) for p in pairs]
+            got = c.batch(dev, "se6")
+            assert c.last_timings()["kernel"] == kernel, tag
+            for i, (g, p) in enumerate(zip(got, dev)):
+                same(g, loop.compute(*p, "se6"), (tag, i))
