@@ -301,7 +301,7 @@ __device__ __forceinline__ int planes_per_cta(const Geom& g, int most) { return 
 
 __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __grid_constant__ DtPair p) {
     extern __shared__ uint4 sm4[];
-    cudaGridDependencySynchronize();  // launched while the packing ends
+    cudaGridDependencySynchronize();  // placed as the packing ends
     const PairInfo I = *p.info;
     // histograms and counters of the depth kernel
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= p.kmax; t += gridDim.x * blockDim.x)
@@ -958,8 +958,10 @@ cudaError_t raise_limits() {
     return e;
 }
 
-// A launch that may be scheduled while the kernel before it ends (it waits
-// for that kernel's results itself).
+// A launch whose CTAs are placed as the kernel before it ends (they wait for
+// that kernel's results themselves): 3 us less per call at 64^3 and 301x287x173
+// than after it.  Not before: CTAs that wait beside a running packing take
+// its SMs' L1 (512^3 197 against 160 us a call, 301x287x173 212 against 202).
 template <class... P, class... A>
 cudaError_t launch_early(void (*kernel)(P...), long long grid, int threads, size_t smem, cudaStream_t s, A... args) {
     cudaLaunchAttribute at{};

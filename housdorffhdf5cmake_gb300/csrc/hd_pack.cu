@@ -393,7 +393,6 @@ __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const Pai
                                                                long long ntiles, int label,
                                                                const __grid_constant__ PairDesc one, Ctl* ctl, uint32_t* zero, int nzero) {
     __shared__ uint32_t s_bits_all[kPackWarps][2][kBitWords];
-    cudaTriggerProgrammaticLaunchCompletion();  // the distance transform's CTAs may take over as these end
     // nobody uses these before the next kernel
     if (ctl && blockIdx.x == 0 && threadIdx.x == 0) *ctl = Ctl{};
     for (int t = blockIdx.x * kPackThreads + threadIdx.x; t < nzero; t += gridDim.x * kPackThreads) zero[t] = 0u;
