@@ -120,6 +120,11 @@ constexpr int kPlaneEnds = 2 * kPlaneWarps * 2 * 32;
 
 }  // namespace
 
+// Barrier `id` of `threads` threads of the CTA.
+__device__ __forceinline__ void plane_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
 // Planes: a warp takes a tile of 64 rows x 32 columns (one word column), the
 // warps of a CTA the tiles of one or several planes; the CTA walks the word
 // columns from left to right.
@@ -135,12 +140,16 @@ constexpr int kPlaneEnds = 2 * kPlaneWarps * 2 * 32;
 // source voxel skips them, and rows are scanned once, from the right (the
 // words come one at a time after that, from L1): 512x512x256 pair 16 to 19 us
 // against 19 to 22 us with the words in groups of four registers, 512^3 with
-// small blobs (both directions) 51 to 65 against 97 to 114 us.  64 registers
-// and 4 CTAs per SM (32 bytes spilled): 8 % slower.
+// small blobs (both directions) 51 to 65 against 97 to 114 us.  The barrier
+// per word column is among the plane's warps only (62 registers against 78, 256
+// ragged pairs' planes and columns 0.767 against 0.791 ms).  4 CTAs per SM: 512^3
+// 165 against 159 us a call, the ragged batch 2 % slower.
+
 // Plane z of a direction: this warp's tile t (a warp without one: act false).
 // claimed() is called once, before the first barrier.
 template <class F>
-__device__ __forceinline__ void plane_unit(const DtPair& p, const Geom& g, int j, int z, int t, bool act, uint32_t* sm, F claimed) {
+__device__ __forceinline__ void plane_unit(const DtPair& p, const Geom& g, int j, int z, int t, bool act, uint32_t* sm,
+                                           F claimed) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t* const tr = sm + warp * kTr;
     uint32_t* const s_end = sm + kPlaneWarps * kTr;  // [2][warps][2][32]
@@ -245,7 +254,8 @@ __device__ __forceinline__ void plane_unit(const DtPair& p, const Geom& g, int j
                 end[warp * 64 + lane] = V[0];
                 end[warp * 64 + 32 + lane] = V[31];
             }
-            __syncthreads();  // ends are double-buffered by word: one barrier per word
+            // ends are double-buffered by word: one barrier per word, of the plane's warps
+            if (act) plane_sync(1 + warp / g.ntile, 32 * g.ntile);
             if (act) {
                 // carries over the segments above (value at the row before
                 // the segment) and below
