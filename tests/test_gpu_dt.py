@@ -114,3 +114,20 @@ def test_batches(hd, loop):
             assert c.last_timings()["kernel"] == kernel, tag
             for i, (g, p) in enumerate(zip(got, dev)):
                 same(g, loop.compute(*p, "se6"), (tag, i))
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 3), (17, 33, 70), (3, 5, 1031)])
+@pytest.mark.parametrize("offset,label", [(0, 0), (0, 3), (1, 0), (6, 3), (8, 0)])
+def test_map_values_outside_the_transform(hd, shape, offset, label):
+    """Maps of masks at any byte offset, with and without a label: -1 outside
+    the mask, 0 on the overlap, at least 1 elsewhere."""
+    rng = np.random.default_rng(6)
+    n = int(np.prod(shape))
+    flat = [torch.from_numpy(rng.integers(0, 5, n + offset, dtype=np.uint8)).cuda() for _ in range(2)]
+    a, b = (f[offset:].view(shape) for f in flat)
+    a.view(-1)[0] = b.view(-1)[-1] = label or 1
+    fa, fb = ((m == label) if label else (m != 0) for m in (a, b))
+    with hd.Context(0, label=label) as c:
+        _, ma, mb = c.distance_map(a, b, "se6")
+    for m, own, other in ((ma, fa, fb), (mb, fb, fa)):
+        assert bool((m[~own] == -1).all()) and bool((m[own & other] == 0).all()) and bool((m[own & ~other] >= 1).all())
