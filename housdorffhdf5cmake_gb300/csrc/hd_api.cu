@@ -870,7 +870,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (stime) cudaEventRecord(ctx->split.ev[0], sq);
     e = hdk::launch_pack(direct ? nullptr : ddesc, n, pack_tiles, grid_pack, ctx->opt.label, split ? prep_sms : 0, sq,
                          direct ? &one : nullptr, direct && !dt ? dctl : nullptr, (uint32_t*)(dbase + off_cols),
-                         (int)(2 * cols_words));
+                         (int)(2 * cols_words), async && !split && mb < 0);
     if (e == cudaSuccess && mb >= 0) e = cudaEventRecord(ctx->mask_free[mb], sq);  // staging buffer read
     if (e != cudaSuccess) return cuda_fail(ctx, e, "pack launch");
     Job* djobs = (Job*)(dbase + off_jobs);

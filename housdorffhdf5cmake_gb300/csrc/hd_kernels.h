@@ -17,10 +17,11 @@ namespace hdk {
 // device's); the grid is one resident wave of them.
 // d_descs null: one pair, whose descriptor `one` (host memory) is passed by
 // value; its counts must hold their start values (pair_info_start), and ctl
-// and nzero words at zero, if given, are cleared.
+// and nzero words at zero, if given, are cleared.  queued: placed as the
+// stream's kernel before it ends.
 cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, int grid, int label, int sms,
                         cudaStream_t s, const PairDesc* one = nullptr, Ctl* ctl = nullptr, uint32_t* zero = nullptr,
-                        int nzero = 0);
+                        int nzero = 0, bool queued = false);
 // zq1 / zq2 (may be null): queues whose first nz slots are zeroed.  d_descs
 // null: one pair, `one` by value as above, copied to desc_out (device).
 cudaError_t launch_setup(const PairDesc* d_descs, int npairs, long long ntiles, int sms, Job* jobs,
