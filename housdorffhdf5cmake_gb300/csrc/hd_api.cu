@@ -885,7 +885,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
     if (!dt)
         e = hdk::launch_setup(direct ? nullptr : ddesc, n, setup_tiles, split ? prep_sms : 0, djobs, dstates, dq[g0 % 3],
                               dctl, g0, bxw, by, bz, setup_mode, sq, dq[(g0 + 1) % 3], dq[(g0 + 2) % 3], nz,
-                              direct ? &one : nullptr, direct ? ddesc : nullptr);
+                              direct ? &one : nullptr, direct ? ddesc : nullptr, true);
     if (e == cudaSuccess && split) {
         // the dilation follows the set-up; the caller's stream follows the
         // packing's reads of its masks (work it queues later may overwrite
