@@ -29,8 +29,8 @@
 // from one list each, as their domains, which only the device knows, differ a
 // lot (CTAs dealt to pairs by volume: 1.4 against 0.8 ms for 256 ragged
 // pairs).  There the work fills the GPU, so a column is one warp's and no
-// warp waits for another.  256 ragged pairs of 64 to 384 voxels a side: 0.79
-// to 0.97 against 1.18 to 1.54 ms of the dilation loop.
+// warp waits for another.  256 ragged pairs of 64 to 384 voxels a side: 0.74
+// to 0.91 against 1.18 to 1.54 ms of the dilation loop.
 #include <algorithm>
 #include <atomic>
 #include <cuda_runtime.h>
@@ -791,10 +791,11 @@ __global__ void __launch_bounds__(kListThreads) dt_list_kernel(const DtPair* man
 // histogram of its own, added to the pair's after each column.
 // Bound by latency (a third of the issue slots, 10 warps per SM: the
 // histograms and carries take the shared memory).  256 ragged pairs, planes
-// and columns: 0.79 to 0.97 ms; the next segment loaded ahead (110 registers)
-// or 64 registers: the same, 4 % more; histograms of 256 bins: 6 % less, but
-// distances have no such limit.
-constexpr int kManyWarps = 4, kManyCtas = 5;
+// and columns: 0.74 to 0.91 ms; 4 warps per CTA and one plane counted at a time
+// 0.77 to 0.94 ms; the next segment loaded ahead (110 registers) or 64 registers:
+// the same, 4 % more; histograms of 256 bins: 6 % less, but distances have no
+// such limit.
+constexpr int kManyWarps = 2, kManyCtas = 12;
 __host__ __device__ constexpr size_t many_warp_smem(int nseg, int bins) {
     return (size_t)kHalf * 32 * 8 + (size_t)nseg * (32 * 8) + ((size_t)nseg * 2 + 31) / 16 * 16 +
            ((size_t)bins * 4 + 15) / 16 * 16;
@@ -905,10 +906,17 @@ __global__ void __launch_bounds__(kManyWarps * 32, kManyCtas)
 #pragma unroll
                 for (int i = 0; i < kHalf; ++i) s_v[i * 32 + lane] = make_uint2(V[h + i][0], V[h + i][1]);
                 __syncwarp();
+                // two planes at a time: their loads overlap
 #pragma unroll 1
-                for (unsigned m = (zm >> h) & ((1u << kHalf) - 1u); m; m &= m - 1u) {
+                for (unsigned m = (zm >> h) & ((1u << kHalf) - 1u); m;) {
                     const int i = __ffs(m) - 1;
-                    count_rows(s_v[i * 32 + lane], s_tgt[warp][h + i], lane, hist_at, dm, [](int, unsigned) {});
+                    m &= m - 1u;
+                    const int i2 = m ? __ffs(m) - 1 : i;
+                    const uint2 v = s_v[i * 32 + lane], v2 = s_v[i2 * 32 + lane];
+                    const uint4 t = s_tgt[warp][h + i], t2 = m ? s_tgt[warp][h + i2] : make_uint4(0u, 0u, 0u, 0u);
+                    m &= m - 1u;
+                    count_rows(v, t, lane, hist_at, dm, [](int, unsigned) {});
+                    count_rows(v2, t2, lane, hist_at, dm, [](int, unsigned) {});
                 }
             }
             __syncwarp();
