@@ -651,9 +651,10 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         }
     };
 
+    if (ro.max_bytes && total_bytes > ro.max_bytes) return set_error(ctx, HD_ERR_OOM, "workspace beyond its limit");
     if (total_bytes > arena.cap) drain_split();
     cudaError_t e = arena.ensure(total_bytes);
-    if (e != cudaSuccess && dt && !ro.force_shape) {
+    if (e != cudaSuccess && dt && !ro.force_shape && !ro.max_bytes) {
         // the distance transform's workspace is larger: the dilation loop's may fit
         RunOpts r2 = ro;
         r2.force_shape = true;

@@ -190,6 +190,7 @@ struct RunOpts {
     hd_result* async_out = nullptr;  // device memory: enqueue only, results decoded on the device
     bool pipelined = false;          // with async_out: the result may complete after a later flush
     bool ordered = false;            // the pairs are already in the shape's order (internal)
+    size_t max_bytes = 0;            // workspace at most (0: any): HD_ERR_OOM beyond it, and no other kernel instead
 };
 
 hd_status set_error(hd_context* ctx, hd_status st, const char* fmt, ...);

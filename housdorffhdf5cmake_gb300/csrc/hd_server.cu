@@ -8,8 +8,11 @@
 // on the device.  A tick is one cooperative launch of the same dilation kernel
 // as the single-pair path, bounded to tick_iterations steps; between ticks the
 // scheduler thread reads the jobs' states, completes finished pairs, frees
-// their memory and admits waiting ones.  Each pair's result depends only on
-// its own masks, so it is identical alone and in any mix.
+// their memory and admits waiting ones.  Under the 6-neighbour element,
+// requests that wait together are first solved in groups by the distance
+// transform (run_pairs on a context of the scheduler's own), between ticks.
+// Each pair's result depends only on its own masks, so it is identical alone
+// and in any mix.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,6 +63,8 @@ struct Request {
     int wxf = 0;
     long long dom_words = 0;
     size_t off_hist = 0, off_info = 0, off_packed = 0;
+    bool loop_only = false;     // beyond the distance transform's sizes or memory
+    size_t group_bytes = 0;     // workspace of the distance transform, at most
 };
 
 // First-fit allocator over [0, cap) (brick ids).
@@ -111,6 +116,15 @@ constexpr int kWaitSpinUs = 1000;
 // kQueueForBatchMode wait.
 constexpr int kFewRequests = 2;
 constexpr int kQueueForBatchMode = 8;
+// Requests that wait together are solved by the distance transform in a
+// group, at least and at most this many, and that many groups before the
+// resident pairs' next tick; fewer join the resident pairs.  Bursts of requests
+// of 10 M voxels in the median (some of 512^3), in the dilation loop alone and
+// with groups of at least 2, 3, 4 and 8:
+//    3 requests  206 us | 250, 207, 210, 208
+//   10 requests  737 us | 610, 620, 664, 740
+//   24 requests 1359 us | 992, 986, 1030, 1091
+constexpr int kGroupMin = 3, kGroupMax = 256, kGroupsPerTick = 8;
 
 }  // namespace
 
@@ -129,6 +143,12 @@ struct hd_server {
         int grid = 0;
     } modes[2];
     int mode = 1;
+    // distance transforms of groups of waiting requests: a context of the
+    // scheduler thread's own (null: every request takes the dilation loop),
+    // what its workspace counts for in bytes_in_use, and the pairs in flight
+    hd_context* group_ctx = nullptr;
+    size_t group_held = 0;
+    int in_group = 0;
     bool draining = false;  // single-pair mode with a queue building up: admit nothing until empty
     Shape shape;
     const void* solve_fn = nullptr;
@@ -208,6 +228,15 @@ void plan_request(hd_server* s, Request* r) {
     const size_t packed = align_up(4ULL * hdk::packed_pitch(r->W) * r->H * r->D);
     r->resident_bytes = r->off_packed + 2 * packed;
     r->transient_bytes = r->dev_a ? 0 : 2 * align_up(nb);
+    // the distance transform's share of a group's workspace, each part rounded up
+    r->loop_only = !s->group_ctx || !hdk::dt_fits(r->W, r->H, r->D);
+    if (!r->loop_only) {
+        const size_t bases = (size_t)hdk::dt_bases(r->W, r->H, r->D);
+        r->group_bytes = 2 * packed + 2 * align_up(nb) * (r->dev_a ? 0 : 1) +
+                         2 * (align_up(4ULL * hdk::dt_vol_words(r->W, r->H, r->D)) + align_up(2 * bases) + align_up(8 * bases)) +
+                         align_up(8ULL * hdk::dt_cols(r->W, r->H)) + align_up(16ULL * (r->kmax + 1)) +
+                         align_up(4ULL * hdk::dt_list(r->W, r->H)) + 4096;  // 4096: descriptors and unused parts
+    }
 }
 
 // Marks a request done (server lock held) and lists it for wait_any.
@@ -226,6 +255,107 @@ void complete(hd_server* s, Request* r, hd_status st) {
     mark_done(s, r);
 }
 
+// Cancelled waiting requests leave at once.  Server lock held.
+void drop_cancelled(hd_server* s) {
+    for (auto it = s->waiting.begin(); it != s->waiting.end();) {
+        if ((*it)->cancel) {
+            (*it)->result.status = HD_ERR_CANCELLED;
+            mark_done(s, *it);
+            s->stats.cancelled += 1;
+            it = s->waiting.erase(it);
+        } else {
+            ++it;
+        }
+    }
+}
+
+// Takes waiting requests for one distance transform: the first ones that it
+// can take, within the free slots and the memory budget.  Server lock held.
+std::vector<Request*> take_group(hd_server* s) {
+    std::vector<Request*> g;
+    if (!s->group_ctx || s->waiting.size() < (size_t)kGroupMin) return g;
+    const size_t others = s->stats.bytes_in_use - s->group_held;
+    const size_t room = s->opt.hbm_budget_bytes > others ? s->opt.hbm_budget_bytes - others : 0;
+    const size_t most = std::min(s->free_slots.size(), (size_t)kGroupMax);
+    size_t bytes = 65536;
+    std::deque<Request*> left;
+    for (Request* r : s->waiting) {
+        if (g.size() < most && !r->loop_only && r->resident_bytes + r->transient_bytes <= s->opt.hbm_budget_bytes &&
+            bytes + r->group_bytes <= room) {
+            bytes += r->group_bytes;
+            g.push_back(r);
+        } else {
+            left.push_back(r);
+        }
+    }
+    if (g.size() < (size_t)kGroupMin) return {};
+    s->waiting.swap(left);
+    // the workspace grows by a quarter at least
+    DeviceArena& arena = s->group_ctx->arena;
+    size_t held = arena.cap;
+    if (bytes > arena.cap) {
+        held = std::max(bytes, arena.cap + arena.cap / 4);
+        if (held > room) {
+            arena.release();
+            held = bytes;
+        }
+    }
+    s->group_held = held;
+    s->stats.bytes_in_use = others + held;
+    s->stats.bytes_peak = std::max(s->stats.bytes_peak, s->stats.bytes_in_use);
+    for (Request* r : g) r->state = kResident;
+    s->in_group = (int)g.size();
+    return g;
+}
+
+// Solves a group; its requests are done afterwards, or (no memory) wait again
+// for the dilation loop.  Called with the server lock NOT held.
+void run_group(hd_server* s, const std::vector<Request*>& g) {
+    std::vector<PairIn> in;
+    for (const Request* r : g)
+        in.push_back(PairIn{r->dev_a, r->dev_b, r->W, r->H, r->D, r->dev_a ? nullptr : r->host_a.data(),
+                            r->dev_a ? nullptr : r->host_b.data()});
+    const int n = (int)g.size();
+    std::vector<hd_result> out(n);
+    constexpr int32_t kUnsolved = INT32_MIN;
+    for (hd_result& r : out) r.status = kUnsolved;
+    RunOpts ro;
+    ro.se = s->se;
+    ro.max_bytes = s->group_held;
+    hd_status st = HD_ERR_OOM;
+    const auto t_begin = std::chrono::steady_clock::now();
+    if (pick_shape(s->group_ctx, s->se, in.data(), n, true).kernel == 3)
+        st = run_pairs(s->group_ctx, in.data(), n, s->stream, ro, out.data());
+    if (s->debug)
+        std::fprintf(stderr, "[hd_server] group of %d pairs: %s, %.3f ms\n", n, hd_status_string(st),
+                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_begin).count());
+    std::lock_guard<std::mutex> lk(s->mu);
+    s->stats.bytes_in_use = s->stats.bytes_in_use - s->group_held + s->group_ctx->arena.cap;
+    s->group_held = s->group_ctx->arena.cap;
+    s->in_group = 0;
+    for (int i = n - 1; i >= 0; --i)
+        if (out[i].status == kUnsolved && st == HD_ERR_OOM && !g[i]->cancel) {
+            g[i]->loop_only = true;
+            g[i]->state = kWaiting;
+            s->waiting.push_front(g[i]);
+        }
+    for (int i = 0; i < n; ++i) {
+        Request* r = g[i];
+        if (r->state == kWaiting) continue;
+        if (r->cancel) {
+            r->result = hd_result{};
+            r->result.status = HD_ERR_CANCELLED;
+            mark_done(s, r);
+            s->stats.cancelled += 1;
+        } else {
+            const bool solved = out[i].status != kUnsolved;
+            r->result = solved ? out[i] : hd_result{};
+            complete(s, r, solved ? (hd_status)out[i].status : st);
+        }
+    }
+    s->done_cv.notify_all();
+}
+
 // One scheduler tick.  Called with the server lock NOT held.
 void tick(hd_server* s) {
     using clk = std::chrono::steady_clock;
@@ -233,19 +363,23 @@ void tick(hd_server* s) {
     std::vector<Request*> admit;
     int32_t ygen = 0;
     int used_hi = 0;  // slots [0, used_hi) hold every resident pair
+    bool grouped = false;
+    for (int i = 0; i < kGroupsPerTick; ++i) {
+        std::vector<Request*> g;
+        {
+            std::lock_guard<std::mutex> lk(s->mu);
+            drop_cancelled(s);
+            for (int q : s->quarantine) s->free_slots.push_back(q);
+            s->quarantine.clear();
+            g = take_group(s);
+        }
+        if (g.empty()) break;
+        run_group(s, g);
+        grouped = true;
+    }
     {
         std::lock_guard<std::mutex> lk(s->mu);
-        // cancelled waiting requests leave at once
-        for (auto it = s->waiting.begin(); it != s->waiting.end();) {
-            if ((*it)->cancel) {
-                (*it)->result.status = HD_ERR_CANCELLED;
-                mark_done(s, *it);
-                s->stats.cancelled += 1;
-                it = s->waiting.erase(it);
-            } else {
-                ++it;
-            }
-        }
+        drop_cancelled(s);
         for (int q : s->quarantine) s->free_slots.push_back(q);
         s->quarantine.clear();
         // Kernel shape per busy period: a server that starts work with few
@@ -272,6 +406,11 @@ void tick(hd_server* s) {
                 complete(s, r, HD_ERR_OOM);
                 continue;
             }
+            if (s->stats.bytes_in_use + need > s->opt.hbm_budget_bytes && s->group_held) {
+                s->group_ctx->arena.release();  // (idle here)
+                s->stats.bytes_in_use -= s->group_held;
+                s->group_held = 0;
+            }
             if (s->stats.bytes_in_use + need > s->opt.hbm_budget_bytes) break;
             r->nbricks = (unsigned long long)hdk::bricks_max(r->W, r->H, r->D, s->shape.bxw, s->shape.by, s->shape.bz);
             unsigned long long b0 = 0;
@@ -285,6 +424,11 @@ void tick(hd_server* s) {
             s->stats.bytes_in_use += need;
             s->stats.bytes_peak = std::max(s->stats.bytes_peak, s->stats.bytes_in_use);
             admit.push_back(r);
+        }
+        if (grouped && !any_resident && admit.empty()) {
+            s->stats.ticks += 1;
+            s->done_cv.notify_all();
+            return;
         }
         // submissions from here on advance the yield word (once per tick):
         // this tick's launch then ends at its next barrier so that they are
@@ -767,6 +911,17 @@ hd_status hd_server_create(hd_context* ctx, const hd_server_options* opt, hd_ser
             return e == cudaErrorMemoryAllocation ? HD_ERR_OOM : HD_ERR_CUDA;
         }
     }
+    if (s->se == 0 && !loop_asked(ctx->opt)) {
+        hd_options o = ctx->opt;
+        o.record_timings = 0;
+        o.tuning_table = nullptr;
+        if (hd_context_create(ctx->device, &o, &s->group_ctx) == HD_OK) {
+            std::lock_guard<std::mutex> lk(ctx->mu);
+            s->group_ctx->tune = ctx->tune;
+        } else {
+            s->group_ctx = nullptr;  // every request takes the loop
+        }
+    }
     s->slots.assign(slots, nullptr);
     s->slot_epoch.assign(slots, 0u);
     for (int i = slots - 1; i >= 0; --i) s->free_slots.push_back(i);
@@ -899,7 +1054,7 @@ hd_status hd_server_get_stats(hd_server* s, hd_server_stats* out) {
     out->waiting_pairs = s->waiting.size();
     unsigned long long res = 0;
     for (auto* r : s->slots) res += r != nullptr;
-    out->resident_pairs = res;
+    out->resident_pairs = res + s->in_group;
     return HD_OK;
 }
 
@@ -912,6 +1067,7 @@ hd_status hd_server_destroy(hd_server* s) {
         s->cv.notify_all();
     }
     if (s->worker.joinable()) s->worker.join();
+    hd_context_destroy(s->group_ctx);
     {
         DeviceGuard g(s->ctx->device);
         for (auto* r : s->slots)

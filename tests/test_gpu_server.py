@@ -181,3 +181,26 @@ def test_lone_request_then_burst_switches_kernel_shape(hd, ctx):
     assert same(r0, want_lone) and same(r1, want_lone)
     for i, (r, w) in enumerate(zip(res, want)):
         assert same(r, w), i
+
+
+@pytest.mark.parametrize("label,budget", [(0, 0), (3, 0), (0, 48 << 20), (0, 20 << 20)])
+def test_burst_in_groups(hd, label, budget):
+    """Requests that wait together are solved in groups, as the memory budget
+    allows; host and device masks, empty ones, a pair beyond the groups' sizes
+    and a request joining behind them get the plain path's results."""
+    pairs = _pairs(24, 51, lo=24, hi=112, edge=0.2)
+    z = torch.zeros((9, 20, 50), dtype=torch.uint8, device="cuda")
+    pairs += [(z, z), (z, z + 1), (z + 1, z + 1), (torch.ones((2, 513, 33), dtype=torch.uint8, device="cuda"),) * 2]
+    if label:
+        pairs = [tuple(m * label for m in p) for p in pairs]
+    with hd.Context(0, label=label) as c:
+        plain = [c.compute(a, b, "se6") for a, b in pairs]
+        with hd.Server(c, hbm_budget_bytes=budget) as srv:
+            for _ in range(2):
+                ts = [srv.submit(*((a.cpu().numpy(), b.cpu().numpy()) if i % 3 == 0 else (a, b)))
+                      for i, (a, b) in enumerate(pairs)]
+                for i, t in enumerate(ts):
+                    assert same(srv.wait(t, 60000), plain[i]), i
+            st = srv.stats()
+    assert st["completed"] == 2 * len(pairs) and st["waiting_pairs"] == st["resident_pairs"] == 0
+    assert not budget or st["bytes_peak"] <= budget
