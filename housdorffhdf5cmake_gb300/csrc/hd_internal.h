@@ -16,7 +16,7 @@ namespace hdh {
 struct DeviceArena {
     void* ptr = nullptr;
     size_t cap = 0;
-    cudaError_t ensure(size_t n);
+    cudaError_t ensure(size_t n, size_t most = ~size_t(0));  // n bytes, and a quarter more as long as it is within `most`
     void release();
 };
 

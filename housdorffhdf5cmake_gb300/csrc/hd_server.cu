@@ -290,16 +290,9 @@ std::vector<Request*> take_group(hd_server* s) {
     }
     if (g.size() < (size_t)kGroupMin) return {};
     s->waiting.swap(left);
-    // the workspace grows by a quarter at least
+    // the workspace: what it has, or up to a quarter more than is asked for
     DeviceArena& arena = s->group_ctx->arena;
-    size_t held = arena.cap;
-    if (bytes > arena.cap) {
-        held = std::max(bytes, arena.cap + arena.cap / 4);
-        if (held > room) {
-            arena.release();
-            held = bytes;
-        }
-    }
+    const size_t held = bytes <= arena.cap ? arena.cap : std::min(room, std::max(bytes, arena.cap) / 4 * 5);
     s->group_held = held;
     s->stats.bytes_in_use = others + held;
     s->stats.bytes_peak = std::max(s->stats.bytes_peak, s->stats.bytes_in_use);
