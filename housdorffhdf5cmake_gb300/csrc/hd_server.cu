@@ -9,7 +9,7 @@
 // as the single-pair path, bounded to tick_iterations steps; between ticks the
 // scheduler thread reads the jobs' states, completes finished pairs, frees
 // their memory and admits waiting ones.  Under the 6-neighbour element,
-// requests that wait together are first solved in groups by the distance
+// waiting requests are first solved in groups by the distance
 // transform (run_pairs on a context of the scheduler's own), between ticks.
 // Each pair's result depends only on its own masks, so it is identical alone
 // and in any mix.
@@ -116,15 +116,17 @@ constexpr int kWaitSpinUs = 1000;
 // kQueueForBatchMode wait.
 constexpr int kFewRequests = 2;
 constexpr int kQueueForBatchMode = 8;
-// Requests that wait together are solved by the distance transform in a
-// group, at least and at most this many, and that many groups before the
-// resident pairs' next tick; fewer join the resident pairs.  Bursts of requests
-// of 10 M voxels in the median (some of 512^3), in the dilation loop alone and
-// with groups of at least 2, 3, 4 and 8:
-//    3 requests  206 us | 250, 207, 210, 208
-//   10 requests  737 us | 610, 620, 664, 740
-//   24 requests 1359 us | 992, 986, 1030, 1091
+// Waiting requests are solved by the distance transform in a group: any number
+// of them (up to kGroupMax) while no pair is resident, but for a lone one of
+// more than kAloneVoxels, which stays in the loop, where later ones can join
+// it; at least kGroupMin beside resident pairs, kGroupsPerTick groups before
+// the next tick of those; fewer join them.  Bursts of 1, 3, 10 and 24 requests
+// of 10 M voxels in the median (some of 512^3), us from the first submission to
+// the last result: in the loop alone 129, 206, 737, 1359; in groups of at least 3
+// beside a first one in the loop 129, 207, 610, 985 (at least 2: 250 for three;
+// at least 8: 740, 1091 for 10 and 24); in groups at once 69, 152, 500-590, 878.
 constexpr int kGroupMin = 3, kGroupMax = 256, kGroupsPerTick = 8;
+constexpr long long kAloneVoxels = 1 << 26;
 
 }  // namespace
 
@@ -269,11 +271,16 @@ void drop_cancelled(hd_server* s) {
     }
 }
 
+bool any_resident(const hd_server* s) {
+    return std::any_of(s->slots.begin(), s->slots.end(), [](const Request* r) { return r != nullptr; });
+}
+
 // Takes waiting requests for one distance transform: the first ones that it
 // can take, within the free slots and the memory budget.  Server lock held.
 std::vector<Request*> take_group(hd_server* s) {
     std::vector<Request*> g;
-    if (!s->group_ctx || s->waiting.size() < (size_t)kGroupMin) return g;
+    if (!s->group_ctx) return g;
+    const size_t least = any_resident(s) ? kGroupMin : 1;
     const size_t others = s->stats.bytes_in_use - s->group_held;
     const size_t room = s->opt.hbm_budget_bytes > others ? s->opt.hbm_budget_bytes - others : 0;
     const size_t most = std::min(s->free_slots.size(), (size_t)kGroupMax);
@@ -288,7 +295,8 @@ std::vector<Request*> take_group(hd_server* s) {
             left.push_back(r);
         }
     }
-    if (g.size() < (size_t)kGroupMin) return {};
+    if (g.size() < least) return {};
+    if (g.size() == 1 && (long long)g[0]->W * g[0]->H * g[0]->D > kAloneVoxels) return {};
     s->waiting.swap(left);
     // the workspace: what it has, or up to a quarter more than is asked for
     DeviceArena& arena = s->group_ctx->arena;
@@ -357,10 +365,15 @@ void tick(hd_server* s) {
     int32_t ygen = 0;
     int used_hi = 0;  // slots [0, used_hi) hold every resident pair
     bool grouped = false;
-    for (int i = 0; i < kGroupsPerTick; ++i) {
+    for (int i = 0;; ++i) {
         std::vector<Request*> g;
         {
             std::lock_guard<std::mutex> lk(s->mu);
+            if (s->stop) break;
+            // others' turn: resident pairs, requests for the loop
+            if (i >= kGroupsPerTick &&
+                (any_resident(s) || std::any_of(s->waiting.begin(), s->waiting.end(), [](Request* r) { return r->loop_only; })))
+                break;
             drop_cancelled(s);
             for (int q : s->quarantine) s->free_slots.push_back(q);
             s->quarantine.clear();

@@ -266,11 +266,12 @@ typedef struct hd_server_options {
 } hd_server_options;
 
 void hd_server_options_init(hd_server_options* opt);
-/* Starts a server with its own scheduler thread on ctx's device.  Requests
- * that wait together under HD_SE6 (three or more) are solved in groups by the
- * distance transform (hd_options.kernel: unless an option of ctx asks for the
- * dilation loop), within the memory budget, whose bytes_in_use then holds the
- * groups' workspace; others join the persistent dilation loop. */
+/* Starts a server with its own scheduler thread on ctx's device.  Under HD_SE6
+ * waiting requests are solved in groups by the distance transform
+ * (hd_options.kernel: unless an option of ctx asks for the dilation loop),
+ * within the memory budget, whose bytes_in_use then holds the groups'
+ * workspace; a lone request of more than 2^26 voxels, one or two that arrive
+ * beside it, and what the transform cannot take join the persistent loop. */
 hd_status hd_server_create(hd_context* ctx, const hd_server_options* opt, hd_server** out);
 /* Queues a pair (host masks are copied in before submit returns unless
  * on_device; device masks must stay valid until the request completes). */
