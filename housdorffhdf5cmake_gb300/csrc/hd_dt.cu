@@ -142,8 +142,7 @@ __device__ __forceinline__ void plane_sync(int id, int threads) {
 // against 19 to 22 us with the words in groups of four registers, 512^3 with
 // small blobs (both directions) 51 to 65 against 97 to 114 us.  The barrier
 // per word column is among the plane's warps only (62 registers against 78, 256
-// ragged pairs' planes and columns 0.767 against 0.791 ms).  4 CTAs per SM: 512^3
-// 165 against 159 us a call, the ragged batch 2 % slower.
+// ragged pairs' planes and columns 0.767 against 0.791 ms).
 
 // Plane z of a direction: this warp's tile t (a warp without one: act false).
 // claimed() is called once, before the first barrier.
@@ -306,10 +305,18 @@ __device__ __forceinline__ void plane_unit(const DtPair& p, const Geom& g, int j
 }
 
 // Planes per CTA: as many as its warps have tiles for, but no fewer CTAs than
-// the grid (most: the grid's share of all planes).
+// are resident (most: planes per resident CTA).
 __device__ __forceinline__ int planes_per_cta(const Geom& g, int most) { return max(1, min(kPlaneWarps / g.ntile, most)); }
 
-__global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __grid_constant__ DtPair p) {
+// One pair: a CTA per group of planes, so that the next group goes to whichever
+// SM is free (planes without a source, or with few words, end early; 512^3 160
+// to 154 us a call against one wave of CTAs that take every n-th).  kCtas per SM:
+// 2 (96 registers) on the whole GPU, where a CTA's time counts (512^3 141, six
+// 301x287x173 pairs 186.7 us), 3 (62) on a group of 48 SMs, where there are
+// more planes than CTAs (eight 512x512x256 pairs 396 us); the other way
+// round 154, 189 and 401 us.
+template <int kCtas>
+__global__ void __launch_bounds__(kPlaneWarps * 32, kCtas) dt_plane_kernel(const __grid_constant__ DtPair p, int sms) {
     extern __shared__ uint4 sm4[];
     cudaGridDependencySynchronize();  // placed as the packing ends
     const PairInfo I = *p.info;
@@ -320,15 +327,14 @@ __global__ void __launch_bounds__(kPlaneWarps * 32, 3) dt_plane_kernel(const __g
     const int nact = dt_directions(I);
     if (nact == 0) return;
     const Geom g = dt_geom(I);
-    const int G = planes_per_cta(g, nact * g.d / (int)gridDim.x);
+    const int G = planes_per_cta(g, nact * g.d / (kCtas * sms));
     const int groups = (g.d + G - 1) / G, warp = threadIdx.x >> 5;
     const int pl = warp / g.ntile, t = warp - pl * g.ntile;
-#pragma unroll 1
-    for (int u = blockIdx.x; u < nact * groups; u += gridDim.x) {
-        const int j = nact == 2 ? (u >= groups) : !(I.n_b > I.n_ab);
-        const int z = (nact == 2 && j ? u - groups : u) * G + pl;
-        plane_unit(p, g, j, z, t, pl < G && z < g.d, (uint32_t*)sm4, [] {});
-    }
+    const int u = blockIdx.x;
+    if (u >= nact * groups) return;
+    const int j = nact == 2 ? (u >= groups) : !(I.n_b > I.n_ab);
+    const int z = (nact == 2 && j ? u - groups : u) * G + pl;
+    plane_unit(p, g, j, z, t, pl < G && z < g.d, (uint32_t*)sm4, [] {});
 }
 
 // Several pairs: their units in one list, claimed from a counter one ahead;
@@ -949,7 +955,8 @@ bool dt_fits(int W, int H, int D) {
 
 namespace {
 
-constexpr int kPlaneCtas = 3;  // resident CTAs per SM
+constexpr int kPlaneCtas = 3;  // resident CTAs per SM (several pairs)
+constexpr int kWholeSms = 100; // launches on fewer SMs share the GPU with others
 
 size_t plane_smem(int quads, int pairs) {
     return sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)quads * 4 * kPlaneWarps * 32) +
@@ -967,7 +974,8 @@ cudaError_t raise_limits() {
     if (e != cudaSuccess || (dev < 64 && raised[dev].load(std::memory_order_acquire))) return e;
     const int lim = 200 * 1024;  // above any size taken (dt_fits), with the static part below 227 KB
     const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    e = cudaFuncSetAttribute(&dt_plane_kernel, attr, lim);
+    e = cudaFuncSetAttribute(&dt_plane_kernel<2>, attr, lim);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_plane_kernel<3>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_planes_kernel, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_depth_kernel<false>, attr, lim);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(&dt_depth_kernel<true>, attr, lim);
@@ -1001,11 +1009,11 @@ cudaError_t launch_dt(const DtPair& p, int sms, cudaStream_t s) {
     cudaError_t e = raise_limits();
     if (e != cudaSuccess) return e;
     const int nseg = segs_of(p), dwarps = nseg > 2 ? kDepthMaxWarps : 4;
-    // one resident wave, or fewer CTAs than that for small volumes
-    const long long pg = std::min<long long>(2ll * p.D, (long long)kPlaneCtas * sms);
-    const long long dg = std::min<long long>(dt_list(p.W, p.H), 4ll * kDepthMaxWarps / dwarps * sms);
-    e = launch_early(dt_plane_kernel, pg, kPlaneWarps * 32, plane_smem(quads_of(p), 0), s, p);
+    e = launch_early(sms < kWholeSms ? dt_plane_kernel<3> : dt_plane_kernel<2>, 2ll * p.D, kPlaneWarps * 32,
+                     plane_smem(quads_of(p), 0), s, p, sms);
     if (e != cudaSuccess) return e;
+    // one resident wave, or fewer CTAs than that for small volumes
+    const long long dg = std::min<long long>(dt_list(p.W, p.H), 4ll * kDepthMaxWarps / dwarps * sms);
     return launch_early(p.map[0] ? dt_depth_kernel<true> : dt_depth_kernel<false>, dg, dwarps * 32,
                         depth_smem(dwarps, nseg, p.W + p.H + p.D, p.ncols), s, p);
 }
