@@ -310,11 +310,8 @@ __device__ __forceinline__ int planes_per_cta(const Geom& g, int most) { return 
 
 // One pair: a CTA per group of planes, so that the next group goes to whichever
 // SM is free (planes without a source, or with few words, end early; 512^3 160
-// to 154 us a call against one wave of CTAs that take every n-th).  kCtas per SM:
-// 2 (96 registers) on the whole GPU, where a CTA's time counts (512^3 141, six
-// 301x287x173 pairs 186.7 us), 3 (62) on a group of 48 SMs, where there are
-// more planes than CTAs (eight 512x512x256 pairs 396 us); the other way
-// round 154, 189 and 401 us.
+// to 154 us a call against one wave of CTAs that take every n-th).  kCtas per
+// SM: plane_ctas.
 template <int kCtas>
 __global__ void __launch_bounds__(kPlaneWarps * 32, kCtas) dt_plane_kernel(const __grid_constant__ DtPair p, int sms) {
     extern __shared__ uint4 sm4[];
@@ -956,7 +953,19 @@ bool dt_fits(int W, int H, int D) {
 namespace {
 
 constexpr int kPlaneCtas = 3;  // resident CTAs per SM (several pairs)
-constexpr int kWholeSms = 100; // launches on fewer SMs share the GPU with others
+
+// Resident CTAs per SM of one pair's planes.  3 (62 registers) on a group of 48
+// SMs, where there are always more planes than CTAs (eight 512x512x256 pairs 396
+// against 401 us), and where the planes of both directions, about 3/4 of all
+// as the domain is smaller than the volume, fill 2 per SM but not much more than
+// 3 (two 512x512x256 pairs 45.6 against 49.4 us, 256x256x200 of 400 planes 45.6
+// against 49.7).  Else 2 (96 registers or more): a plane's own time counts
+// (301x287x173 187 against 189 us for six), and many planes without a source
+// (512^3 141 against 154 us a call).
+int plane_ctas(int D, int sms) {
+    const double planes = 1.5 * D;
+    return sms < 100 || (planes > 2 * sms && planes <= 3.5 * sms) ? 3 : 2;
+}
 
 size_t plane_smem(int quads, int pairs) {
     return sizeof(uint32_t) * (kPlaneWarps * kTr + kPlaneEnds + (size_t)quads * 4 * kPlaneWarps * 32) +
@@ -1009,7 +1018,7 @@ cudaError_t launch_dt(const DtPair& p, int sms, cudaStream_t s) {
     cudaError_t e = raise_limits();
     if (e != cudaSuccess) return e;
     const int nseg = segs_of(p), dwarps = nseg > 2 ? kDepthMaxWarps : 4;
-    e = launch_early(sms < kWholeSms ? dt_plane_kernel<3> : dt_plane_kernel<2>, 2ll * p.D, kPlaneWarps * 32,
+    e = launch_early(plane_ctas(p.D, sms) == 3 ? dt_plane_kernel<3> : dt_plane_kernel<2>, 2ll * p.D, kPlaneWarps * 32,
                      plane_smem(quads_of(p), 0), s, p, sms);
     if (e != cudaSuccess) return e;
     // one resident wave, or fewer CTAs than that for small volumes
