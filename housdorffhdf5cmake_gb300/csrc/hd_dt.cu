@@ -141,8 +141,8 @@ __device__ __forceinline__ void plane_sync(int id, int threads) {
 // words come one at a time after that, from L1): 512x512x256 pair 16 to 19 us
 // against 19 to 22 us with the words in groups of four registers, 512^3 with
 // small blobs (both directions) 51 to 65 against 97 to 114 us.  The barrier
-// per word column is among the plane's warps only (62 registers against 78, 256
-// ragged pairs' planes and columns 0.767 against 0.791 ms).
+// per word column is among the plane's warps only (256 ragged pairs' planes and
+// columns 0.767 against 0.791 ms).
 
 // Plane z of a direction: this warp's tile t (a warp without one: act false).
 // claimed() is called once, before the first barrier.
@@ -954,12 +954,12 @@ namespace {
 
 constexpr int kPlaneCtas = 3;  // resident CTAs per SM (several pairs)
 
-// Resident CTAs per SM of one pair's planes.  3 (62 registers) on a group of 48
+// Resident CTAs per SM of one pair's planes.  3 (80 registers) on a group of 48
 // SMs, where there are always more planes than CTAs (eight 512x512x256 pairs 396
 // against 401 us), and where the planes of both directions, about 3/4 of all
 // as the domain is smaller than the volume, fill 2 per SM but not much more than
 // 3 (two 512x512x256 pairs 45.6 against 49.4 us, 256x256x200 of 400 planes 45.6
-// against 49.7).  Else 2 (96 registers or more): a plane's own time counts
+// against 49.7).  Else 2 (122 registers): a plane's own time counts
 // (301x287x173 187 against 189 us for six), and many planes without a source
 // (512^3 141 against 154 us a call).
 int plane_ctas(int D, int sms) {
