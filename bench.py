@@ -516,7 +516,7 @@ def bench_batched(ctx, args):
         tctx.compute(a, b, "se6")
         dev_plain += tctx.last_timings()["total_ms"]
     gvox = sum(max(0, r["hd"]) * 2 * (s.shape[0] * s.shape[1] * s.shape[2]) for r, s in zip(batch, specs))
-    # roofline of the batch's dilation launch: the frontier bytes of every
+    # roofline of the batch's solve: in the dilation loop the frontier bytes of every
     # pair (32^3 tiles gaining voxels per step, counted by the instrumented
     # run) over the batch's solve time
     tiles = 0
@@ -526,6 +526,10 @@ def bench_batched(ctx, args):
         res, tab, tba, _ = ctx.profile(a, b, "se6")
         tiles += int(sum(int(v) for v in tab[1: res["hd_ab"] + 1]) + sum(int(v) for v in tba[1: res["hd_ba"] + 1]))
     b_iter = 3 * 4096 * tiles
+    if bt["kernel"] == 3:
+        # distance transform: a byte per voxel of each pair's domain and
+        # direction, written once and read once
+        b_iter = sum(4 * _domain_voxels(a, b) for (a, b), r in zip(pairs, batch) if r["hd"] > 0)
     peak, peak_kind = _peaks()
     solve_gbs = b_iter / (bt["solve_ms"] * 1e-3) / 1e9
     out = {
@@ -769,7 +773,7 @@ def bench_worst_case(ctx, tctx, dev):
     per_step = [(int(tab[k]) if k <= res["hd_ab"] else 0) + (int(tba[k]) if k <= res["hd_ba"] else 0)
                 for k in range(1, steps + 1)]
     frac = [x / (2 * n_tiles) for x in per_step]
-    alg = 3 * 4096 * sum(per_step)
+    alg = 4 * _domain_voxels(a, b) if tim["kernel"] == 3 else 3 * 4096 * sum(per_step)
     return {
         "workload": "512^3, 8 balls r 3-6 vs 8 balls >= 200 voxels away, 6-neighbour element",
         "hd": r["hd"], "checked_against_oracle": bool(checked),
