@@ -307,6 +307,19 @@ __device__ __forceinline__ void put_words(const PackWalk& k, const PackSpan& n, 
     }
 }
 
+// Asks for the bytes of a span of aligned words of both masks (from byte lo
+// on), a line per lane, in L2.  Taken on part of the SMs, where the packing is bound
+// by the latency of its loads (eight pipelined 512x512x256 pairs 395 -> 363 us;
+// two spans ahead 366); on all of them HBM is the bound (512^3 141 against 143
+// us), and the kernel for other words waits for its instructions (509x511x250
+// 60.5 against 60.8 us a pair).
+__device__ __forceinline__ void fetch_ahead(const PackWalk& k, size_t lo) {
+    const size_t o = lo + 128u * (threadIdx.x & 31);
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+        if (o < k.nbytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(k.src[m] + o));
+}
+
 // 32 mask bytes at p (32-byte aligned), read once: one 256-bit load, first to
 // leave L2 (without that hint 512x512x256 takes 32 instead of 27 us: the
 // masks push the packed words and the next kernels' data out).
@@ -322,7 +335,7 @@ __device__ __forceinline__ void load32(const uint8_t* p, uint32_t (&v)[8]) {
 // stream, at less than half the instructions.  On every SM it is as fast as
 // the other kernel (27 us at 512x512x256, 51 at 512^3: HBM), on the 56 SMs of
 // the pipelined entry, where instructions count, 44 against 58 us.
-template <bool kLabel>
+template <bool kLabel, bool kAhead>
 __device__ __forceinline__ void pack_aligned(const PackWalk& k, unsigned t0, unsigned t1, unsigned r, unsigned w,
                                              unsigned y, PackAcc& acc, unsigned label) {
     const int lane = threadIdx.x & 31;
@@ -335,6 +348,7 @@ __device__ __forceinline__ void pack_aligned(const PackWalk& k, unsigned t0, uns
 #pragma unroll
             for (int i = 0; i < kWords; ++i)
                 load32(k.src[m] + 32 * (size_t)min(t0 + 32u * i + lane, k.total - 1u), v[m][i]);
+        if (kAhead && t0 + (unsigned)kPackTileWords < t1) fetch_ahead(k, 32 * (size_t)(t0 + (unsigned)kPackTileWords));
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
             bool general = kLabel;
@@ -388,7 +402,7 @@ __device__ __forceinline__ void pack_aligned(const PackWalk& k, unsigned t0, uns
 // warp on a contiguous share of the CTA's run 1.043 ms).  64-word spans at 3
 // CTAs per SM were 14 % slower at 512^3, with the next span's loads issued
 // between the two masks' 37 %.
-template <bool kLabel, bool kAligned>
+template <bool kLabel, bool kAligned, bool kAhead = false>
 __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const PairDesc* __restrict__ descs, int npairs,
                                                                long long ntiles, int label,
                                                                const __grid_constant__ PairDesc one, Ctl* ctl, uint32_t* zero, int nzero,
@@ -417,7 +431,7 @@ __global__ void __launch_bounds__(kPackThreads, kPackCtas) pack_kernel(const Pai
         unsigned r = (t0 + lane) / k.wxf;
         unsigned w = t0 + lane - r * k.wxf;
         unsigned y = r % k.H;
-        if constexpr (kAligned) pack_aligned<kLabel>(k, t0, t1, r, w, y, acc, (unsigned)label);
+        if constexpr (kAligned) pack_aligned<kLabel, kAhead>(k, t0, t1, r, w, y, acc, (unsigned)label);
 #pragma unroll 1
         for (; !kAligned && t0 < t1; t0 += (unsigned)kPackTileWords) {
             const PackSpan n = locate(k, t0, __shfl_sync(0xffffffffu, r, 0), __shfl_sync(0xffffffffu, w, 0));
@@ -804,12 +818,15 @@ cudaError_t launch_pack(const PairDesc* d_descs, int npairs, long long ntiles, i
     // a single pair of 32-byte aligned words takes the kernel without the bit stream
     const PairDesc P = one ? *one : PairDesc{};
     const bool aligned = one && (P.W & 31) == 0 && (((uintptr_t)P.a | (uintptr_t)P.b) & 31) == 0;
-    const int v = (label ? 1 : 0) + (aligned ? 2 : 0);
-    auto* const fn = v == 0 ? pack_kernel<false, false> : v == 1 ? pack_kernel<true, false>
-                   : v == 2 ? pack_kernel<false, true> : pack_kernel<true, true>;
+    const int v = (label ? 1 : 0) + (aligned ? (sms > 0 ? 4 : 2) : 0);
+    using Kernel = void (*)(const PairDesc*, int, long long, int, PairDesc, Ctl*, uint32_t*, int, bool);
+    static const Kernel kernels[6] = {pack_kernel<false, false>,      pack_kernel<true, false>,
+                                      pack_kernel<false, true>,       pack_kernel<true, true>,
+                                      pack_kernel<false, true, true>, pack_kernel<true, true, true>};
+    const Kernel fn = kernels[v];
     // one wave of resident CTAs (per device and variant, from the occupancy calculator)
-    static int resident[4][64] = {{0}};
-    static int per_sm_of[4][64] = {{0}};
+    static int resident[6][64] = {{0}};
+    static int per_sm_of[6][64] = {{0}};
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
