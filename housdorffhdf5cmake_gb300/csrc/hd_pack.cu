@@ -310,9 +310,10 @@ __device__ __forceinline__ void put_words(const PackWalk& k, const PackSpan& n, 
 // Asks for the bytes of a span of aligned words of both masks (from byte lo
 // on), a line per lane, in L2.  Taken on part of the SMs, where the packing is bound
 // by the latency of its loads (eight pipelined 512x512x256 pairs 395 -> 363 us;
-// two spans ahead 366); on all of them HBM is the bound (512^3 141 against 143
-// us), and the kernel for other words waits for its instructions (509x511x250
-// 60.5 against 60.8 us a pair).
+// two spans ahead 366, bulk prefetches that leave L2 first the same; pairs whose
+// distances take the longer part 1 % slower); on all of them HBM is the bound
+// (512^3 141 against 143 us), and the kernel for other words waits for its
+// instructions (509x511x250 60.5 against 60.8 us a pair).
 __device__ __forceinline__ void fetch_ahead(const PackWalk& k, size_t lo) {
     const size_t o = lo + 128u * (threadIdx.x & 31);
 #pragma unroll
