@@ -753,6 +753,7 @@ __global__ void __launch_bounds__(kListThreads) dt_list_kernel(const DtPair* man
     const int lane = threadIdx.x & 31;
     const PairInfo I = *p.info;
     const int nact = dt_directions(I);
+    __syncthreads();  // every thread has its copy: the decode puts *p.info back to the start values
     if (nact == 0) {
         if (threadIdx.x < 32) dt_decode(p, I);
         return;

@@ -131,3 +131,22 @@ def test_map_values_outside_the_transform(hd, shape, offset, label):
         _, ma, mb = c.distance_map(a, b, "se6")
     for m, own, other in ((ma, fa, fb), (mb, fb, fa)):
         assert bool((m[~own] == -1).all()) and bool((m[own & other] == 0).all()) and bool((m[own & ~other] >= 1).all())
+
+
+def test_groups_of_pairs_without_targets(hd, loop):
+    """Full groups of identical, one-sided empty and empty masks, whose results are
+    decoded (and whose counts are put back) where the columns are listed, with a
+    few pairs that have columns between them, many times over."""
+    rng = np.random.default_rng(7)
+    pairs = []
+    for i in range(128):
+        a, b = masks(rng, SHAPES[1 + 7 * i % 15], ("random", "slabs")[i % 2])
+        z = np.zeros_like(a)
+        pairs.append(((a, a), (a, z), (z, b), (z, z), (b, b))[i % 5] if i % 16 else (a, b))
+    dev = [tuple(torch.from_numpy(m).cuda() for m in p) for p in pairs]
+    want = [loop.compute(*p, "se6") for p in dev]
+    with hd.Context(0) as c:
+        batch = c.prepare_batch(dev, "se6")
+        for turn in range(50):
+            for i, (g, w) in enumerate(zip(batch.run(), want)):
+                same(g, w, (turn, i))
