@@ -465,6 +465,16 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
                     hd_result* out) {
     if (n <= 0) return HD_OK;
     if (n > hdk::kMaxPairsPerLaunch) return set_error(ctx, HD_ERR_BAD_ARG, "too many pairs in one launch");
+    {
+        // Not under stream capture: the workspace and the step counter belong
+        // to the calls, not to a replay.  Refused before any other call of the
+        // runtime (an allocation, an event of another stream would end the
+        // caller's capture, and a workspace could not be given back).
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        cudaError_t e = cudaStreamIsCapturing(s, &cap);
+        if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "stream");
+    }
     const int se = ro.se;
     const bool stats = ro.stats != 0;
     Shape sh = ro.force_shape ? ro.shape : pick_shape(ctx, se, pairs, n, !stats);
@@ -695,14 +705,6 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         if (e != cudaSuccess) return cuda_fail(ctx, e, "stamp reset");
         ctx->stamp_slots = want;
         ctx->g_next = 1;
-    }
-    {
-        // not under stream capture: the workspace and the step counter belong
-        // to the calls, not to a replay
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        e = cudaStreamIsCapturing(s, &cap);
-        if (e == cudaSuccess && cap != cudaStreamCaptureStatusNone) e = cudaErrorStreamCaptureUnsupported;
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "stream");
     }
     if (!async) {
         e = ctx->pinned.ensure(pinned_bytes);
