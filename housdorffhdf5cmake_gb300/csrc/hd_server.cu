@@ -127,6 +127,7 @@ constexpr int kQueueForBatchMode = 8;
 // at least 8: 740, 1091 for 10 and 24); in groups at once 69, 152, 500-590, 878.
 constexpr int kGroupMin = 3, kGroupMax = 256, kGroupsPerTick = 8;
 constexpr long long kAloneVoxels = 1 << 26;
+constexpr size_t kGroupBytes = 65536;  // of a group's workspace, besides its pairs' shares
 
 }  // namespace
 
@@ -238,6 +239,8 @@ void plan_request(hd_server* s, Request* r) {
                          2 * (align_up(4ULL * hdk::dt_vol_words(r->W, r->H, r->D)) + align_up(2 * bases) + align_up(8 * bases)) +
                          align_up(8ULL * hdk::dt_cols(r->W, r->H)) + align_up(16ULL * (r->kmax + 1)) +
                          align_up(4ULL * hdk::dt_list(r->W, r->H)) + 4096;  // 4096: descriptors and unused parts
+        // no group can hold it, the loop may
+        r->loop_only = kGroupBytes + r->group_bytes > s->opt.hbm_budget_bytes;
     }
 }
 
@@ -276,20 +279,23 @@ bool any_resident(const hd_server* s) {
 }
 
 // Takes waiting requests for one distance transform: the first ones that it
-// can take, within the free slots and the memory budget.  Server lock held.
-std::vector<Request*> take_group(hd_server* s) {
+// can take, within the free slots and the memory budget; `passed` becomes true
+// if one of them waited behind a request that stays.  Server lock held.
+std::vector<Request*> take_group(hd_server* s, bool& passed) {
     std::vector<Request*> g;
     if (!s->group_ctx) return g;
     const size_t least = any_resident(s) ? kGroupMin : 1;
     const size_t others = s->stats.bytes_in_use - s->group_held;
     const size_t room = s->opt.hbm_budget_bytes > others ? s->opt.hbm_budget_bytes - others : 0;
     const size_t most = std::min(s->free_slots.size(), (size_t)kGroupMax);
-    size_t bytes = 65536;
+    size_t bytes = kGroupBytes;
+    bool over = false;
     std::deque<Request*> left;
     for (Request* r : s->waiting) {
         if (g.size() < most && !r->loop_only && r->resident_bytes + r->transient_bytes <= s->opt.hbm_budget_bytes &&
             bytes + r->group_bytes <= room) {
             bytes += r->group_bytes;
+            over = over || !left.empty();
             g.push_back(r);
         } else {
             left.push_back(r);
@@ -297,6 +303,7 @@ std::vector<Request*> take_group(hd_server* s) {
     }
     if (g.size() < least) return {};
     if (g.size() == 1 && (long long)g[0]->W * g[0]->H * g[0]->D > kAloneVoxels) return {};
+    passed = passed || over;
     s->waiting.swap(left);
     // the workspace: what it has, or up to a quarter more than is asked for
     DeviceArena& arena = s->group_ctx->arena;
@@ -364,20 +371,19 @@ void tick(hd_server* s) {
     std::vector<Request*> admit;
     int32_t ygen = 0;
     int used_hi = 0;  // slots [0, used_hi) hold every resident pair
-    bool grouped = false;
+    bool grouped = false, passed = false;
     for (int i = 0;; ++i) {
         std::vector<Request*> g;
         {
             std::lock_guard<std::mutex> lk(s->mu);
             if (s->stop) break;
-            // others' turn: resident pairs, requests for the loop
-            if (i >= kGroupsPerTick &&
-                (any_resident(s) || std::any_of(s->waiting.begin(), s->waiting.end(), [](Request* r) { return r->loop_only; })))
-                break;
+            // others' turn: resident pairs, and requests that groups have passed
+            // over, which the admission below takes strictly from the front
+            if (i >= kGroupsPerTick && (passed || any_resident(s))) break;
             drop_cancelled(s);
             for (int q : s->quarantine) s->free_slots.push_back(q);
             s->quarantine.clear();
-            g = take_group(s);
+            g = take_group(s, passed);
         }
         if (g.empty()) break;
         run_group(s, g);
