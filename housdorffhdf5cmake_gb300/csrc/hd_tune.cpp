@@ -62,6 +62,7 @@ bool TuneTable::load(const std::string& path) {
     const std::string s = ss.str();
     size_t pos = s.find("\"entries\"");
     if (pos == std::string::npos) return false;
+    pos += 9;  // behind "entries"
     auto field = [](const std::string& body, const char* name, double* v) {
         const std::string key = std::string("\"") + name + "\"";
         size_t p = body.find(key);
@@ -72,7 +73,7 @@ bool TuneTable::load(const std::string& path) {
         return true;
     };
     while (true) {
-        size_t k0 = s.find('"', pos + 9);
+        size_t k0 = s.find('"', pos);
         if (k0 == std::string::npos) break;
         size_t k1 = s.find('"', k0 + 1);
         size_t b0 = s.find('{', k1);
@@ -100,7 +101,7 @@ bool TuneTable::load(const std::string& path) {
             e.us = us;
             entries[key] = e;
         }
-        pos = b1;
+        pos = b1 + 1;
     }
     return true;
 }

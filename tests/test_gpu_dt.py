@@ -150,3 +150,23 @@ def test_groups_of_pairs_without_targets(hd, loop):
         for turn in range(50):
             for i, (g, w) in enumerate(zip(batch.run(), want)):
                 same(g, w, (turn, i))
+
+
+def test_tuning_table_of_several_entries(hd, loop, tmp_path):
+    """Every entry of a table is read: workload classes with an entry of the loop
+    take it, one whose entry names the transform and one without an entry do not."""
+    rng = np.random.default_rng(8)
+    entry = lambda kernel, steps: (f'{{"kernel": {kernel}, "bxw": 4, "bz": 8, "steps": {steps}, "ctas_per_sm": 0, '
+                                   '"order": 0, "spread": 0, "us": 1.5}')
+    table = {"se6/v12/p1": entry(2, 3), "se6/v15/p1": entry(1, 1), "se6/v15/p2": entry(2, 2), "se6/v18/p1": entry(3, 0)}
+    path = tmp_path / "table.json"
+    path.write_text('{\n  "version": 1,\n  "entries": {' + ",".join(f'\n    "{k}": {v}' for k, v in table.items()) +
+                    "\n  }\n}\n")  # as the library writes it
+    with hd.Context(0, tuning_table=str(path), record_timings=True) as c:
+        for side, n, kernel, steps in ((16, 1, 2, 3), (32, 1, 1, 1), (32, 4, 2, 2), (64, 1, 3, 0), (64, 4, 3, 0)):
+            a, b = (torch.from_numpy(m).cuda() for m in masks(rng, (side,) * 3, "random"))
+            want = loop.compute(a, b, "se6")
+            for g in [c.compute(a, b, "se6")] if n == 1 else c.batch([(a, b)] * n, "se6"):
+                same(g, want, (side, n))
+            t = c.last_timings()
+            assert (t["kernel"], t["steps_per_barrier"]) == (kernel, steps), (side, n, t)
