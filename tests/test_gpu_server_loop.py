@@ -1,6 +1,11 @@
 """The server where its groups (the distance transform) do not solve every
-request: requests that only the dilation loop can take, among ones that groups
-take."""
+request: requests that only the dilation loop can take among ones that groups
+take, and servers whose element or options ask for the loop.  A result whose
+`iterations` is not 0 came from the loop."""
+import json
+import time
+
+import numpy as np
 import pytest
 import torch
 
@@ -43,3 +48,94 @@ def test_request_for_the_loop_before_many_others(hd, ctx, shape, budget):
         st = srv.stats()
     assert at < before + after // 2, at
     assert not budget or st["bytes_peak"] <= budget
+
+
+LOOP = [("se18", {}), ("se6", {"kernel": 2})]
+
+
+def _from_loop(r):
+    return r["iterations"] > 0 or r["hd"] <= 0
+
+
+@pytest.mark.parametrize("metric,opts", LOOP)
+def test_lone_request_then_burst(hd, metric, opts):
+    """A long lone request, then a burst that fills the two slots and queues up
+    behind: the server drains and goes on in its other brick shape, and the lone
+    request after the burst has the first shape again."""
+    lone = synth.pair_far_blobs(3, (192, 192, 192), "cuda", min_dist=75.0)
+    burst = _pairs(30, 41, 32, 96, edge=0.1)
+    with hd.Context(0, **opts) as c:
+        want_lone, want = c.compute(*lone, metric), [c.compute(*p, metric) for p in burst]
+        with hd.Server(c, metric=metric, max_inflight=2) as srv:
+            for _ in range(3):
+                t0 = srv.submit(*lone)
+                ts = [srv.submit(*p) for p in burst]
+                res = [srv.wait(t, 60000) for t in ts] + [srv.wait(t0, 60000)]
+                for i, (r, w) in enumerate(zip(res, want + [want_lone])):
+                    assert same(r, w) and _from_loop(r), i
+                r = srv.wait(srv.submit(*lone), 60000)
+                assert same(r, want_lone) and _from_loop(r)
+
+
+@pytest.mark.parametrize("metric,opts", LOOP)
+def test_cancel_in_the_loop(hd, metric, opts):
+    """A pair cancelled while it dilates leaves the loop; pairs beside it and pairs
+    that take its slot afterwards get their own results."""
+    far = synth.pair_far_blobs(5, (512, 512, 512), "cuda")
+    pairs = _pairs(6, 43, 64, 128)
+    with hd.Context(0, **opts) as c:
+        want = [c.compute(*p, metric) for p in pairs]
+        with hd.Server(c, metric=metric, tick_iterations=1, max_inflight=3) as srv:
+            for _ in range(2):
+                tf = srv.submit(*far)
+                t0 = time.time()
+                while srv.stats()["resident_pairs"] == 0 and time.time() - t0 < 10:
+                    pass
+                ts = [srv.submit(*p) for p in pairs[:2]]
+                srv.cancel(tf)
+                ts += [srv.submit(*p) for p in pairs[2:]]
+                assert srv.wait(tf, 60000)["status"] == hd.HD_ERR_CANCELLED
+                for i, t in enumerate(ts):
+                    r = srv.wait(t, 60000)
+                    assert same(r, want[i]) and _from_loop(r), i
+            st = srv.stats()
+    assert st["cancelled"] == 2 and st["resident_pairs"] == st["waiting_pairs"] == 0
+
+
+@pytest.mark.parametrize("metric,opts", LOOP)
+def test_budget_and_mix_in_the_loop(hd, metric, opts):
+    """Loop admission under a budget of a few pairs, an oversize request, and each
+    result the same alone and in the mix."""
+    pairs = _pairs(16, 13, 64, 96)
+    budget = 24 << 20
+    with hd.Context(0, **opts) as c:
+        want = [c.compute(*p, metric) for p in pairs]
+        with hd.Server(c, metric=metric, hbm_budget_bytes=budget, tick_iterations=2) as srv:
+            for i in (0, 9):
+                r = srv.wait(srv.submit(*pairs[i]), 60000)
+                assert same(r, want[i]) and _from_loop(r)
+            big = torch.zeros((320, 320, 320), dtype=torch.uint8, device="cuda")
+            tbig = srv.submit(big, big)
+            ts = [srv.submit(*p) for p in pairs]
+            for i, t in enumerate(ts):
+                r = srv.wait(t, 60000)
+                assert same(r, want[i]) and _from_loop(r), i
+            assert srv.wait(tbig, 60000)["status"] == hd.HD_ERR_OOM
+            assert srv.stats()["bytes_peak"] <= budget
+
+
+def test_groups_given_back_to_the_loop(hd, ctx, tmp_path):
+    """A tuning table that names the dilation loop: every group is refused and its
+    requests go to the loop."""
+    entry = {"kernel": 2, "bxw": 4, "bz": 8, "steps": 2, "ctas_per_sm": 0, "order": 0, "spread": 0, "us": 1.0}
+    table = tmp_path / "table.json"
+    table.write_text(json.dumps({"version": 1, "entries": {f"se6/v{v}/{p}": entry for v in range(30)
+                                                           for p in ("p1", "p2", "p16")}}))
+    pairs = _pairs(24, 71, 24, 112, edge=0.2)
+    host = [tuple(np.ascontiguousarray(m.cpu().numpy()) for m in p) for p in pairs]
+    want = [ctx.compute(*p, "se6") for p in pairs]
+    with hd.Context(0, tuning_table=str(table)) as c, hd.Server(c) as srv:
+        ts = [srv.submit(*(h if i % 3 == 0 else p)) for i, (p, h) in enumerate(zip(pairs, host))]
+        for i, t in enumerate(ts):
+            r = srv.wait(t, 60000)
+            assert same(r, want[i]) and _from_loop(r), i
