@@ -40,3 +40,30 @@ def test_span_ends(hd, ctx, oracle, shape, offs):
             g = c.compute(at_offset(ma, offs[0]), at_offset(mb, offs[1]), "se6")
             for k in ("n_a", "n_b", "n_a_not_b", "n_b_not_a", "hd", "hd_ab", "hd_ba", "sum_ab", "sum_ba", "avg_hd"):
                 assert g[k] == o[k], (k, g, o)
+
+
+@pytest.mark.parametrize("shape", [(520, 512, 32), (311, 301, 96), (131, 257, 256)])
+@pytest.mark.parametrize("label", [0, 3])
+def test_pipelined_aligned_words(hd, ctx, shape, label):
+    """The packing of the pipelined entry (rows of whole words, the next span asked
+    for ahead: several spans per warp, a ragged end), with and without a label,
+    against the blocking entry on masks of 0 and 1."""
+    g = torch.Generator(device="cuda").manual_seed(sum(shape) + label)
+    pairs, want = [], []
+    for i in range(5):
+        p = [torch.randint(0, 6, shape, generator=g, device="cuda", dtype=torch.uint8) for _ in range(2)]
+        p[i % 2][i:] = 0
+        p[i % 2].view(-1)[-1] = label or 1
+        fg = [((m == label) if label else (m != 0)) for m in p]
+        pairs.append(p)
+        want.append(ctx.compute(*(m.to(torch.uint8) for m in fg), "se6"))
+        assert (want[-1]["n_a"], want[-1]["n_b"]) == tuple(int(m.sum()) for m in fg)
+    outs = [torch.empty(hd.RESULT_BYTES, dtype=torch.uint8, device="cuda") for _ in pairs]
+    with hd.Context(0, label=label) as c:
+        for p, o in zip(pairs, outs):
+            c.compute_pipelined(*p, "se6", out=o)
+        c.flush()
+        torch.cuda.synchronize()
+    for i, (o, w) in enumerate(zip(outs, want)):
+        r = hd.result_from_bytes(o.cpu())
+        assert all(r[k] == w[k] for k in r if k != "iterations"), (i, r, w)
