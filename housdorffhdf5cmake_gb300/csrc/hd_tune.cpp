@@ -222,6 +222,8 @@ extern "C" hd_status hd_autotune(hd_context* ctx, const hd_pair_desc* pairs, int
             c.finish();
             double med = 0;
             const hd_status st = measure(c, &med);
+            // (its workspace may be larger than the loop's: no candidate then)
+            if (st == HD_ERR_OOM && c.kernel == 3) continue;
             if (st != HD_OK) return st;
             scored.emplace_back(med, c);
         }

@@ -170,3 +170,28 @@ def test_tuning_table_of_several_entries(hd, loop, tmp_path):
                 same(g, want, (side, n))
             t = c.last_timings()
             assert (t["kernel"], t["steps_per_barrier"]) == (kernel, steps), (side, n, t)
+
+
+def test_no_memory_for_the_workspace(hd, ctx):
+    """With room for the loop's workspace (1.6 GB) but not for the transform's (3.6
+    GB): calls take the loop, and the autotuner measures the loop alone."""
+    g = torch.Generator(device="cuda").manual_seed(5)
+    pair = [(torch.rand((512, 512, 512), generator=g, device="cuda") < 0.01).to(torch.uint8) for _ in range(2)]
+    want = ctx.compute(*pair, "se6")
+    pairs = [pair] * 12
+    torch.cuda.empty_cache()
+    with hd.Context(0, record_timings=True) as c:
+        c.compute(*(m[:8, :8, :8].contiguous() for m in pair), "se6")
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (2600 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            got = c.batch(pairs, "se6")
+            timings = c.last_timings()
+            report = c.autotune(pairs, "se6", repeats=1)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        assert timings["kernel"] == 2 and "kernel=2" in report and "kernel=3" not in report
+        for x in got:
+            same(x, want, "loop")
+        again = c.prepare_batch(pairs, "se6")
+        assert again.run()[0]["sum_ab"] == want["sum_ab"]
