@@ -953,7 +953,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         cudaEventRecord(ctx->split.ev[4], sv);
         ctx->split.timed = true;
         hd_timings& T = ctx->split.shape;
-        T.grid_ctas = (int)grid.x;
+        T.grid_ctas = dt ? 0 : (int)grid.x;
         T.brick_x_words = bxw;
         T.brick_z = bz;
         T.kernel = sh.kernel;
@@ -1004,7 +1004,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         cudaEventElapsedTime(&T.solve_ms, ctx->ev[2], ctx->ev[3]);
         cudaEventElapsedTime(&T.total_ms, ctx->ev[0], ctx->ev[3]);
         T.iterations = iters;
-        T.grid_ctas = (int)grid.x;
+        T.grid_ctas = dt ? 0 : (int)grid.x;
         T.brick_x_words = bxw;
         T.brick_z = bz;
         T.kernel = sh.kernel;

@@ -115,8 +115,8 @@ typedef struct hd_timings {
     int32_t grid_ctas;   /* CTAs of the persistent launch */
     int32_t brick_x_words, brick_z;
     int32_t kernel;      /* 1 = one step per barrier, 2 = temporally blocked, 3 = distance
-                            transform (no loop: iterations, bricks and steps are 0; its
-                            kernels count as solve_ms) */
+                            transform (no loop: iterations, grid_ctas, bricks and steps
+                            are 0; its kernels count as solve_ms) */
     int32_t steps_per_barrier;
     int32_t brick_rows;
     int32_t dilation_partitions; /* pipelined entry on split SMs: dilations in

@@ -195,3 +195,23 @@ def test_no_memory_for_the_workspace(hd, ctx):
             same(x, want, "loop")
         again = c.prepare_batch(pairs, "se6")
         assert again.run()[0]["sum_ab"] == want["sum_ab"]
+
+
+def test_timings_name_no_loop(hd):
+    """Timings of the transform: no iterations, no persistent grid, no bricks; of the
+    loop: all of them."""
+    a, b = (torch.from_numpy(m).cuda() for m in masks(np.random.default_rng(9), (40, 60, 70), "sparse"))
+    out = torch.empty(hd.RESULT_BYTES, dtype=torch.uint8, device="cuda")
+    fields = ("grid_ctas", "brick_x_words", "brick_z", "brick_rows", "steps_per_barrier")
+    for opts in ({}, {"kernel": 2}):
+        with hd.Context(0, record_timings=True, **opts) as c:
+            def pipelined():
+                c.compute_pipelined(a, b, "se6", out=out)
+                c.flush()
+                torch.cuda.synchronize()
+
+            for call in (lambda: c.compute(a, b, "se6"), lambda: c.batch([(a, b)] * 3, "se6"), pipelined):
+                call()
+                t = c.last_timings()
+                assert all((t[f] > 0) == bool(opts) for f in fields), (opts, t)
+                assert t["kernel"] == opts.get("kernel", 3) and t["solve_ms"] > 0
