@@ -9,7 +9,7 @@ available; the masks are seeded synthetic stand-ins with the stated shapes.
 
   value  pairs/s with the masks resident in HBM: K pairs enqueued back to
          back through hd_compute_u8_device_pipelined and one flush (packing
-         and set-up on a few SMs, consecutive pairs dilating side by side on
+         on a few SMs, consecutive pairs solved side by side on
          groups of the other SMs; each result decoded on the device and
          checked afterwards), CUDA events on the launch stream around the K
          steps; two distinct pairs alternate so every step reads
@@ -21,8 +21,8 @@ available; the masks are seeded synthetic stand-ins with the stated shapes.
          blocking hd_compute_u8 (one call per pair) is reported beside it
 Extra keys: Gvoxel-iter/s, the roofline of the dominant kernel, the serial
 CPU baseline (the oracle's restatement of the reference loop, 1 core), the
-ragged 256-pair batch (one persistent launch) against the same pairs one call
-each, the 512^3 far-blob worst case of the frontier queue, and a Poisson
+ragged 256-pair batch against the same pairs one call each, the 512^3 far-blob
+worst case (the dilation's longest frontier), and a Poisson
 serving stream through the continuous-batching server.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
@@ -303,11 +303,10 @@ def bench_ours(args):
     bricks //= 2
     kernel = phases[-1]["kernel"]
     solve_name = {1: "solve_kernel", 2: "solve_tb_kernel", 3: "dt_plane_kernel + dt_depth_kernel"}[kernel]
+    ctas = lambda p: f" ({p['grid_ctas']} CTAs)" if p["grid_ctas"] else ""  # (no persistent launch: 0)
     b_iter = 3 * 4096 * tiles
     if kernel == 3:
-        # distance transform: a byte per voxel of the domain (bounding box of
-        # A u B, x in words) and direction, written once and read once
-        b_iter = sum(4 * _domain_voxels(x, y) for x, y in pairs) / 2
+        b_iter = sum(_transform_bytes(x, y) for x, y in pairs) / 2
     b_pack = 2 * N + 2 * (N // 8)
     pk = statistics.mean(p["pack_ms"] for p in phases)
     su = statistics.mean(p["setup_ms"] for p in phases)
@@ -340,7 +339,7 @@ def bench_ours(args):
     if split_ph and dom == "solve":
         so_split = statistics.mean(p["solve_ms"] for p in split_ph)
         value_launch = {
-            "launch": f"{solve_name} on the dilation SMs of the pipelined entry ({split_ph[0]['grid_ctas']} CTAs)",
+            "launch": f"{solve_name} on the dilation SMs of the pipelined entry{ctas(split_ph[0])}",
             "solve_ms": round(so_split, 4), "pack_ms": round(statistics.mean(p["pack_ms"] for p in split_ph), 4),
             "setup_ms": round(statistics.mean(p["setup_ms"] for p in split_ph), 4),
             "achieved": round(b_iter / (so_split * 1e-3) / 1e9, 1)}
@@ -358,7 +357,8 @@ def bench_ours(args):
         achieved = value_launch["achieved"]
         so = so_split
     roofline = {
-        "bound": "hbm", "kernel": kname + {"solve": " (distance transform)" if kernel == 3 else " (persistent frontier dilation)", "pack": " (uint8 -> bits)",
+        # (the distance transform's kernels are chains of loads and barriers; their data stay in L2)
+        "bound": "latency" if kernel == 3 and dom == "solve" else "hbm", "kernel": kname + {"solve": " (distance transform)" if kernel == 3 else " (persistent frontier dilation)", "pack": " (uint8 -> bits)",
                                            "setup": " (crop + first queue)"}[dom],
         "achieved": round(achieved, 1) if achieved else None, "peak": peak, "unit": "GB/s",
         "frac": round(achieved / peak, 4) if achieved else None, "peak_source": f"{peak_kind} MEASURED_PEAKS hbm_gbs",
@@ -373,7 +373,7 @@ def bench_ours(args):
                                       "profile kernels launched in a green context")
         roofline["value_launch"] = value_launch
         roofline["whole_gpu_launch"] = {
-            "launch": f"{solve_name} of the blocking entry on every SM ({phases[-1]['grid_ctas']} CTAs)",
+            "launch": f"{solve_name} of the blocking entry on every SM{ctas(phases[-1])}",
             "solve_ms": round(so_whole, 4), "achieved": round(b_iter / (so_whole * 1e-3) / 1e9, 1),
             "frac": round(b_iter / (so_whole * 1e-3) / 1e9 / peak, 4)}
     gvox = (refs[0]["hd"] + refs[1]["hd"]) / 2 * 2 * N / (step_ms * 1e-3) / 1e9
@@ -456,7 +456,7 @@ def _check_fixture(r, cfg, name, se, what):
 
 
 def bench_batched(ctx, args):
-    """256 ragged pairs: one persistent launch vs one call per pair (own
+    """256 ragged pairs in one call vs one call per pair (own
     contexts sharing one tuning table: the timed calls uninstrumented, the
     phase times from an instrumented one)."""
     import torch
@@ -527,9 +527,7 @@ def bench_batched(ctx, args):
         tiles += int(sum(int(v) for v in tab[1: res["hd_ab"] + 1]) + sum(int(v) for v in tba[1: res["hd_ba"] + 1]))
     b_iter = 3 * 4096 * tiles
     if bt["kernel"] == 3:
-        # distance transform: a byte per voxel of each pair's domain and
-        # direction, written once and read once
-        b_iter = sum(4 * _domain_voxels(a, b) for (a, b), r in zip(pairs, batch) if r["hd"] > 0)
+        b_iter = sum(_transform_bytes(a, b) for a, b in pairs)
     peak, peak_kind = _peaks()
     solve_gbs = b_iter / (bt["solve_ms"] * 1e-3) / 1e9
     out = {
@@ -547,7 +545,7 @@ def bench_batched(ctx, args):
         "batched_phase_ms": {"pack": round(bt["pack_ms"], 3), "setup": round(bt["setup_ms"], 3),
                              "solve": round(bt["solve_ms"], 3), "barrier_iterations": bt["iterations"]},
         "pack_gbs_batched": round((2 * voxels + 2 * voxels / 8) / (bt["pack_ms"] * 1e-3) / 1e9, 1),
-        "solve_roofline": {"bound": "hbm", "algorithmic_bytes": b_iter, "frontier_tiles": tiles,
+        "solve_roofline": {"bound": "latency" if bt["kernel"] == 3 else "hbm", "algorithmic_bytes": b_iter, "frontier_tiles": tiles,
                            "solve_ms": round(bt["solve_ms"], 4), "achieved": round(solve_gbs, 1), "peak": peak,
                            "unit": "GB/s", "frac": round(solve_gbs / peak, 4),
                            "peak_source": f"{peak_kind} MEASURED_PEAKS hbm_gbs"},
@@ -773,7 +771,7 @@ def bench_worst_case(ctx, tctx, dev):
     per_step = [(int(tab[k]) if k <= res["hd_ab"] else 0) + (int(tba[k]) if k <= res["hd_ba"] else 0)
                 for k in range(1, steps + 1)]
     frac = [x / (2 * n_tiles) for x in per_step]
-    alg = 4 * _domain_voxels(a, b) if tim["kernel"] == 3 else 3 * 4096 * sum(per_step)
+    alg = _transform_bytes(a, b) if tim["kernel"] == 3 else 3 * 4096 * sum(per_step)
     return {
         "workload": "512^3, 8 balls r 3-6 vs 8 balls >= 200 voxels away, 6-neighbour element",
         "hd": r["hd"], "checked_against_oracle": bool(checked),
@@ -789,12 +787,30 @@ def bench_worst_case(ctx, tctx, dev):
     }
 
 
-def _domain_voxels(a, b):
-    """Voxels of the pair's domain: the bounding box of A u B, x in whole words."""
-    u = (a != 0) | (b != 0)
-    axes = [u.any(2).any(1), u.any(2).any(0), u.any(1).any(0)]  # z, y, x
-    lo, hi = zip(*[(int(v.nonzero().min()), int(v.nonzero().max())) for v in axes])
-    return (hi[0] - lo[0] + 1) * (hi[1] - lo[1] + 1) * 32 * (hi[2] // 32 - lo[2] // 32 + 1)
+def _transform_bytes(a, b):
+    """Bytes that the distance transform's two kernels hand on, a byte per voxel:
+    per direction with targets, the rows of the domain (bounding box of A u B, x
+    in whole words) in the planes that hold a source voxel, written once, and the
+    same planes of the columns (four rows x one word) that hold a target in some
+    plane, read once.  (They are no HBM traffic: most of them stay in L2.)"""
+    import torch
+    a, b = a != 0, b != 0
+    u = a | b
+    spans = [v.nonzero() for v in (u.any(2).any(1), u.any(2).any(0), u.any(1).any(0))]  # z, y, x
+    if any(v.numel() == 0 for v in spans):
+        return 0
+    (z0, z1), (y0, y1), (x0, x1) = [(int(v.min()), int(v.max()) + 1) for v in spans]
+    x0, words = x0 // 32 * 32, -(-x1 // 32) - x0 // 32
+    total = 0
+    for s, t in ((a, b & ~a), (b, a & ~b)):
+        if not (bool(s.any()) and bool(t.any())):
+            continue
+        planes = int(s[z0:z1].any(2).any(1).sum())
+        rows = t[z0:z1, y0:y1, x0:x1].any(0)
+        rows = torch.nn.functional.pad(rows, (0, 32 * words - rows.shape[1], 0, -rows.shape[0] % 4))
+        columns = int(rows.view(-1, 4, words, 32).any(3).any(1).sum())
+        total += planes * ((y1 - y0) * 32 * words + columns * 4 * 32)
+    return total
 
 
 def cpu_baseline(a_np, b_np, ref):
