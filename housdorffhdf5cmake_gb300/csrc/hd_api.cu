@@ -793,7 +793,6 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         Dd.D = P.D;
         Dd.wxf = q.wxf;
         Dd.se = se;
-        Dd.aligned = ((((uintptr_t)Dd.a) | ((uintptr_t)Dd.b)) & 15) == 0;
         Dd.kmax = q.kmax;
         Dd.job0 = 2 * i;
         Dd.info = direct ? dinfos : (PairInfo*)(dbase + off_infos) + i;

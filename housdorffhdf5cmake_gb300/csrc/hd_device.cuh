@@ -70,7 +70,6 @@ struct PairDesc {
     unsigned long long* hist[2];  // per job: kmax + 1 counters
     int32_t W, H, D, wxf;  // wxf = ceil(W / 32) words of a row (pitch: packed_pitch(W))
     int32_t se;          // 0: 6-neighbour, 1: 18-neighbour (forBench default)
-    int32_t aligned;     // a and b are 16-byte aligned
     int32_t kmax;        // iteration cap per job
     int32_t job0;        // index of this pair's first job (jobs 2p, 2p+1)
     unsigned long long brick0[2];  // first global brick id of each job

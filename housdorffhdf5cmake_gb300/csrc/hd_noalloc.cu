@@ -110,7 +110,6 @@ __global__ void noalloc_prepare(unsigned char* base, Layout L, const uint8_t* a,
     P->D = D;
     P->wxf = L.wxf;
     P->se = se;
-    P->aligned = ((((uintptr_t)a) | ((uintptr_t)b)) & 15) == 0;
     P->kmax = L.kmax;
     P->job0 = 0;
     P->info = I;

@@ -522,7 +522,6 @@ void tick(hd_server* s) {
         d.D = r->D;
         d.wxf = r->wxf;
         d.se = s->se;
-        d.aligned = ((((uintptr_t)d.a) | ((uintptr_t)d.b)) & 15) == 0;
         d.kmax = r->kmax;
         d.job0 = 2 * r->slot;
         d.epoch = ++s->slot_epoch[r->slot];
