@@ -718,10 +718,14 @@ def bench_serving(ctx, args):
     switch = sys.getswitchinterval()
     sys.setswitchinterval(2e-5)
     try:
-        # one server for every rate, warmed up by a burst of the whole
-        # stream (its memory pool then holds what the timed runs need)
+        # one server for every rate, warmed up by a burst of the whole stream
+        # (groups of requests: their workspace) and by each pair alone (the
+        # large ones take the dilation loop: its memory pool, whose first
+        # growth takes 3 ms)
         with hd.Server(ctx, hbm_budget_bytes=120 << 30) as srv:
             run(srv, 0.0)
+            for a, b in pool:
+                srv.wait(srv.submit(a, b), 60000)
             rows = [run(srv, f * plain_rate) for f in (0.5, 0.9, 1.5, 3.0)]
             rows.append(run(srv, 0.0))  # every request at t = 0: saturation throughput
     finally:
