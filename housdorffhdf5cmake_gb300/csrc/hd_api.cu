@@ -2,11 +2,14 @@
 //
 // Replaces HausdorffDistance::computeDistance (forBench/HausdorffDistance.cu:
 // 101-187) and the prototype's orchestration (hello.cu:892-1055, 1910-2062).
-// Per call: one upload of descriptors, the packing launch, the set-up launch,
-// ONE cooperative launch of the persistent dilation kernel that runs every
-// step on the device, and one read-back of a few hundred bytes.  No host
-// round trip per step (the reference does a blocking symbol read per step at
-// :167), no cudaDeviceReset, no exit.
+// Per call: the packing launch, then either the distance transform (two
+// launches of a single pair, three per group of a batch's pairs) or the set-up
+// launch and ONE cooperative launch of the persistent dilation kernel that runs
+// every step on the device.  A single pair's descriptor travels by value, a
+// batch's are uploaded once; the kernels write the results to pinned host memory
+// (asynchronous calls: to the caller's device memory).  No host round trip per
+// step (the reference does a blocking symbol read per step at :167), no
+// cudaDeviceReset, no exit.
 #include <cuda.h>
 #include <cuda_runtime.h>
 

@@ -21,8 +21,15 @@
 // byte per voxel over a base per tile holds them exactly.
 //
 // Both kernels together, against the dilation loop with its set-up: 512^3
-// with 451 steps 0.09 against 3.5 ms, 512x512x256 with 19 to 30 steps 0.037
-// against 0.10 to 0.13 ms, 64^3 0.019 against 0.08 ms.
+// with 445 steps 0.072 against 3.5 ms, 512x512x256 with 19 and 28 steps 0.045
+// against 0.10 to 0.13 ms, 64^3 0.019 against 0.08 ms.  Their time follows the
+// domain, not the steps: for masks that fill a large volume and differ by a few
+// steps the loop is the faster one (whole calls, us, transform / loop: 512x512x256
+// filled at random with 1 in 1000, 33 and 2 voxels, HD 22, 8 and 3: 282 / 345,
+// 355 / 166, 363 / 107; a box against itself moved by one voxel, HD 3: 216 / 93;
+// the same at 117x131x75 and below: the transform throughout).  Neither the
+// domain nor the number of steps is known before the launches; the options and
+// the autotuner choose the loop.
 //
 // Several pairs share launches (dt_planes_kernel, dt_list_kernel,
 // dt_columns_kernel): their planes and their columns with targets are claimed
@@ -136,11 +143,12 @@ __device__ __forceinline__ void plane_sync(int id, int threads) {
 //      rows; segments of 32 rows (the two halves) sweep on their own, then
 //      take the carry over the segments above and below from shared memory
 // About 400 warp instructions per 2048 voxels; issue slots 40 % busy (the
-// barrier per word column and the sweeps' chains).  A CTA whose planes have no
-// source voxel skips them, and rows are scanned once, from the right (the
-// words come one at a time after that, from L1): 512x512x256 pair 16 to 19 us
-// against 19 to 22 us with the words in groups of four registers, 512^3 with
-// small blobs (both directions) 51 to 65 against 97 to 114 us.  The barrier
+// barrier per word column and the sweeps' chains): 19 and 31 us for 512x512x256
+// pairs with 19 and 28 steps (cold caches).  A CTA whose planes have no source
+// voxel skips them, and rows are scanned once, from the right (the words come one
+// at a time after that, from L1): 3 us less for a 512x512x256 pair than with the
+// words in groups of four registers, 512^3 with small blobs (both directions) half
+// (51 to 65 against 97 to 114 us).  The barrier
 // per word column is among the plane's warps only (256 ragged pairs' planes and
 // columns 0.767 against 0.791 ms).
 
@@ -512,11 +520,12 @@ __host__ __device__ constexpr size_t depth_smem(int warps, int nseg, int bins, i
 // passes share one piece of code, and the targets of a task are visited in a
 // rolled loop: a CTA runs a few tasks only, so instruction fetches count.
 // Bound by the chain of loads, barriers and counters of one unit: a
-// 512x512x256 pair has 400 to 530 units for 608 CTAs.  512x512x256 pair 17 to
-// 22 us, 512^3 29 to 34 us, 64^3 12.5 us.  Before: with every column visited
-// and its segments' masks read behind a barrier 25-29 / 40-44 / 14 us; units
-// claimed from a counter 28-35 us at 512x512x256 (the claim waits once per
-// unit); 16 warps per CTA holding their segments over the barrier likewise.
+// 512x512x256 pair has 400 to 530 units for 608 CTAs.  512x512x256 pairs with 19
+// and 28 steps 17 and 28 us (cold caches).  When it was written, 512x512x256 pair /
+// 512^3 / 64^3: 17 to 22 / 29 to 34 / 12.5 us; with every column visited and its
+// segments' masks read behind a barrier 25-29 / 40-44 / 14; units claimed from a
+// counter 28-35 at 512x512x256 (the claim waits once per unit); 16 warps per CTA
+// holding their segments over the barrier likewise.
 template <bool kMap>
 __global__ void __launch_bounds__(kDepthMaxWarps * 32, 4) dt_depth_kernel(const __grid_constant__ DtPair p) {
     extern __shared__ uint4 sm4[];
@@ -955,14 +964,18 @@ namespace {
 
 constexpr int kPlaneCtas = 3;  // resident CTAs per SM (several pairs)
 
-// Resident CTAs per SM of one pair's planes.  3 (80 registers) on a group of 48
-// SMs, where there are always more planes than CTAs (eight 512x512x256 pairs 396
-// against 401 us), and where the planes of both directions, about 3/4 of all
-// as the domain is smaller than the volume, fill 2 per SM but not much more than
-// 3 (two 512x512x256 pairs 45.6 against 49.4 us, 256x256x200 of 400 planes 45.6
-// against 49.7).  Else 2 (122 registers): a plane's own time counts
-// (301x287x173 187 against 189 us for six), and many planes without a source
-// (512^3 141 against 154 us a call).
+// Resident CTAs per SM of one pair's planes: 3 (80 registers) or 2 (122), by the
+// depth alone, as the host knows neither the domain nor the planes with a source.
+// On a group of 48 SMs there are always more planes than CTAs: 3 (eight
+// 512x512x256 pairs 396 against 401 us).  On the whole GPU 3 where the planes of
+// both directions, taken as 3/4 of all, are more than 2 per SM but not much more
+// than 3.  Both kernels, 2 / 3 per SM, us, mean of 24 CT-like pairs (a single one
+// is 20 % either way, as its last round of CTAs fills up): 301x287x173 25.9 /
+// 25.6, 512x512 at D 210 / 256 / 300 / 340 / 440 30.1 / 29.6, 33.2 / 32.2, 35.9 /
+// 33.9, 38.9 / 36.6, 47.2 / 45.5, 256^3 30.0 / 28.7.  Domains of the whole volume: 1
+// % for 2 at 512x512, 2 to 5 % for 3 at 256x256 and 301x287 from D 173 on.  Few
+// planes with a source (far blobs) want 2: 512x512 at D 256 / 370 / 512 57.9 /
+// 70.2, 64.0 / 76.1, 74.0 / 82.2, hence the upper end.
 int plane_ctas(int D, int sms) {
     const double planes = 1.5 * D;
     return sms < 100 || (planes > 2 * sms && planes <= 3.5 * sms) ? 3 : 2;

@@ -172,7 +172,7 @@ struct PackWalk {
 };
 
 // One warp's span of a pair: words t0 .. t0 + kSpan - 1 of both masks (word t =
-// row r, word w of the row, stored at r * pitch + w), the bytes that hold them
+// row r, word w of the row, stored at PackWalk::at), the bytes that hold them
 // and the 16-byte chunks that cover these.
 struct PackSpan {
     unsigned cnt;            // words of the span
@@ -756,7 +756,7 @@ __global__ void zero_i32_kernel(int32_t* p, long long n) {
 // Bound by the maps' writes (the masks come from L2): 256^3 20 us (6.7 TB/s)
 // against 33.5 us with one voxel per thread and round; 1, 2, 8 rounds or 4 CTAs
 // per SM the same.
-constexpr int kMapThreads = 256, kMapRounds = 4, kMapGrid = 8 * 152;
+constexpr int kMapThreads = 256, kMapRounds = 4, kMapGrid = 8 * 152;  // 8 CTAs per SM of GB300
 template <bool kVec>
 __global__ void __launch_bounds__(kMapThreads) map_init_kernel(const __grid_constant__ PairDesc P, int32_t* __restrict__ map_a,
                                                                int32_t* __restrict__ map_b, int label) {

@@ -94,7 +94,12 @@ typedef struct hd_options {
     int32_t record_timings;      /* record CUDA events around each kernel (hd_context_last_timings) */
     int32_t kernel;              /* dilation kernel: 0 = tuned/default (pairs under HD_SE6 without any
                                     option that asks for the dilation loop - a kernel, a brick shape, a cap on
-                                    its steps or waits - take an exact distance transform instead), 1 = one step per grid barrier
+                                    its steps or waits - and up to 2048 x 512 x 1024 voxels, W + H + D <= 2304,
+                                    take an exact distance transform instead; a batch only if all its pairs do.
+                                    Its time does not grow with the distance, but with the bounding box of
+                                    A u B: for masks that fill more than 2^23 voxels and differ by a few steps
+                                    kernel = 2 is 1.5 to 4 times faster, and hd_autotune finds out),
+                                    1 = one step per grid barrier
                                     (brick_x_words x 32/brick_x_words rows x brick_z planes),
                                     2 = temporally blocked (steps_per_barrier steps per barrier,
                                     4 words x (32 - 2 steps) rows x brick_z planes) */
