@@ -136,6 +136,13 @@ constexpr int kQueueForBatchMode = 8;
 // barrier instead of waiting for a launch to end.
 constexpr int kGroupMin = 3, kGroupMax = 256, kGroupsPerTick = 8;
 constexpr long long kAloneVoxels = 1 << 26;
+// Barrier iterations of a tick after groups, which submissions do not end early:
+// with steady arrivals a tick that ends at its next barrier gave the resident pairs
+// one iteration per eight groups.  A request that only the loop takes (513 rows, 255
+// steps) among 24 k / 36 k others a second, ms: 12 to 21 / 115 so, 2.6 / 7.7 with 16
+// iterations, 1.9 / 4.4 with 32 (all in the loop: 8.8 / 27); p99 of the others 1.6
+// to 2.9 / 12, 0.5 / 0.5, 0.7 / 0.7 (1.2 / 3.6).
+constexpr int kTurnIterations = 32;
 constexpr size_t kGroupBytes = 65536;  // of a group's workspace, besides its pairs' shares
 
 }  // namespace
@@ -592,8 +599,12 @@ void tick(hd_server* s) {
         sp.pct = pct;
         sp.out = s->d_results;
         sp.decode_done_only = 1;
-        sp.yield = s->d_yield;
-        sp.yield_gen = ygen;
+        if (!grouped) {
+            sp.yield = s->d_yield;
+            sp.yield_gen = ygen;
+        } else if (!s->draining) {  // (a draining server admits nothing: no turn of others is due)
+            sp.max_iters = std::min(sp.max_iters, kTurnIterations);
+        }
         if (resident == 1 && s->shape.kernel == 2) {
             // a lone request: its two jobs are read from a per-CTA copy (the
             // jobs change only between ticks: set-up and retire run on this

@@ -50,6 +50,29 @@ def test_request_for_the_loop_before_many_others(hd, ctx, shape, budget):
     assert not budget or st["bytes_peak"] <= budget
 
 
+def test_resident_pair_among_steady_others(hd, ctx):
+    """A pair of 64 barrier iterations that only the loop takes is done before most
+    of the requests that arrive at a steady 38 k a second and are solved in groups."""
+    far = synth.pair_far_blobs(5, (200, 513, 300), "cuda", min_dist=80.0)
+    others = _pairs(8, 63, 190, 210)
+    want_far, want = ctx.compute(*far, "se6"), [ctx.compute(*p, "se6") for p in others]
+    n, pace = 4000, 26e-6
+    with hd.Server(ctx, max_queue=2 * n) as srv:
+        kind, at, t0 = {}, None, time.perf_counter()
+        for i in range(n):
+            while time.perf_counter() - t0 < i * pace:
+                pass
+            if i == 200:
+                t_far = srv.submit(*far)
+            kind[srv.submit(*others[i % 8])] = i % 8
+        for i in range(n + 1):
+            t, r = srv.wait_any(60000)
+            if t == t_far:
+                at = i
+            assert same(r, want_far if t == t_far else want[kind[t]]), i
+    assert at < n // 3, at
+
+
 LOOP = [("se18", {}), ("se6", {"kernel": 2})]
 
 
