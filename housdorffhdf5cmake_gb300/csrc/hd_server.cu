@@ -680,6 +680,7 @@ void tick(hd_server* s) {
     }
     if (stalled) hard_err = HD_ERR_ITER_LIMIT;
     unsigned long long cancelled_active = 0;
+    std::vector<size_t> left;  // slots of cancelled pairs (their requests are the callers' once they are done)
     uint32_t* hretire = (uint32_t*)(hp + s->off_h_retire);
     int nretire = 0;
     for (Request* r : finished) {
@@ -689,6 +690,7 @@ void tick(hd_server* s) {
         if (r->cancel) {
             st_r = HD_ERR_CANCELLED;
             cancelled_active += (s0.active != 0) + (s1.active != 0);
+            left.push_back(sl);
             r->result = hd_result{};
         } else if (hard_err) {
             r->result = hd_result{};
@@ -743,10 +745,8 @@ void tick(hd_server* s) {
             cudaMemcpyAsync(s->d_ctl, &z, sizeof z, cudaMemcpyHostToDevice, st);
             s->g_next += 2;
         } else {
-            for (Request* r : finished) {
-                if (!r->cancel) continue;
+            for (const size_t sl : left) {
                 JobState off{};
-                const size_t sl = (size_t)r->slot;
                 cudaMemcpyAsync(s->d_states + 2 * sl, &off, sizeof off, cudaMemcpyHostToDevice, st);
                 cudaMemcpyAsync(s->d_states + 2 * sl + 1, &off, sizeof off, cudaMemcpyHostToDevice, st);
             }
