@@ -201,7 +201,9 @@ __device__ __forceinline__ bool tb_decode(const SolveParams& p, unsigned long lo
     it.iter = g - k0;
     it.kb = it.iter * T;
     if (it.kb + 1 > kmax) {
-        if (lane == 0) {
+        // (entries of a job that finished in the iteration before are dropped:
+        // its last steps may have ended on the cap)
+        if (lane == 0 && it.active != 0) {
             it.st->status = kErrIterLimit;
             atomicCAS(&p.ctl->err, 0, kErrIterLimit);
         }
