@@ -570,14 +570,14 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         q.ncols = dt ? hdk::dt_cols(P.W, P.H) : 0;
         q.off_cols = sizeof(uint32_t) * 2 * (size_t)cols_words;  // from off_cols
         cols_words += q.ncols;
-        hist_words += 2ULL * (kmax + 1);
+        hist_words += 2ULL * (kmax + 1 + hdk::kHistRoom);
     }
     const size_t off_cols = take(sizeof(uint32_t) * 2 * cols_words);
     const size_t off_hist = take(sizeof(uint64_t) * hist_words);
     size_t hcur = 0;
     for (int i = 0; i < n; ++i) {
         plan[i].off_hist = off_hist + hcur * sizeof(uint64_t);
-        hcur += 2ULL * (plan[i].kmax + 1);
+        hcur += 2ULL * (plan[i].kmax + 1 + hdk::kHistRoom);
     }
     const size_t qbytes = sizeof(unsigned long long) * std::max<unsigned long long>(total_bricks, 1);
     const size_t off_q[3] = {take(qbytes), take(qbytes), take(qbytes)};
@@ -786,7 +786,7 @@ hd_status run_pairs(hd_context* ctx, const PairIn* pairs, int n, cudaStream_t s,
         Dd.pb = (uint32_t*)(dbase + q.off_pb);
         for (int j = 0; j < 2; ++j) {
             for (int b = 0; b < 3 && !dt; ++b) Dd.jb[j][b] = (uint32_t*)(dbase + q.off_jb[j][b]);
-            Dd.hist[j] = (unsigned long long*)(dbase + q.off_hist) + (size_t)j * (q.kmax + 1);
+            Dd.hist[j] = (unsigned long long*)(dbase + q.off_hist) + (size_t)j * (q.kmax + 1 + hdk::kHistRoom);
             Dd.brick0[j] = q.brick0 + (unsigned long long)j * q.bricks;
             Dd.tstamp[j] = stats ? (int32_t*)(dbase + q.off_tstamp[j]) : nullptr;
             Dd.tcount[j] = stats ? (unsigned long long*)(dbase + q.off_tcount[j]) : nullptr;

@@ -82,6 +82,10 @@ struct PairDesc {
     long long stile0;              // first set-up tile of this pair
 };
 
+// Counters past kmax where a caller caps the steps: the blocked kernel's
+// iteration that reaches the cap runs all its steps and counts their hits.
+constexpr int kHistRoom = 4;
+
 // Distance transform: sizes it takes (a plane's tiles of 64 rows in one CTA,
 // a column's segments and the distances' counters in shared memory).
 constexpr int kDtMaxW = 2048;

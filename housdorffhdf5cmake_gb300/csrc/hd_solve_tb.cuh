@@ -251,6 +251,7 @@ __device__ __forceinline__ void tb_issue(const SolveParams& p, unsigned long lon
 
 // What the epilogue of an item needs from its compute phase.
 constexpr int kTbMaxSteps = 5;
+static_assert(kTbMaxSteps - 1 <= kHistRoom, "steps of an iteration past the cap");
 constexpr unsigned kTbClaimRounds = 4;  // items per warp from which the queue's tail is claimed
 struct TbOut {
     unsigned cnt[kTbMaxSteps];  // newly covered voxels per step of the item

@@ -48,3 +48,21 @@ def test_short_pairs_join_a_long_one(hd, oracle, metric, opts):
             r, rf = srv.wait(t, 60000), srv.wait(tf, 60000)
             assert all(r[k] == want[i][k] for k in KEYS), (i, r, want[i])
             assert all(rf[k] == wfar[k] for k in KEYS), (i, rf, wfar)
+
+
+def test_hits_past_a_cap_on_the_steps(hd):
+    """With 4 steps per barrier and at most 5 steps the second iteration runs to step
+    8: B's voxels at distance 7 are counted, and A's counts (2 voxels at distance 5,
+    which set the robust HD) stay their own."""
+    a = torch.zeros((1, 40, 200), dtype=torch.uint8, device="cuda")
+    a[:, 10:30, 50:150] = 1
+    b = a.clone()
+    a[:, 20:22, 154] = 1
+    b[:, 30:33, 50:150] = 1
+    b[:, 36, 100:105] = 1
+    with hd.Context(0, kernel=2, steps_per_barrier=4) as c:
+        want = c.compute(a, b, "se6")
+    assert (want["hd_ab"], want["hd_ba"], want["hd_robust"]) == (5, 7, 5)
+    with hd.Context(0, kernel=2, steps_per_barrier=4, max_iterations=5) as c:
+        for r in [c.compute(a, b, "se6")] + c.batch([(a, b)] * 3, "se6"):
+            assert all(r[k] == want[k] for k in KEYS + ("hd_robust", "avg_hd")), (r, want)
